@@ -359,7 +359,12 @@ def run_gpu(args):
     peak, peak_kind = _peaks()
     tr = _traffic()
     shapes = {1: "8x4", 2: "4x8", 3: "16x2"}
-    if NEAR64[0]:
+    # the default on a uniform grid is the wave-step kernel, which a tuning entry reports as the
+    # choice whose time is the default's
+    wave = KERNEL[0] == 0 and not PAIR[0] and (not tuning or tuning["ms_per_sweep"] == tuning["default_ms_per_sweep"])
+    if wave:
+        kernel_name = "sweep3WaveKernel<float,near64>" if NEAR64[0] else "sweep3WaveKernel<float>"
+    elif NEAR64[0]:
         # the FP64 factor runs the chunk-step kernel's table instances, never the pair or
         # node-step kernels
         kernel_name = f"sweep3ChunkNear64Kernel<float,uniform,{shapes.get(tuning['block_shape'] if tuning else 1, '8x4')}>"

@@ -154,7 +154,7 @@ struct ScheduleKey {
         warm = 0, early = 0, nearFp64 = 0, warmGate = 0;
     double tol = 0, h = 0, dx = 0, dy = 0, dz = 0, gate = 0;
     unsigned long long spin = 0;
-    const void *tt = nullptr, *sp = nullptr, *srcs = nullptr, *corners = nullptr, *flags = nullptr;
+    const void *tt = nullptr, *sp = nullptr, *hs = nullptr, *srcs = nullptr, *corners = nullptr, *flags = nullptr;
     bool operator==(const ScheduleKey &o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
 };
 
@@ -165,6 +165,12 @@ struct TuneKey {
     bool operator<(const TuneKey &o) const {
         return std::tie(precision, uniform, nx, ny, nz, nsrc) < std::tie(o.precision, o.uniform, o.nx, o.ny, o.nz, o.nsrc);
     }
+};
+// A tuning entry: the reported choice, and whether it is the default step kernel of the class
+// (wave-step), which eikx_tuning has no value for (it then reads chunk-step, 8x4).
+struct Tuned {
+    eikx_tuning t{};
+    bool wave = false;
 };
 TuneKey tuneKey(int precision, bool uniform, int nx, int ny, int nz, int nSrc) {
     int p2 = 1;
@@ -213,7 +219,7 @@ struct eikx_ctx {
     DevBuf scratch;                // staging for host inputs and analytic fields
     Workspace ws;
     BatchWorkspace bw;
-    std::map<TuneKey, eikx_tuning> tuning;   // eikx_autotune3d results per grid class
+    std::map<TuneKey, Tuned> tuning;   // eikx_autotune3d results per grid class
     // the last eikx_solve3d / eikx_solve2d: its fields stay in ws.tt (row pitch Px)
     struct {
         bool valid = false;
@@ -384,7 +390,7 @@ cudaError_t assignFactorTables(std::vector<eikx::SourceFp64> &recs, DevBuf &buf)
     return cudaSuccess;
 }
 
-// A stream of sources through S = o.max_in_flight slots (3D, chunk-step).  Each slot solves
+// A stream of sources through S = o.max_in_flight slots (3D, wave-step or chunk-step).  Each slot solves
 // one source at a time in one of S + S/2 field buffers; the sweeps run iteration by
 // iteration (8 launches, each followed by the per-slot convergence test), and at each
 // iteration boundary the host reads the slots' flags: a field that converged (or ran
@@ -395,24 +401,23 @@ cudaError_t assignFactorTables(std::vector<eikx::SourceFp64> &recs, DevBuf &buf)
 template <class T>
 eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std::vector<eikx::SourceT<T>> &srcT,
                          const std::vector<eikx::SourceFp64> &srcT64In, const std::vector<eikx::Corner3> &corners,
-                         bool uniform, int shape, void *tOut, int where, DevBuf *spad) {
+                         bool uniform, bool wave, int shape, void *tOut, int where, DevBuf *spad) {
     StreamWorkspace &w = c->sw;
-    DevBuf *shad = c->shad3[sizeof(T) == 4 ? EIKX_F32 : EIKX_F64];   // uniform FP64 grids: the scaled copies
+    DevBuf *shad = c->shad3[sizeof(T) == 4 ? EIKX_F32 : EIKX_F64];   // uniform grids: the scaled copies
     const int nx = c->nx, ny = c->ny, nz = c->nz;
     const double dx = c->dx, dy = c->dy, dz = c->dz;
     const int Px = roundUp(nx, 4), spPitch = Px + 8;
     const long long fieldStride = static_cast<long long>(Px) * ny * nz;
     const int S = o.max_in_flight;
     const int nBufs = S + (S + 1) / 2;
-    const int ly = eikx::shapeLY(shape), lz = eikx::shapeLZ(shape);
-    const int tilesY = (ny + ly - 1) / ly, tilesZ = (nz + lz - 1) / lz;
+    const eikx::Tiling3 tl = eikx::tiling3<T>(wave, shape, Px, ny, nz);
+    const int ly = tl.ly, lz = tl.lz, tilesY = tl.tilesY, tilesZ = tl.tilesZ;
     const long long nProgressL = static_cast<long long>(S) * tilesY * tilesZ;
     if (nProgressL > std::numeric_limits<int>::max()) return fail(EIKX_ERR_INVALID, "too many slots for this grid");
     const int nProgress = static_cast<int>(nProgressL);
     const int nSweeps = std::max(0, o.n_sweeps);
     const int initSweeps = o.init_sweeps ? 1 : 0;
     const int resStride = 8 * (1 + nSweeps);
-    const int W = static_cast<int>(sizeof(T) / 4);
     // the stream's sweeps: every slot is busy until the sources run out, and a source takes
     // at most (init + n_sweeps) iterations
     const long long perSource = initSweeps + nSweeps;
@@ -421,7 +426,7 @@ eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std
     const int epochStride = static_cast<int>(8 * maxIters + 1);
 
     // buffers
-    const size_t mboxBytes = static_cast<size_t>(nProgress) * (ly + lz) * Px * W * 8;
+    const size_t mboxBytes = static_cast<size_t>(nProgress) * tl.faceWords * 8;
     EIKX_CUDA(w.tt.ensure(static_cast<size_t>(fieldStride) * nBufs * sizeof(T)));
     if (w.mbox.bytes < mboxBytes || !w.mbox.p) {
         EIKX_CUDA(w.mbox.ensure(mboxBytes));
@@ -494,7 +499,8 @@ eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std
     st.totalItems = nProgress - drop;
     const int spinLog2 = o.spin_limit_log2 > 0 ? std::min(o.spin_limit_log2, 40) : 22;
     st.spinLimit = 1ull << spinLog2;
-    int perSM = eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape);
+    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(false, near64)
+                       : eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
     const int blocks = std::max(1, std::min(c->numSMs * perSM, (nProgress + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock));
 
@@ -596,11 +602,12 @@ eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std
             a.srcs64 = near64 ? w.srcs64.as<eikx::SourceFp64>() : nullptr;
             a.slots = w.slots.as<int2>();
             a.initSweeps = initSweeps;
-            if (uniform && sizeof(T) == 8) {
+            if (wave || (uniform && sizeof(T) == 8)) {
                 a.hsPos = shad[0].as<T>(); a.hsNeg = shad[1].as<T>();
                 a.cells = c->slow3.p; a.cells64 = 1;
             }
-            EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
+            if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, blocks, c->stream));
+            else EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
             EIKX_CUDA(eikx::launchCheckStream(st, w.slots.as<int2>(), S, sweepsRun, initSweeps, o.tolerance, c->stream));
             if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * profiled + 1], c->stream));
             ++profiled;
@@ -781,9 +788,42 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     // geometry in the sweep type (include/private/solver3d.hpp:31-44, solver2d.hpp:29-46)
     const double eps = std::numeric_limits<T>::epsilon() * 100;
     const bool uniform = DIM == 3 ? (std::abs(dx - dy) < eps && std::abs(dx - dz) < eps) : (std::abs(dx - dz) < eps);
-    // uniform 3D grids in FP64: the padded copies multiplied by h, which the chunk-step kernel reads
+    // options left at "auto" take the tuned configuration of this grid class
+    if (DIM == 3 && o.sweep_kernel == 0 && o.block_shape == 0 && o.blocks_per_sm == 0 && !o.pair_fields) {
+        // a stream launches its slots' fields, not all of its sources
+        const int perLaunch = o.max_in_flight > 0 && o.max_in_flight < nSrc ? o.max_in_flight : nSrc;
+        auto it = c->tuning.find(tuneKey(P, uniform, nx, ny, nz, perLaunch));
+        if (it != c->tuning.end()) {
+            o.sweep_kernel = it->second.wave ? eikx::kWaveStep : it->second.t.sweep_kernel;
+            o.pair_fields = it->second.t.pair_fields;
+            o.block_shape = it->second.wave ? 0 : it->second.t.block_shape;
+            o.blocks_per_sm = it->second.t.blocks_per_sm;
+        }
+    }
+    // the FP64 factored branch runs in the wave-step and chunk-step kernels (their own instances)
+    if (DIM == 3 && P == EIKX_F32 && o.near_fp64) {
+        if (o.sweep_kernel == eikx::kNodeStep) o.sweep_kernel = eikx::kChunkStep;
+        o.pair_fields = 0;
+    }
+    // a stream runs on the wave-step or chunk-step kernel too
+    const bool stream = DIM == 3 && !warm && o.max_in_flight > 0 && o.max_in_flight < nSrc &&
+                        (o.init_sweeps || o.n_sweeps > 0);
+    if (stream) {
+        if (o.sweep_kernel == eikx::kNodeStep) o.sweep_kernel = eikx::kChunkStep;
+        o.pair_fields = 0;
+    }
+    // FP32 uniform 3D batches run two fields per lane (the paired kernel) on request
+    const bool paired = DIM == 3 && P == EIKX_F32 && uniform && nSrc >= 2 && o.pair_fields;
+    // the default on uniform grids is the wave-step kernel; a warp-block shape asks for chunk-step
+    const bool wave = DIM == 3 && uniform && !paired &&
+                        (o.sweep_kernel == eikx::kWaveStep || (o.sweep_kernel == 0 && o.block_shape == 0));
+    const int variant = wave ? eikx::kWaveStep : o.sweep_kernel == eikx::kNodeStep ? eikx::kNodeStep : eikx::kChunkStep;
+    const bool chunkStep = DIM == 3 && !paired && variant == eikx::kChunkStep;
+    // uniform 3D grids: the padded copies multiplied by h, which the wave-step kernel and the
+    // FP64 chunk-step kernel read
     DevBuf *shad = c->shad3[P];
-    if (DIM == 3 && sizeof(T) == 8 && uniform && (!c->shadValid3[P] || shad[0].bytes < spElems * sizeof(T))) {
+    if (DIM == 3 && uniform && (wave || (sizeof(T) == 8 && chunkStep)) &&
+        (!c->shadValid3[P] || shad[0].bytes < spElems * sizeof(T))) {
         if (shad[0].bytes < spElems * sizeof(T)) dropGraph(c);
         for (int k = 0; k < 2; ++k) {
             EIKX_CUDA(shad[k].ensure(spElems * sizeof(T)));
@@ -793,53 +833,32 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
         }
         c->shadValid3[P] = true;
     }
-    // options left at "auto" take the tuned configuration of this grid class
-    if (DIM == 3 && o.sweep_kernel == 0 && o.block_shape == 0 && o.blocks_per_sm == 0 && !o.pair_fields) {
-        // a stream launches its slots' fields, not all of its sources
-        const int perLaunch = o.max_in_flight > 0 && o.max_in_flight < nSrc ? o.max_in_flight : nSrc;
-        auto it = c->tuning.find(tuneKey(P, uniform, nx, ny, nz, perLaunch));
-        if (it != c->tuning.end()) {
-            o.sweep_kernel = it->second.sweep_kernel;
-            o.pair_fields = it->second.pair_fields;
-            o.block_shape = it->second.block_shape;
-            o.blocks_per_sm = it->second.blocks_per_sm;
-        }
-    }
-    // the FP64 factored branch runs in the chunk-step kernel (its own instances)
-    if (DIM == 3 && P == EIKX_F32 && o.near_fp64) {
-        o.sweep_kernel = eikx::kChunkStep;
-        o.pair_fields = 0;
-    }
-    // a stream of the sources through max_in_flight slots (chunk-step)
+    // a stream of the sources through max_in_flight slots
     if constexpr (DIM == 3) {
-        if (!warm && o.max_in_flight > 0 && o.max_in_flight < nSrc && (o.init_sweeps || o.n_sweeps > 0))
-            return solveStream3<T>(c, o, nSrc, srcT, srcT64, corners, uniform,
+        if (stream)
+            return solveStream3<T>(c, o, nSrc, srcT, srcT64, corners, uniform, wave,
                                    o.block_shape > 0 ? o.block_shape - 1 : eikx::kShape8x4, tOut, where, spad);
     }
-    // FP32 uniform 3D batches run two fields per lane (the paired kernel)
-    const bool paired = DIM == 3 && P == EIKX_F32 && uniform && nSrc >= 2 && o.pair_fields;
     const int nUnits = paired ? (nSrc + 1) / 2 : nSrc;   // work units: fields or field pairs
 
-    // sweep kernel and warp-block shape
-    const int variant = o.sweep_kernel == eikx::kNodeStep ? eikx::kNodeStep : eikx::kChunkStep;
-    const bool chunkStep = DIM == 3 && !paired && variant == eikx::kChunkStep;
+    // warp-block shape
     // 2D grids of up to 512 rows can run one CTA per field (sweep_kernel = 2); the warp-block
     // kernel is the default: measured faster on GB300 for 1 to 512 fields of 501 x 251 nodes
     const bool block2 = DIM == 2 && nz <= eikx::kMaxBlockRows2 && o.sweep_kernel == eikx::kChunkStep;
     const int shape = chunkStep && o.block_shape > 0 ? o.block_shape - 1 : eikx::kShape8x4;
 
     // workspace
-    const int ly = DIM == 3 ? eikx::shapeLY(shape) : 1, lz = DIM == 3 ? eikx::shapeLZ(shape) : eikx::LZ2;
-    const int tilesY = DIM == 3 ? (ny + ly - 1) / ly : 1;
-    const int tilesZ = (nz + lz - 1) / lz;
+    eikx::Tiling3 tl{1, eikx::LZ2, 1, (nz + eikx::LZ2 - 1) / eikx::LZ2, static_cast<long long>(Px) * (sizeof(T) / 4)};
+    if (DIM == 3) tl = eikx::tiling3<T>(wave, shape, Px, ny, nz);
+    if (paired) tl.faceWords *= 2;   // the two fields' values
+    const int ly = tl.ly, lz = tl.lz, tilesY = tl.tilesY, tilesZ = tl.tilesZ;
     const int nProgress = nUnits * tilesY * tilesZ;
     const int nSweepKinds = DIM == 3 ? 8 : 4;
     const int nSweeps = std::max(0, o.n_sweeps);
     const int resStride = nSweepKinds * (1 + nSweeps);
     Workspace &w = c->ws;
     const size_t ttBytes = static_cast<size_t>(fieldStride) * nSrc * sizeof(T);
-    const int mailWords = paired ? 2 : static_cast<int>(sizeof(T) / 4);   // tagged 64-bit words per unit
-    const size_t mboxBytes = static_cast<size_t>(nProgress) * (DIM == 3 ? ly + lz : 1) * Px * mailWords * 8;
+    const size_t mboxBytes = static_cast<size_t>(nProgress) * tl.faceWords * 8;
     const void *before[] = {w.tt.p, w.mbox.p, w.epoch.p, w.residual.p, w.converged.p,
                             w.iterations.p, w.order.p, w.srcs.p, w.corners.p, w.srcs64.p, w.factor.p};
     EIKX_CUDA(w.tt.ensure(ttBytes));
@@ -943,6 +962,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
 
     int perSM = paired ? eikx::sweep3PairBlocksPerSM()
                 : DIM == 2 ? eikx::sweep2BlocksPerSM<T>(uniform)
+                : wave ? eikx::sweep3WaveBlocksPerSM<T>(false, !srcT64.empty())
                 : chunkStep ? eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape)
                             : eikx::sweep3BlocksPerSM<T>(uniform);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
@@ -978,7 +998,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     sk.warmGate = warm ? o.warm_gate : 0;
     sk.variant = variant;
     sk.shape = shape;
-    sk.tt = w.tt.p; sk.sp = spad[0].p; sk.srcs = w.srcs.p; sk.corners = w.corners.p;
+    sk.tt = w.tt.p; sk.sp = spad[0].p; sk.hs = shad[0].p; sk.srcs = w.srcs.p; sk.corners = w.corners.p;
     sk.early = early ? 1 : 0;
     sk.flags = iterFlags;
 
@@ -1030,7 +1050,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                 a.sweepIndex = sweepsLaunched;
                 a.sweep = e; a.init = init; a.radius = o.factored_radius; a.h = static_cast<T>(dx);
                 a.srcs64 = srcs64;
-                if (uniform && sizeof(T) == 8) {
+                if (wave || (uniform && sizeof(T) == 8)) {
                     a.hsPos = shad[0].as<T>(); a.hsNeg = shad[1].as<T>();
                     a.cells = c->slow3.p; a.cells64 = 1;
                 }
@@ -1054,7 +1074,8 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                     }
                 }
                 if (!done) {
-                    if (chunkStep) EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
+                    if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, blocks, c->stream));
+                    else if (chunkStep) EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
                     else EIKX_CUDA(eikx::launchSweep3<T>(a, uniform, blocks, c->stream));
                 }
             } else {
@@ -1292,9 +1313,9 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
                         const eikx_options &o, eikx_stats &agg) {
     BatchWorkspace &w = c->bw;
     constexpr int V = 16 / sizeof(T);
-    constexpr int W = sizeof(T) / 4;
     const int shape = o.block_shape > 0 ? o.block_shape - 1 : eikx::kShape8x4;
-    const int ly = eikx::shapeLY(shape), lz = eikx::shapeLZ(shape);
+    const bool wave = uniform && o.sweep_kernel == 0 && o.block_shape == 0;   // as solveImpl
+    const int nCopies = wave ? 4 : 2;   // padded slowness copies: shifted, unshifted, then both times h
     const int nM = static_cast<int>(sel.size());
     struct Layout {
         int nx, ny, nz, Px, spPitch, tilesY, tilesZ, firstUnit, nSrc;
@@ -1310,18 +1331,19 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
         l.nx = m.nx; l.ny = m.ny; l.nz = m.nz;
         l.Px = roundUp(m.nx, 4);
         l.spPitch = l.Px + 8;
-        l.tilesY = (m.ny + ly - 1) / ly;
-        l.tilesZ = (m.nz + lz - 1) / lz;
+        const eikx::Tiling3 tl = eikx::tiling3<T>(wave, shape, l.Px, m.ny, m.nz);
+        l.tilesY = tl.tilesY;
+        l.tilesZ = tl.tilesZ;
         l.nSrc = m.n_src;
         l.firstUnit = nUnits;
         l.fieldStride = static_cast<long long>(l.Px) * m.ny * m.nz;
         l.spPlane = static_cast<long long>(l.spPitch) * (m.ny + 1);
         l.spElems = l.spPlane * (m.nz + 1);
-        l.faceWords = static_cast<long long>(ly + lz) * l.Px * W;
+        l.faceWords = tl.faceWords;
         l.ttOff = ttElems;
         ttElems += static_cast<size_t>(l.fieldStride) * m.n_src;
         l.spOff = spElems;
-        spElems += 2 * static_cast<size_t>(l.spElems);
+        spElems += static_cast<size_t>(nCopies) * l.spElems;
         l.mboxOff = mboxWords;
         mboxWords += static_cast<size_t>(m.n_src) * l.tilesY * l.tilesZ * l.faceWords;
         nUnits += m.n_src;
@@ -1427,6 +1449,9 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
                                                        c->stream)));
         EIKX_CUDA((eikx::launchPadSlowness3<T, double>(spBase + l.spOff + l.spElems, l.spPitch, 0, slow, m.nx, m.ny,
                                                        m.nz, c->stream)));
+        for (int k = 2; k < nCopies; ++k)
+            EIKX_CUDA((eikx::launchPadSlowness3<T, double>(spBase + l.spOff + k * l.spElems, l.spPitch, k == 2 ? V - 1 : 0,
+                                                           slow, m.nx, m.ny, m.nz, c->stream, static_cast<T>(m.dx))));
         for (int j = 0; j < m.n_src; ++j) {
             const int u = l.firstUnit + j;
             const size_t cell = (static_cast<size_t>(srcT[u].isz) * (m.ny - 1) + srcT[u].isy) * (m.nx - 1) + srcT[u].isx;
@@ -1438,6 +1463,8 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
             gu.tt = ttBase + l.ttOff + static_cast<size_t>(j) * l.fieldStride;
             gu.spPos = spBase + l.spOff;
             gu.spNeg = spBase + l.spOff + l.spElems;
+            gu.hsPos = wave ? spBase + l.spOff + 2 * l.spElems : nullptr;
+            gu.hsNeg = wave ? spBase + l.spOff + 3 * l.spElems : nullptr;
             gu.mbox = mbBase + l.mboxOff + static_cast<size_t>(j) * l.tilesY * l.tilesZ * l.faceWords;
             gu.spPlane = l.spPlane;
             gu.spPitch = l.spPitch;
@@ -1479,6 +1506,8 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     }
 
     // work order: every unit's warp blocks, sorted by the step at which they can start
+    const int ly = wave ? eikx::kWaveLY : eikx::shapeLY(shape);
+    const int lz = wave ? eikx::kWaveLZ : eikx::shapeLZ(shape);
     struct Item { int key, u, b, c; };
     std::vector<Item> items;
     items.reserve(nItems);
@@ -1531,7 +1560,8 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     st.totalItems = static_cast<int>(nItems);
     const int spinLog2 = o.spin_limit_log2 > 0 ? std::min(o.spin_limit_log2, 40) : 22;
     st.spinLimit = 1ull << spinLog2;
-    int perSM = eikx::sweep3ChunkBlocksPerSM<T>(uniform, true, shape);
+    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(true, near64)
+                       : eikx::sweep3ChunkBlocksPerSM<T>(uniform, true, shape);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
     const int blocks = std::max(1, static_cast<int>(std::min<size_t>(
                                        static_cast<size_t>(c->numSMs) * perSM,
@@ -1586,7 +1616,8 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
             a.sweep = e; a.init = init; a.radius = o.factored_radius;
             a.units = w.units.as<eikx::Grid3Unit<T>>();
             a.srcs64 = near64 ? w.srcs64.as<eikx::SourceFp64>() : nullptr;
-            EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
+            if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, blocks, c->stream));
+            else EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
             if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * sweepsLaunched + 1], c->stream));
             buf ^= 1;
             ++launches;
@@ -1616,7 +1647,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
                                static_cast<double>(o.n_sweeps), static_cast<double>(o.factored_radius),
                                static_cast<double>(o.init_sweeps), static_cast<double>(o.init_fp64), o.tolerance,
                                static_cast<double>(st.spinLimit), static_cast<double>(blocks),
-                               static_cast<double>(shape), static_cast<double>(o.near_fp64 ? 1 : 0)};
+                               static_cast<double>(wave ? -1 : shape), static_cast<double>(o.near_fp64 ? 1 : 0)};
     for (int i = 0; i < nM; ++i) {
         const eikx_model3d &m = models[sel[i]];
         for (double v : {static_cast<double>(m.nx), static_cast<double>(m.ny), static_cast<double>(m.nz), m.dx, m.dy,
@@ -1756,6 +1787,8 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
         o.blocks_per_sm = perSM;
         cands.push_back(o);
     };
+    // the untuned default first: wave-step on uniform grids, else chunk-step 8x4
+    if (uniform) add(eikx::kWaveStep, 0, 0, eikx::sweep3WaveBlocksPerSM<T>(false, false));
     for (int shape = 0; shape < eikx::kNumShapes; ++shape) {
         const int mx = eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape);
         add(eikx::kChunkStep, 0, shape + 1, mx);
@@ -1764,7 +1797,8 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
     add(eikx::kNodeStep, 0, 1, eikx::sweep3BlocksPerSM<T>(uniform));
     if (std::is_same<T, float>::value && uniform && nSrc >= 2) add(eikx::kChunkStep, 1, 1, eikx::sweep3PairBlocksPerSM());
     double best = 1e300, dflt = -1;
-    eikx_tuning pick{};
+    Tuned entry;
+    eikx_tuning &pick = entry.t;
     for (size_t i = 0; i < cands.size(); ++i) {
         double ms = 0;
         for (int rep = 0; rep < 2; ++rep) {
@@ -1772,19 +1806,20 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
                 return r;
             ms = c->stats.sweep_ms / std::max(1, c->stats.sweeps_launched);
         }
-        if (i == 0) dflt = ms;   // chunk-step, 8x4, full grid: the untuned default
+        if (i == 0) dflt = ms;
         if (ms < best) {
             best = ms;
-            pick.sweep_kernel = cands[i].sweep_kernel;
+            entry.wave = cands[i].sweep_kernel == eikx::kWaveStep;
+            pick.sweep_kernel = entry.wave ? eikx::kChunkStep : cands[i].sweep_kernel;
             pick.pair_fields = cands[i].pair_fields;
-            pick.block_shape = cands[i].block_shape;
+            pick.block_shape = entry.wave ? 1 : cands[i].block_shape;
             pick.blocks_per_sm = cands[i].blocks_per_sm;
         }
     }
     pick.ms_per_sweep = best;
     pick.default_ms_per_sweep = dflt;
     pick.candidates = static_cast<int>(cands.size());
-    c->tuning[tuneKey(P, uniform, c->nx, c->ny, c->nz, nSrc)] = pick;
+    c->tuning[tuneKey(P, uniform, c->nx, c->ny, c->nz, nSrc)] = entry;
     if (res) *res = pick;
     return EIKX_OK;
 }
@@ -2072,13 +2107,13 @@ eikx_status eikx_tuning_save(const eikx_ctx *c, const char *path) {
     if (!f) return fail(EIKX_ERR_INVALID, std::string("cannot write ") + path);
     for (const auto &kv : c->tuning) {
         const TuneKey &k = kv.first;
-        const eikx_tuning &t = kv.second;
+        const eikx_tuning &t = kv.second.t;
         f << "{\"precision\": " << k.precision << ", \"uniform\": " << k.uniform << ", \"nx\": " << k.nx
           << ", \"ny\": " << k.ny << ", \"nz\": " << k.nz << ", \"nsrc\": " << k.nsrc
           << ", \"sweep_kernel\": " << t.sweep_kernel << ", \"pair_fields\": " << t.pair_fields
           << ", \"block_shape\": " << t.block_shape << ", \"blocks_per_sm\": " << t.blocks_per_sm
           << ", \"ms_per_sweep\": " << t.ms_per_sweep << ", \"default_ms_per_sweep\": " << t.default_ms_per_sweep
-          << ", \"candidates\": " << t.candidates << "}\n";
+          << ", \"candidates\": " << t.candidates << (kv.second.wave ? ", \"wave\": 1" : "") << "}\n";
     }
     return f ? EIKX_OK : fail(EIKX_ERR_INVALID, std::string("cannot write ") + path);
 }
@@ -2090,12 +2125,13 @@ eikx_status eikx_tuning_load(eikx_ctx *c, const char *path) {
     if (!f) return fail(EIKX_ERR_INVALID, std::string("cannot read ") + path);
     std::string line;
     int lineNo = 0;
-    std::map<TuneKey, eikx_tuning> add;
+    std::map<TuneKey, Tuned> add;
     while (std::getline(f, line)) {
         ++lineNo;
         if (line.find_first_not_of(" \t\r") == std::string::npos) continue;
         TuneKey k{};
-        eikx_tuning t{};
+        Tuned entry;
+        eikx_tuning &t = entry.t;
         const int got = std::sscanf(line.c_str(),
                                     " {\"precision\": %d, \"uniform\": %d, \"nx\": %d, \"ny\": %d, \"nz\": %d, "
                                     "\"nsrc\": %d, \"sweep_kernel\": %d, \"pair_fields\": %d, \"block_shape\": %d, "
@@ -2107,7 +2143,8 @@ eikx_status eikx_tuning_load(eikx_ctx *c, const char *path) {
         if (got != 13 || t.sweep_kernel < 1 || t.sweep_kernel > 2 || t.block_shape < 1 ||
             t.block_shape > eikx::kNumShapes || t.blocks_per_sm < 0)
             return fail(EIKX_ERR_INVALID, std::string(path) + ":" + std::to_string(lineNo) + ": not a tuning entry");
-        add[k] = t;
+        entry.wave = line.find("\"wave\": 1") != std::string::npos;
+        add[k] = entry;
     }
     for (const auto &kv : add) c->tuning[kv.first] = kv.second;
     return EIKX_OK;

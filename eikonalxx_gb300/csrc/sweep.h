@@ -40,6 +40,7 @@ template <class T> struct Grid3Unit {
     int spPitch, Px, nx, ny, nz, tilesY, tilesZ, pad;
     T h;                          // uniform spacing
     Spacing3<T> sp3;              // non-uniform constants
+    const T *hsPos, *hsNeg;       // the padded copies multiplied by h (wave-step kernel)
 };
 
 template <class T> struct Sweep3Args {
@@ -72,10 +73,10 @@ template <class T> struct Sweep3Args {
     // stream and `sweep` its ordering (sweepIndex mod 8).
     const int2 *slots;
     int initSweeps;           // 1 = a slot's first 8 sweeps are its initialisation pass
-    // FP64 chunk-step kernel on a uniform grid, one model (required there): the padded
-    // slowness copies multiplied by h (launchPadSlowness3 with h), laid out as spPos / spNeg,
-    // and the model's natural-order cell slowness for the factored branch (FP64 cells, or FP32
-    // cells with cells64 = 0)
+    // Wave-step kernel, and FP64 chunk-step kernel on a uniform grid, one model (required
+    // there): the padded slowness copies multiplied by h (launchPadSlowness3 with h), laid out
+    // as spPos / spNeg; for the latter's factored branch also the model's natural-order cell
+    // slowness (FP64 cells, or FP32 cells with cells64 = 0)
     const T *hsPos, *hsNeg;
     const void *cells;
     int cells64;
@@ -138,8 +139,29 @@ template <class T> inline int sweep3ChunkBlocksPerSM(bool uniform, bool batch, i
     if (shape == kShape16x2) return sweep3ChunkBlocksPerSM_16x2<T>(uniform, batch);
     return sweep3ChunkBlocksPerSM_8x4<T>(uniform, batch);
 }
-// 3D sweep kernel variants (eikx_options.sweep_kernel).
-enum Sweep3Variant { kNodeStep = 1, kChunkStep = 2 };
+// 3D sweep kernel variants (eikx_options.sweep_kernel; kWaveStep is not a value of the
+// option: it is what the default takes on uniform grids).
+enum Sweep3Variant { kNodeStep = 1, kChunkStep = 2, kWaveStep = 3 };
+// Wave-step 3D kernel (sweep_wave.cu, uniform grids): a warp owns kWaveLY y'-rows x kWaveLZ
+// z'-rows, the blocks starting at the first updated rows; its mailbox holds waveStepCap(Px)
+// steps of kWaveLY + kWaveLZ values per block.
+constexpr int kWaveLY = 8, kWaveLZ = 4;
+__host__ __device__ constexpr int waveStepCap(int Px) { return Px + 32; }
+template <class T> cudaError_t launchSweep3Wave(const Sweep3Args<T> &a, int blocks, cudaStream_t s);
+template <class T> int sweep3WaveBlocksPerSM(bool batch, bool near64);
+// Warp blocks of one field, and the mailbox words each needs.
+struct Tiling3 {
+    int ly, lz, tilesY, tilesZ;
+    long long faceWords;
+};
+template <class T> inline Tiling3 tiling3(bool wave, int shape, int Px, int ny, int nz) {
+    constexpr long long W = sizeof(T) / 4;
+    if (wave)   // the first row of each axis is never updated
+        return {kWaveLY, kWaveLZ, (ny - 1 + kWaveLY - 1) / kWaveLY, (nz - 1 + kWaveLZ - 1) / kWaveLZ,
+                static_cast<long long>(waveStepCap(Px)) * (kWaveLY + kWaveLZ) * W};
+    const int ly = shapeLY(shape), lz = shapeLZ(shape);
+    return {ly, lz, (ny + ly - 1) / ly, (nz + lz - 1) / lz, static_cast<long long>(ly + lz) * Px * W};
+}
 // Paired 3D kernel (sweep_pair.cu): FP32, uniform grid, two fields of one model per lane.
 cudaError_t launchSweep3Pair(const Sweep3Args<float> &a, int blocks, cudaStream_t s);
 int sweep3PairBlocksPerSM();

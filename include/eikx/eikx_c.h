@@ -71,10 +71,12 @@ typedef struct {
                               size (the paired kernel needs 168 registers per thread, which
                               leaves 12 resident warps per SM).  Both give identical times. */
     int sweep_kernel;      /* 3D sweep kernel: 0 (default) = the tuned kernel of this grid class
-                              if eikx_autotune3d ran, else chunk-step; 1 = node-step (a
-                              lane updates one node per wavefront step), 2 = chunk-step (a
-                              lane updates one 16-byte chunk, 4 FP32 / 2 FP64 nodes, per
-                              step).  2D: 0 and 1 = warp blocks of 32 rows; 2 = one CTA
+                              if eikx_autotune3d ran, else wave-step on uniform grids (a lane
+                              updates one node per wavefront step, rows through a
+                              shared-memory ring) unless block_shape asks for chunk-step,
+                              and chunk-step on others; 1 = node-step (the earlier kernel of
+                              one node per lane and step), 2 = chunk-step (a lane updates one
+                              16-byte chunk, 4 FP32 / 2 FP64 nodes, per step).  2D: 0 and 1 = warp blocks of 32 rows; 2 = one CTA
                               per field, one thread per row (grids of up to 512 rows; slower
                               on GB300, whose FP64 units one SM cannot keep fed).  All give
                               identical travel times. */
@@ -95,7 +97,8 @@ typedef struct {
                               upwind neighbours and the candidate T0 + correction, each
                               rounded to FP32; the quadratic solves stay in FP32.  0 (default)
                               = all in FP32, as the reference's sweep type.  Runs on the
-                              chunk-step kernel (sweep_kernel and pair_fields give way).
+                              wave-step or chunk-step kernel (node-step and pair_fields
+                              give way).
                               Ignored by FP64 solves and 2D. */
     int warm_gate;         /* eikx_solve3d_warm's residual gate: 0 (default) = reset nodes
                               whose initial time lies more than gate_tol below the smallest
@@ -107,8 +110,8 @@ typedef struct {
                               copied out and takes the next source at the next iteration
                               boundary, its initialisation sweeps running inside the same
                               launches as the other slots' refinement sweeps.  The fields
-                              are bit-identical to solving each source alone.  Chunk-step
-                              kernel (sweep_kernel and pair_fields give way); no CUDA graph
+                              are bit-identical to solving each source alone.  Wave-step
+                              or chunk-step kernel (node-step and pair_fields give way); no CUDA graph
                               (the schedule follows convergence); the fields do not stay on
                               the device for eikx_gradient3d / eikx_station_times3d. */
     int reserved;
@@ -271,12 +274,15 @@ eikx_status eikx_trace_rays2d(eikx_ctx *ctx, int nx, int nz, double dx, double d
 
 /* The configuration eikx_autotune3d chose for one grid class. */
 typedef struct {
-    int sweep_kernel;              /* 1 = node-step, 2 = chunk-step */
+    int sweep_kernel;              /* 1 = node-step, 2 = chunk-step; where the untuned default
+                                      of a uniform grid (wave-step, no value here) is the
+                                      fastest, 2 with block_shape 1 and ms_per_sweep equal to
+                                      default_ms_per_sweep */
     int pair_fields;               /* 1 = two FP32 fields per lane */
     int block_shape;               /* 1 = 8x4, 2 = 4x8, 3 = 16x2 (chunk-step) */
     int blocks_per_sm;             /* resident blocks per SM of the persistent grid */
     double ms_per_sweep;           /* measured mean sweep launch of the choice */
-    double default_ms_per_sweep;   /* the untuned default (chunk-step, 8x4, full grid) */
+    double default_ms_per_sweep;   /* the untuned default, full grid */
     int candidates;                /* configurations timed */
 } eikx_tuning;
 
