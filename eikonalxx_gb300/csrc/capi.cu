@@ -216,6 +216,8 @@ struct eikx_ctx {
     PinnedBuf srcSlow;             // source-cell slownesses of a solve, read from the device
     DevBuf spad2[2][2];
     bool spadValid2[2] = {false, false};
+    DevBuf shad2[2];               // FP64, the same multiplied by h (uniform grids)
+    bool shadValid2 = false;
     DevBuf scratch;                // staging for host inputs and analytic fields
     Workspace ws;
     BatchWorkspace bw;
@@ -325,7 +327,7 @@ eikx_status finishModel(eikx_ctx *c, int dim) {
     } else {
         c->haveSlow2 = false;
         c->hostSlow2Valid = false;
-        c->spadValid2[0] = c->spadValid2[1] = false;
+        c->spadValid2[0] = c->spadValid2[1] = c->shadValid2 = false;
     }
     if (bad) return fail(EIKX_ERR_INVALID, "Non-positive velocities detected");
     (dim == 3 ? c->haveSlow3 : c->haveSlow2) = true;
@@ -788,6 +790,17 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     // geometry in the sweep type (include/private/solver3d.hpp:31-44, solver2d.hpp:29-46)
     const double eps = std::numeric_limits<T>::epsilon() * 100;
     const bool uniform = DIM == 3 ? (std::abs(dx - dy) < eps && std::abs(dx - dz) < eps) : (std::abs(dx - dz) < eps);
+    // 2D, FP64, uniform: the padded copies multiplied by h, which the wave-step kernel reads
+    if (DIM == 2 && sizeof(T) == 8 && uniform && (!c->shadValid2 || c->shad2[0].bytes < spElems * sizeof(T))) {
+        if (c->shad2[0].bytes < spElems * sizeof(T)) dropGraph(c);
+        for (int k = 0; k < 2; ++k) {
+            EIKX_CUDA(c->shad2[k].ensure(spElems * sizeof(T)));
+            const int shift = k == 0 ? static_cast<int>(16 / sizeof(T)) - 1 : 0;
+            EIKX_CUDA((eikx::launchPadSlowness2<T, double>(c->shad2[k].as<T>(), spPitch, shift, c->slow2.as<double>(), nx, nz,
+                                                           c->stream, static_cast<T>(dx))));
+        }
+        c->shadValid2 = true;
+    }
     // options left at "auto" take the tuned configuration of this grid class
     if (DIM == 3 && o.sweep_kernel == 0 && o.block_shape == 0 && o.blocks_per_sm == 0 && !o.pair_fields) {
         // a stream launches its slots' fields, not all of its sources
@@ -848,7 +861,8 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     const int shape = chunkStep && o.block_shape > 0 ? o.block_shape - 1 : eikx::kShape8x4;
 
     // workspace
-    eikx::Tiling3 tl{1, eikx::LZ2, 1, (nz + eikx::LZ2 - 1) / eikx::LZ2, static_cast<long long>(Px) * (sizeof(T) / 4)};
+    eikx::Tiling3 tl{1, eikx::kWaveRows2, 1, (nz - 1 + eikx::kWaveRows2 - 1) / eikx::kWaveRows2,
+                     static_cast<long long>(eikx::waveStepCap2(Px)) * (sizeof(T) / 4)};
     if (DIM == 3) tl = eikx::tiling3<T>(wave, shape, Px, ny, nz);
     if (paired) tl.faceWords *= 2;   // the two fields' values
     const int ly = tl.ly, lz = tl.lz, tilesY = tl.tilesY, tilesZ = tl.tilesZ;
@@ -961,7 +975,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     st.spinLimit = 1ull << spinLog2;
 
     int perSM = paired ? eikx::sweep3PairBlocksPerSM()
-                : DIM == 2 ? eikx::sweep2BlocksPerSM<T>(uniform)
+                : DIM == 2 ? eikx::sweep2WaveBlocksPerSM<T>(uniform)
                 : wave ? eikx::sweep3WaveBlocksPerSM<T>(false, !srcT64.empty())
                 : chunkStep ? eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape)
                             : eikx::sweep3BlocksPerSM<T>(uniform);
@@ -996,9 +1010,9 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     sk.gate = gateTol;
     sk.nearFp64 = DIM == 3 && P == EIKX_F32 && o.near_fp64 ? 1 : 0;
     sk.warmGate = warm ? o.warm_gate : 0;
-    sk.variant = variant;
+    sk.variant = DIM == 3 ? variant : block2 ? 1 : 0;
     sk.shape = shape;
-    sk.tt = w.tt.p; sk.sp = spad[0].p; sk.hs = shad[0].p; sk.srcs = w.srcs.p; sk.corners = w.corners.p;
+    sk.tt = w.tt.p; sk.sp = spad[0].p; sk.hs = DIM == 3 ? shad[0].p : c->shad2[0].p; sk.srcs = w.srcs.p; sk.corners = w.corners.p;
     sk.early = early ? 1 : 0;
     sk.flags = iterFlags;
 
@@ -1093,7 +1107,12 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                 g.sinTheta = static_cast<T>(dz / std::hypot(dx, dz));
                 a.sp2 = g;
                 if (block2) EIKX_CUDA(eikx::launchSweep2Block<T>(a, uniform, nSrc, c->stream));
-                else EIKX_CUDA(eikx::launchSweep2<T>(a, uniform, blocks, c->stream));
+                else {
+                    if (sizeof(T) == 8 && uniform) {
+                        a.hsPos = c->shad2[0].as<T>(); a.hsNeg = c->shad2[1].as<T>();
+                    }
+                    EIKX_CUDA(eikx::launchSweep2Wave<T>(a, uniform, blocks, c->stream));
+                }
             }
             if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * sweepsLaunched + 1], c->stream));
             buf ^= 1;
@@ -1939,7 +1958,7 @@ eikx_status eikx_set_grid2d(eikx_ctx *c, int nx, int nz, double dx, double dz, d
     c->nx2 = nx; c->nz2 = nz; c->dx2 = dx; c->dz2 = dz; c->x02 = x0; c->z02 = z0;
     c->haveGrid2 = true;
     c->haveSlow2 = false;
-    c->spadValid2[0] = c->spadValid2[1] = false;
+    c->spadValid2[0] = c->spadValid2[1] = c->shadValid2 = false;
     dropGraph(c);
     return EIKX_OK;
 }

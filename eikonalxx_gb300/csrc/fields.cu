@@ -249,7 +249,7 @@ __global__ void pad3Kernel(T *sp, int spPitch, int shift, const U *s, int nx, in
 
 
 template <class T, class U>
-__global__ void pad2Kernel(T *sp, int spPitch, int shift, const U *s, int nx, int nz) {
+__global__ void pad2Kernel(T *sp, int spPitch, int shift, const U *s, int nx, int nz, T h) {
     const int ncx = nx - 1, ncz = nz - 1;
     const long long n = static_cast<long long>(spPitch) * (nz + 1);
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
@@ -257,7 +257,8 @@ __global__ void pad2Kernel(T *sp, int spPitch, int shift, const U *s, int nx, in
         const int px = static_cast<int>(i % spPitch);
         const int pz = static_cast<int>(i / spPitch);
         const int cx = clampi(px - 1 - shift, 0, ncx - 1), cz = clampi(pz - 1, 0, ncz - 1);
-        sp[i] = static_cast<T>(s[static_cast<long long>(cz) * ncx + cx]);
+        const T v = static_cast<T>(s[static_cast<long long>(cz) * ncx + cx]);
+        sp[i] = h > 0 ? v * h : v;
     }
 }
 
@@ -516,9 +517,9 @@ cudaError_t launchPadSlowness3(T *sp, int spPitch, int shift, const U *s, int nx
     return cudaGetLastError();
 }
 template <class T, class U>
-cudaError_t launchPadSlowness2(T *sp, int spPitch, int shift, const U *s, int nx, int nz, cudaStream_t st) {
+cudaError_t launchPadSlowness2(T *sp, int spPitch, int shift, const U *s, int nx, int nz, cudaStream_t st, T h) {
     const long long n = static_cast<long long>(spPitch) * (nz + 1);
-    pad2Kernel<T, U><<<gridFor(n), kThreads, 0, st>>>(sp, spPitch, shift, s, nx, nz);
+    pad2Kernel<T, U><<<gridFor(n), kThreads, 0, st>>>(sp, spPitch, shift, s, nx, nz, h);
     return cudaGetLastError();
 }
 template <class U>
@@ -648,8 +649,8 @@ template cudaError_t launchPadSlowness3<double, double>(double *, int, int, cons
                                                         cudaStream_t, double);
 template cudaError_t launchPadSlowness3<float, float>(float *, int, int, const float *, int, int, int, cudaStream_t,
                                                       float);
-template cudaError_t launchPadSlowness2<float, double>(float *, int, int, const double *, int, int, cudaStream_t);
-template cudaError_t launchPadSlowness2<double, double>(double *, int, int, const double *, int, int, cudaStream_t);
+template cudaError_t launchPadSlowness2<float, double>(float *, int, int, const double *, int, int, cudaStream_t, float);
+template cudaError_t launchPadSlowness2<double, double>(double *, int, int, const double *, int, int, cudaStream_t, double);
 template cudaError_t launchNodalToCell3<float>(double *, const float *, int, int, int, int, cudaStream_t);
 template cudaError_t launchNodalToCell3<double>(double *, const double *, int, int, int, int, cudaStream_t);
 template cudaError_t launchNodalToCell2<float>(double *, const float *, int, int, int, cudaStream_t);

@@ -677,14 +677,12 @@ template <class T> struct Spacing2 {
 };
 
 // 2D uniform update (solverUtilities2d.hpp:347-472).  t1 = x-up, t2 = diagonal,
-// t3 = z-up; s0 home cell, s1 x-neighbour cell, s3 z-neighbour cell.
+// t3 = z-up; s0 home cell, s1 x-neighbour cell, s3 z-neighbour cell.  Split at the branch on
+// the factored radius: the Cartesian operators, and the factored one near the source.
 template <class T>
-__device__ __forceinline__ T fd2Uniform(int radius, T h, const SourceT<T> &src,
-                                        const SweepSigns &sg, int ix, int iz, T s0, T s1, T s3,
-                                        T t1, T t2, T t3) {
+__device__ __forceinline__ T fd2UniformFar(T h, T s0, T s1, T s3, T t1, T t2, T t3) {
     const T huge = static_cast<T>(1.e10);
     const T sqrt1_2 = static_cast<T>(0.70710678118654752440);
-    T tUpd;
     T t0x = t1 + h * dmin(s0, s3);
     T t0z = t3 + h * dmin(s0, s1);
     T t0Update1 = dmin(t0x, t0z);
@@ -693,59 +691,70 @@ __device__ __forceinline__ T fd2Uniform(int radius, T h, const SourceT<T> &src,
     T dTz = t1 - t2;
     T sx = sqrt1_2 * s0;
     T sz = sqrt1_2 * s0;
-    if (abs(src.isx - ix) > radius || abs(src.isz - iz) > radius) {
-        T t0a = huge;
-        T deta = hs0 * hs0 - dTz * dTz;
-        if (dTz >= 0 && deta >= 0 && dTz <= h * sz) t0a = t1 + h * dsqrt(deta);
-        T t0b = huge;
-        T detb = hs0 * hs0 - dTx * dTx;
-        if (dTx >= 0 && detb >= 0 && dTx <= h * sx) t0b = t3 + h * dsqrt(detb);
-        T t0Update2 = dmin(t0a, t0b);
-        T dtCross = t1 - t3;
-        T detc = 2 * (hs0 * hs0) - dtCross * dtCross;
-        T t0Update3 = huge;
-        if (dTx >= 0 && dTz >= 0 && detc > 0 && t3 <= t1 + hs0 && t1 <= t3 + hs0)
-            t0Update3 = t2 + dsqrt(detc);
-        tUpd = dmin(dmin(t0Update1, t0Update2), t0Update3);
-    } else {
-        T t0Update3 = huge;
-        if (dTx >= 0 && dTz >= 0 && t1 < t3 + hs0 && t3 < t1 + hs0) {
-            const T sSrc = src.sSrc;
-            T dt0dx, dt0dz, t0;
-            analyticTG2(ix, iz, h, h, src.xs, src.zs, sSrc, t0, dt0dx, dt0dz);
-            T tau1 = t1 - analyticT2(ix + sg.ixShift, iz, h, h, src.xs, src.zs, sSrc);
-            T tau2 = t2 - analyticT2(ix + sg.ixShift, iz + sg.izShift, h, h, src.xs, src.zs, sSrc);
-            T tau3 = t3 - analyticT2(ix, iz + sg.izShift, h, h, src.xs, src.zs, sSrc);
-            dt0dx = sg.signX * dt0dx;
-            dt0dz = sg.signZ * dt0dz;
-            T tauX = tau1 - tau3 + tau2;
-            T tauZ = tau3 - tau1 + tau2;
-            const T one = 1, two = 2, four = 4;
-            T h2 = h * h;
-            T a = one / h2;
-            T b = two / h * (dt0dx + dt0dz) - two / h2 * tau2;
-            T c = one / (two * h2) * (tauX * tauX + tauZ * tauZ) -
-                  two / h * (dt0dx * tauX + dt0dz * tauZ) + two * (sSrc * sSrc - s0 * s0);
-            T det = b * b - four * a * c;
-            if (det >= 0) {
-                T tau = (-b + dsqrt(det)) / (two * a);
-                t0Update3 = t0 + tau;
-            }
-            if (t0Update3 < t1 || t0Update3 < t3) t0Update3 = huge;
+    T t0a = huge;
+    T deta = hs0 * hs0 - dTz * dTz;
+    if (dTz >= 0 && deta >= 0 && dTz <= h * sz) t0a = t1 + h * dsqrt(deta);
+    T t0b = huge;
+    T detb = hs0 * hs0 - dTx * dTx;
+    if (dTx >= 0 && detb >= 0 && dTx <= h * sx) t0b = t3 + h * dsqrt(detb);
+    T t0Update2 = dmin(t0a, t0b);
+    T dtCross = t1 - t3;
+    T detc = 2 * (hs0 * hs0) - dtCross * dtCross;
+    T t0Update3 = huge;
+    if (dTx >= 0 && dTz >= 0 && detc > 0 && t3 <= t1 + hs0 && t1 <= t3 + hs0)
+        t0Update3 = t2 + dsqrt(detc);
+    return dmin(dmin(t0Update1, t0Update2), t0Update3);
+}
+template <class T>
+__device__ __forceinline__ T fd2UniformNear(T h, const SourceT<T> &src, const SweepSigns &sg, int ix, int iz, T s0,
+                                            T s1, T s3, T t1, T t2, T t3) {
+    const T huge = static_cast<T>(1.e10);
+    T t0x = t1 + h * dmin(s0, s3);
+    T t0z = t3 + h * dmin(s0, s1);
+    T t0Update1 = dmin(t0x, t0z);
+    T hs0 = h * s0;
+    T dTx = t3 - t2;
+    T dTz = t1 - t2;
+    T t0Update3 = huge;
+    if (dTx >= 0 && dTz >= 0 && t1 < t3 + hs0 && t3 < t1 + hs0) {
+        const T sSrc = src.sSrc;
+        T dt0dx, dt0dz, t0;
+        analyticTG2(ix, iz, h, h, src.xs, src.zs, sSrc, t0, dt0dx, dt0dz);
+        T tau1 = t1 - analyticT2(ix + sg.ixShift, iz, h, h, src.xs, src.zs, sSrc);
+        T tau2 = t2 - analyticT2(ix + sg.ixShift, iz + sg.izShift, h, h, src.xs, src.zs, sSrc);
+        T tau3 = t3 - analyticT2(ix, iz + sg.izShift, h, h, src.xs, src.zs, sSrc);
+        dt0dx = sg.signX * dt0dx;
+        dt0dz = sg.signZ * dt0dz;
+        T tauX = tau1 - tau3 + tau2;
+        T tauZ = tau3 - tau1 + tau2;
+        const T one = 1, two = 2, four = 4;
+        T h2 = h * h;
+        T a = one / h2;
+        T b = two / h * (dt0dx + dt0dz) - two / h2 * tau2;
+        T c = one / (two * h2) * (tauX * tauX + tauZ * tauZ) -
+              two / h * (dt0dx * tauX + dt0dz * tauZ) + two * (sSrc * sSrc - s0 * s0);
+        T det = b * b - four * a * c;
+        if (det >= 0) {
+            T tau = (-b + dsqrt(det)) / (two * a);
+            t0Update3 = t0 + tau;
         }
-        tUpd = dmin(t0Update1, t0Update3);
+        if (t0Update3 < t1 || t0Update3 < t3) t0Update3 = huge;
     }
-    return tUpd;
+    return dmin(t0Update1, t0Update3);
+}
+template <class T>
+__device__ __forceinline__ T fd2Uniform(int radius, T h, const SourceT<T> &src,
+                                        const SweepSigns &sg, int ix, int iz, T s0, T s1, T s3,
+                                        T t1, T t2, T t3) {
+    if (abs(src.isx - ix) > radius || abs(src.isz - iz) > radius) return fd2UniformFar(h, s0, s1, s3, t1, t2, t3);
+    return fd2UniformNear(h, src, sg, ix, iz, s0, s1, s3, t1, t2, t3);
 }
 
-// 2D non-uniform update (solverUtilities2d.hpp:474-614).
+// 2D non-uniform update (solverUtilities2d.hpp:474-614), split like the uniform one.
 template <class T>
-__device__ __forceinline__ T fd2NonUniform(int radius, const Spacing2<T> &g, const SourceT<T> &src,
-                                           const SweepSigns &sg, int ix, int iz, T s0, T s1, T s3,
-                                           T t1, T t2, T t3) {
+__device__ __forceinline__ T fd2NonUniformFar(const Spacing2<T> &g, T s0, T s1, T s3, T t1, T t2, T t3) {
     const T huge = static_cast<T>(1.e10);
     const T dx = g.dx, dz = g.dz;
-    T tUpd;
     T t0x = t1 + dx * dmin(s0, s3);
     T t0z = t3 + dz * dmin(s0, s1);
     T t0Update1 = dmin(t0x, t0z);
@@ -755,59 +764,75 @@ __device__ __forceinline__ T fd2NonUniform(int radius, const Spacing2<T> &g, con
     T sz = g.sinTheta * s0;
     T hxs0 = dx * s0;
     T hzs0 = dz * s0;
-    if (abs(src.isx - ix) > radius || abs(src.isz - iz) > radius) {
-        T t0a = huge;
-        T deta = hzs0 * hzs0 - dTz * dTz;
-        if (dTz >= 0 && deta >= 0 && dTz <= dz * sz) t0a = t1 + g.dx_dz * dsqrt(deta);
-        T t0b = huge;
-        T detb = hxs0 * hxs0 - dTx * dTx;
-        if (dTx >= 0 && detb >= 0 && dTx <= dx * sx) t0b = t3 + g.dz_dx * dsqrt(detb);
-        T t0Update2 = dmin(t0a, t0b);
-        T dxdz = g.cosTheta * g.sinTheta;
-        T tildeTx = t1 - t3 + t2;
-        T tildeTz = t3 - t1 + t2;
-        T dtCross = t1 - t3;
-        T detc = hxs0 * hxs0 + hzs0 * hzs0 - dtCross * dtCross;
-        T t0Update3 = huge;
-        if (dTx >= 0 && dTz >= 0 && detc > 0 && t1 < t3 + hzs0 && t3 < t1 + hxs0) {
-            t0Update3 = tildeTx * g.dz_dx + tildeTz * g.dx_dz + 2 * dsqrt(detc);
-            t0Update3 = dxdz * t0Update3;
-        }
-        if (t0Update3 < 0) t0Update3 = huge;
-        tUpd = dmin(dmin(t0Update1, t0Update2), t0Update3);
-    } else {
-        T t0Update3 = huge;
-        if (dTx >= 0 && dTz >= 0 && t1 < t3 + hzs0 && t3 < t1 + hxs0) {
-            const T sSrc = src.sSrc;
-            T dt0dx, dt0dz, t0;
-            analyticTG2(ix, iz, dx, dz, src.xs, src.zs, sSrc, t0, dt0dx, dt0dz);
-            T tau1 = t1 - analyticT2(ix + sg.ixShift, iz, dx, dz, src.xs, src.zs, sSrc);
-            T tau2 = t2 - analyticT2(ix + sg.ixShift, iz + sg.izShift, dx, dz, src.xs, src.zs, sSrc);
-            T tau3 = t3 - analyticT2(ix, iz + sg.izShift, dx, dz, src.xs, src.zs, sSrc);
-            dt0dx = sg.signX * dt0dx;
-            dt0dz = sg.signZ * dt0dz;
-            T tauX = tau1 - tau3 + tau2;
-            T tauZ = tau3 - tau1 + tau2;
-            const T one = 1, two = 2, four = 4;
-            T hx2inv = one / (dx * dx);
-            T hz2inv = one / (dz * dz);
-            T dxinv = one / dx;
-            T dzinv = one / dz;
-            T a = hx2inv + hz2inv;
-            T b = four * (dxinv * dt0dx + dzinv * dt0dz) - two * (tauX * hx2inv + tauZ * hz2inv);
-            T c = (tauX * tauX) * hx2inv + (tauZ * tauZ) * hz2inv -
-                  four * ((dt0dx * tauX) * dxinv + (dt0dz * tauZ) * dzinv) +
-                  four * (sSrc * sSrc - s0 * s0);
-            T det = b * b - four * a * c;
-            if (det >= 0) {
-                T tau = (-b + dsqrt(det)) / (two * a);
-                t0Update3 = t0 + tau;
-            }
-            if (t0Update3 < t1 || t0Update3 < t3) t0Update3 = huge;
-        }
-        tUpd = dmin(t0Update1, t0Update3);
+    T t0a = huge;
+    T deta = hzs0 * hzs0 - dTz * dTz;
+    if (dTz >= 0 && deta >= 0 && dTz <= dz * sz) t0a = t1 + g.dx_dz * dsqrt(deta);
+    T t0b = huge;
+    T detb = hxs0 * hxs0 - dTx * dTx;
+    if (dTx >= 0 && detb >= 0 && dTx <= dx * sx) t0b = t3 + g.dz_dx * dsqrt(detb);
+    T t0Update2 = dmin(t0a, t0b);
+    T dxdz = g.cosTheta * g.sinTheta;
+    T tildeTx = t1 - t3 + t2;
+    T tildeTz = t3 - t1 + t2;
+    T dtCross = t1 - t3;
+    T detc = hxs0 * hxs0 + hzs0 * hzs0 - dtCross * dtCross;
+    T t0Update3 = huge;
+    if (dTx >= 0 && dTz >= 0 && detc > 0 && t1 < t3 + hzs0 && t3 < t1 + hxs0) {
+        t0Update3 = tildeTx * g.dz_dx + tildeTz * g.dx_dz + 2 * dsqrt(detc);
+        t0Update3 = dxdz * t0Update3;
     }
-    return tUpd;
+    if (t0Update3 < 0) t0Update3 = huge;
+    return dmin(dmin(t0Update1, t0Update2), t0Update3);
+}
+template <class T>
+__device__ __forceinline__ T fd2NonUniformNear(const Spacing2<T> &g, const SourceT<T> &src, const SweepSigns &sg, int ix,
+                                               int iz, T s0, T s1, T s3, T t1, T t2, T t3) {
+    const T huge = static_cast<T>(1.e10);
+    const T dx = g.dx, dz = g.dz;
+    T t0x = t1 + dx * dmin(s0, s3);
+    T t0z = t3 + dz * dmin(s0, s1);
+    T t0Update1 = dmin(t0x, t0z);
+    T dTx = t3 - t2;
+    T dTz = t1 - t2;
+    T hxs0 = dx * s0;
+    T hzs0 = dz * s0;
+    T t0Update3 = huge;
+    if (dTx >= 0 && dTz >= 0 && t1 < t3 + hzs0 && t3 < t1 + hxs0) {
+        const T sSrc = src.sSrc;
+        T dt0dx, dt0dz, t0;
+        analyticTG2(ix, iz, dx, dz, src.xs, src.zs, sSrc, t0, dt0dx, dt0dz);
+        T tau1 = t1 - analyticT2(ix + sg.ixShift, iz, dx, dz, src.xs, src.zs, sSrc);
+        T tau2 = t2 - analyticT2(ix + sg.ixShift, iz + sg.izShift, dx, dz, src.xs, src.zs, sSrc);
+        T tau3 = t3 - analyticT2(ix, iz + sg.izShift, dx, dz, src.xs, src.zs, sSrc);
+        dt0dx = sg.signX * dt0dx;
+        dt0dz = sg.signZ * dt0dz;
+        T tauX = tau1 - tau3 + tau2;
+        T tauZ = tau3 - tau1 + tau2;
+        const T one = 1, two = 2, four = 4;
+        T hx2inv = one / (dx * dx);
+        T hz2inv = one / (dz * dz);
+        T dxinv = one / dx;
+        T dzinv = one / dz;
+        T a = hx2inv + hz2inv;
+        T b = four * (dxinv * dt0dx + dzinv * dt0dz) - two * (tauX * hx2inv + tauZ * hz2inv);
+        T c = (tauX * tauX) * hx2inv + (tauZ * tauZ) * hz2inv -
+              four * ((dt0dx * tauX) * dxinv + (dt0dz * tauZ) * dzinv) +
+              four * (sSrc * sSrc - s0 * s0);
+        T det = b * b - four * a * c;
+        if (det >= 0) {
+            T tau = (-b + dsqrt(det)) / (two * a);
+            t0Update3 = t0 + tau;
+        }
+        if (t0Update3 < t1 || t0Update3 < t3) t0Update3 = huge;
+    }
+    return dmin(t0Update1, t0Update3);
+}
+template <class T>
+__device__ __forceinline__ T fd2NonUniform(int radius, const Spacing2<T> &g, const SourceT<T> &src,
+                                           const SweepSigns &sg, int ix, int iz, T s0, T s1, T s3,
+                                           T t1, T t2, T t3) {
+    if (abs(src.isx - ix) > radius || abs(src.isz - iz) > radius) return fd2NonUniformFar(g, s0, s1, s3, t1, t2, t3);
+    return fd2NonUniformNear(g, src, sg, ix, iz, s0, s1, s3, t1, t2, t3);
 }
 
 }  // namespace eikx

@@ -1,4 +1,5 @@
-// Level-set fast-sweeping kernels (3D and 2D) for sm_103a.
+// Level-set fast-sweeping kernels for sm_103a: the node-step 3D kernel (eikx_options.sweep_kernel
+// = 1) and the 2D kernel of one block per field (2).
 //
 // One launch performs one sweep (one of the 8 / 4 orderings) over every field of a
 // batch.  The warp-block wavefront is described in wavefront.cuh; the per-node update
@@ -16,7 +17,6 @@ namespace {
 
 constexpr int HY3 = LY3 + 1, HZ3 = LZ3 + 1;          // ring plane incl. halo row/column
 constexpr int kPlane3 = HY3 * HZ3;
-constexpr int kPlane2 = LZ2 + 1;
 constexpr int kThreads = 32 * kWarpsPerBlock;
 
 template <class T> __device__ __forceinline__ T hugeT() { return static_cast<T>(1.e10); }
@@ -253,158 +253,6 @@ __global__ void __launch_bounds__(kThreads) sweep3Kernel(const Sweep3Args<T> a) 
     }
 }
 
-template <class T, bool UNIFORM>
-__global__ void __launch_bounds__(kThreads) sweep2Kernel(const Sweep2Args<T> a) {
-    extern __shared__ __align__(16) unsigned char smemRaw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int lz = lane;
-    T *tring = reinterpret_cast<T *>(smemRaw) + warp * (2 * kRing * kPlane2);
-    T *sring = tring + kRing * kPlane2;
-    const SolveState &st = a.st;
-    clearNext(st, a.buf);
-    if (ldVolatile(st.abortFlag)) return;
-    constexpr int W = Mail<T>::kWords;
-    const unsigned tag = *st.epoch + static_cast<unsigned>(a.sweepIndex);
-
-    const int fx = a.sweep & 1, fz = (a.sweep >> 1) & 1;
-    SweepSigns sg;
-    sg.ixShift = fx ? 1 : -1; sg.iyShift = 0; sg.izShift = fz ? 1 : -1;
-    sg.signX = fx ? -1 : 1; sg.signY = 1; sg.signZ = fz ? -1 : 1;
-    const int Px = a.pitch;
-    const int nSteps = Px + LZ2 - 1;
-    const T *sp = fx ? a.spNeg : a.spPos;
-    const T huge = hugeT<T>();
-    const int myslot = lz + 1;
-    const long long faceWords = static_cast<long long>(Px) * W;
-
-    while (true) {
-        unsigned q = 0;
-        if (lane == 0) q = atomicAdd(st.queue[a.buf], 1u);
-        q = __shfl_sync(kFull, q, 0);
-        if (q >= static_cast<unsigned>(st.totalItems)) break;
-        const int4 item = st.order[q];
-        const int f = item.x, c = item.z;
-        if (st.converged[f]) continue;
-        const SourceT<T> src = a.srcs[f];
-        const int z0 = c * LZ2;
-        const int zp = z0 + lz;
-        const bool laneValid = zp < a.nz;
-        const int za = laneValid ? reflect(zp, a.nz, fz) : 0;
-        int xlo, xhi, zlo, zhi;
-        axisBounds(a.nx, fx, a.init, src.isx, xlo, xhi);
-        axisBounds(a.nz, fz, a.init, src.isz, zlo, zhi);
-        const bool zUpd = laneValid && za >= zlo && za <= zhi;
-        T *field = a.tt + static_cast<long long>(f) * a.fieldStride;
-        T *row = field + static_cast<long long>(za) * a.pitch;
-        RowStream<T> rs;
-        rs.row = row;
-        rs.srow = sp + static_cast<long long>(za + (fz ? 0 : 1)) * a.spPitch;
-        rs.Px = Px;
-        rs.rev = fx;
-        rs.nChunks = Px / RowStream<T>::V;
-        if (laneValid) rs.start();
-        const long long tileId = static_cast<long long>(f) * a.tilesZ + c;
-        unsigned long long *face = st.mbox + tileId * faceWords;   // written by lane LZ2-1
-        // lane 0 also stands in for the virtual lane z' = z0 - 1 (row LZ2-1 of block c-1)
-        const bool vValid = (lane == 0) && c > 0;
-        const unsigned long long *vbox = st.mbox + (tileId - (c > 0 ? 1 : 0)) * faceWords;
-        const int vza = vValid ? reflect(z0 - 1, a.nz, fz) : 0;
-        const T *vsrow = sp + static_cast<long long>(vza + (fz ? 0 : 1)) * a.spPitch;
-
-        // Halo pipeline as in the 3D kernel: lane 0 stands in for the virtual lane, whose
-        // value at step sv is node x' = sv + 1 of the upstream block's last row.
-        auto haloValid = [&](int xv) { return vValid && xv >= 0 && xv < Px; };
-        auto haloStore = [&](int sv, T tv, T svv) {
-            const int slot = (sv & (kRing - 1)) * kPlane2;
-            tring[slot] = tv;
-            sring[slot] = svv;
-        };
-        auto fillNow = [&](int sv) -> bool {
-            bool good = true;
-            if (lane == 0) {
-                const int xv = sv + 1;
-                T tv = huge, svv = huge;
-                if (haloValid(xv)) {
-                    good = Mail<T>::get(vbox + static_cast<long long>(xv) * W, tag, tv, st.abortFlag, st.spinLimit);
-                    svv = vsrow[fx ? Px - 1 - xv : xv + RowStream<T>::V];
-                }
-                haloStore(sv, tv, svv);
-            }
-            return __all_sync(kFull, good);
-        };
-        MailSlot<T> mslot[kPref];
-        T sslot[kPref];
-        auto issue = [&](int j, int sv) {
-            const int xv = sv + 1;
-            if (lane == 0 && haloValid(xv)) {
-                mslot[j].issue(vbox + static_cast<long long>(xv) * W);
-                sslot[j] = vsrow[fx ? Px - 1 - xv : xv + RowStream<T>::V];
-            }
-        };
-        auto consume = [&](int j, int sv) -> bool {
-            bool good = true;
-            if (lane == 0) {
-                const int xv = sv + 1;
-                T tv = huge, svv = huge;
-                if (haloValid(xv)) {
-                    good = mslot[j].take(vbox + static_cast<long long>(xv) * W, tag, tv, st.abortFlag, st.spinLimit);
-                    svv = sslot[j];
-                }
-                haloStore(sv, tv, svv);
-            }
-            return __all_sync(kFull, good);
-        };
-
-        bool ok = fillNow(-1);
-#pragma unroll
-        for (int j = 0; j < kPref; ++j) issue(j, j);
-        T res = 0;
-        for (int s0 = 0; s0 < nSteps && ok; s0 += kPref) {
-#pragma unroll
-            for (int j = 0; j < kPref; ++j) {
-                const int s = s0 + j;
-                if (!ok || s >= nSteps) continue;
-                ok = consume(j, s);
-                if (!ok) continue;
-                issue(j, s + kPref);
-                const int xp = s - lz;
-                const bool active = laneValid && xp >= 0 && xp < Px;
-                const int xa = reflect(xp, Px, fx);
-                T t0 = huge, sOwn = huge;
-                if (active) rs.take(xp, t0, sOwn);
-                const int cur = (s & (kRing - 1)) * kPlane2;
-                const int p1 = ((s - 1) & (kRing - 1)) * kPlane2;
-                const int p2 = ((s - 2) & (kRing - 1)) * kPlane2;
-                sring[cur + myslot] = sOwn;
-                __syncwarp();
-                const T t1 = tring[p1 + myslot];
-                const T t3 = tring[p1 + myslot - 1];
-                const T t2 = tring[p2 + myslot - 1];
-                const T s0 = sring[p2 + myslot - 1];
-                const T s1 = sring[p1 + myslot - 1];
-                const T s3 = sring[p1 + myslot];
-                T v = t0;
-                if (active && zUpd && xa >= xlo && xa <= xhi) {
-                    const T tu = UNIFORM ? fd2Uniform<T>(a.radius, a.h, src, sg, xa, za, s0, s1, s3, t1, t2, t3)
-                                         : fd2NonUniform<T>(a.radius, a.sp2, src, sg, xa, za, s0, s1, s3, t1, t2, t3);
-                    if (tu < t0) {
-                        v = tu;
-                        row[xa] = tu;
-                        res = dmax(res, t0 - tu);
-                    }
-                }
-                tring[cur + myslot] = v;
-                if (active && lz == LZ2 - 1) Mail<T>::put(face + static_cast<long long>(xp) * W, tag, v);
-            }
-        }
-        if (!ok) break;
-        const double r = warpMax(static_cast<double>(res));
-        if (lane == 0 && r > 0)
-            atomicMax(st.residual + static_cast<long long>(f) * st.residualStride + a.residualSlot,
-                      static_cast<unsigned long long>(__double_as_longlong(r)));
-    }
-}
-
 // One CTA per field for 2D grids of up to 512 rows (sweep2BlockKernel): thread z' owns
 // row z' and updates x' = s - z' at step s; the only upwind value from another thread is
 // the row above's result of the step before, passed through shared memory with one
@@ -501,21 +349,12 @@ __global__ void __launch_bounds__(512) sweep2BlockKernel(const Sweep2Args<T> a) 
 }  // namespace
 
 size_t sweep3SmemBytes(size_t elem) { return elem * 2 * kRing * kPlane3 * kWarpsPerBlock; }
-size_t sweep2SmemBytes(size_t elem) { return elem * 2 * kRing * kPlane2 * kWarpsPerBlock; }
 
 template <class T>
 cudaError_t launchSweep3(const Sweep3Args<T> &a, bool uniform, int blocks, cudaStream_t s) {
     const size_t smem = sweep3SmemBytes(sizeof(T));
     if (uniform) sweep3Kernel<T, true><<<blocks, kThreads, smem, s>>>(a);
     else sweep3Kernel<T, false><<<blocks, kThreads, smem, s>>>(a);
-    return cudaGetLastError();
-}
-
-template <class T>
-cudaError_t launchSweep2(const Sweep2Args<T> &a, bool uniform, int blocks, cudaStream_t s) {
-    const size_t smem = sweep2SmemBytes(sizeof(T));
-    if (uniform) sweep2Kernel<T, true><<<blocks, kThreads, smem, s>>>(a);
-    else sweep2Kernel<T, false><<<blocks, kThreads, smem, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -537,21 +376,9 @@ template <class T> int sweep3BlocksPerSM(bool uniform) {
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep3Kernel<T, false>, kThreads, smem);
     return n > 0 ? n : 1;
 }
-template <class T> int sweep2BlocksPerSM(bool uniform) {
-    int n = 0;
-    const size_t smem = sweep2SmemBytes(sizeof(T));
-    if (uniform) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep2Kernel<T, true>, kThreads, smem);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep2Kernel<T, false>, kThreads, smem);
-    return n > 0 ? n : 1;
-}
-
 template cudaError_t launchSweep3<float>(const Sweep3Args<float> &, bool, int, cudaStream_t);
 template cudaError_t launchSweep3<double>(const Sweep3Args<double> &, bool, int, cudaStream_t);
-template cudaError_t launchSweep2<float>(const Sweep2Args<float> &, bool, int, cudaStream_t);
-template cudaError_t launchSweep2<double>(const Sweep2Args<double> &, bool, int, cudaStream_t);
 template int sweep3BlocksPerSM<float>(bool);
 template int sweep3BlocksPerSM<double>(bool);
-template int sweep2BlocksPerSM<float>(bool);
-template int sweep2BlocksPerSM<double>(bool);
 
 }  // namespace eikx

@@ -9,8 +9,6 @@ namespace eikx {
 
 // Warp-block shape of the 3D kernel: LY3 x LZ3 x-pencils per warp.
 constexpr int LY3 = 8, LZ3 = 4;
-// 2D kernel: 32 x-rows per warp.
-constexpr int LZ2 = 32;
 constexpr int kWarpsPerBlock = 4;
 
 // Device state shared by all sweeps of one solve (one entry per field unless noted).
@@ -101,13 +99,19 @@ template <class T> struct Sweep2Args {
     int radius;
     T h;
     Spacing2<T> sp2;
+    const T *hsPos, *hsNeg;   // FP64 wave-step kernel on a uniform grid: the copies multiplied by h
 };
 
 // Launchers (sweep.cu).  blocks = persistent grid size.
 template <class T>
 cudaError_t launchSweep3(const Sweep3Args<T> &a, bool uniform, int blocks, cudaStream_t s);
+// Wave-step 2D kernel (sweep_wave2.cu): warp blocks of kWaveRows2 z'-rows from the first updated
+// one on, waveStepCap2(Px) steps of one value per block in the mailbox.
+constexpr int kWaveRows2 = 32;
+__host__ __device__ constexpr int waveStepCap2(int Px) { return Px + 80; }
 template <class T>
-cudaError_t launchSweep2(const Sweep2Args<T> &a, bool uniform, int blocks, cudaStream_t s);
+cudaError_t launchSweep2Wave(const Sweep2Args<T> &a, bool uniform, int blocks, cudaStream_t s);
+template <class T> int sweep2WaveBlocksPerSM(bool uniform);
 // 2D grids of at most kMaxBlockRows2 rows: one CTA per field, one thread per row.
 constexpr int kMaxBlockRows2 = 512;
 template <class T>
@@ -168,9 +172,7 @@ int sweep3PairBlocksPerSM();
 size_t sweep3PairSmemBytes();
 // Resident blocks per SM of the sweep kernels (for the persistent grid size).
 template <class T> int sweep3BlocksPerSM(bool uniform);
-template <class T> int sweep2BlocksPerSM(bool uniform);
 size_t sweep3SmemBytes(size_t elem);
-size_t sweep2SmemBytes(size_t elem);
 
 // Field kernels (fields.cu).
 struct Corner3 {
@@ -190,7 +192,7 @@ template <class T, class U>
 cudaError_t launchPadSlowness3(T *sp, int spPitch, int shift, const U *s, int nx, int ny, int nz,
                                cudaStream_t st, T h = 0);
 template <class T, class U>
-cudaError_t launchPadSlowness2(T *sp, int spPitch, int shift, const U *s, int nx, int nz, cudaStream_t st);
+cudaError_t launchPadSlowness2(T *sp, int spPitch, int shift, const U *s, int nx, int nz, cudaStream_t st, T h = 0);
 template <class U>
 cudaError_t launchNodalToCell3(double *slow, const U *v, int nx, int ny, int nz, int ordering,
                                cudaStream_t s);

@@ -1,5 +1,6 @@
-"""The wave-step 3D kernel (the default on uniform grids) at the edges of its 8 x 4 warp block, of
-its 4-node ring chunks and of its group of four steps, against the oracle, bit for bit."""
+"""The wave-step kernels (the 3D default on uniform grids, the 2D default) at the edges of their
+warp blocks (8 x 4 rows, 32 rows), of their 4-node ring chunks and of their groups of four steps,
+against the oracle, bit for bit."""
 import numpy as np
 import pytest
 
@@ -36,4 +37,31 @@ def test_wave_step_block_edges_match_the_oracle(ctx, oracle, grid, precision, ne
     for p, a in zip(pos, t):
         cell = [min(n - 2, int(q / h)) for q, n in zip(p, grid)]
         ref = oracle.solve3d(s, (nx, ny, nz, h, h, h), cell, p, n_sweeps=3, radius=2, tol=1e-6, near_fp64=near)
+        assert np.array_equal(_bits(a), _bits(ref)), (p, np.abs(a - ref).max())
+
+
+# rows from the first updated one: nz - 1 = 31, 32, 33, 65 straddle the 32-row block; h = 0.01
+# (kilometres) makes the cell-edge operators t1 + h sqrt(.) the smallest ones, h = 10 the others
+GRIDS2 = [(3, 32), (4, 33), (5, 34), (6, 66), (33, 33), (34, 34), (61, 40)]
+
+
+@pytest.mark.parametrize("precision", [ex.F32, ex.F64])
+@pytest.mark.parametrize("spacing", [(10.0, 10.0), (0.01, 0.01), (10.0, 12.5)])
+@pytest.mark.parametrize("grid", GRIDS2)
+def test_wave_step_2d_block_edges_match_the_oracle(ctx, oracle, grid, spacing, precision):
+    nx, nz = grid
+    dx, dz = spacing
+    rng = np.random.default_rng(nx * 100 + nz)
+    dt = np.float32 if precision == ex.F32 else np.float64
+    s = random_slowness(rng, (nz - 1) * (nx - 1), dtype=dt)
+    if dx < 1:
+        s = (s * 1000).astype(dt)
+    ctx.set_grid2d(nx, nz, dx, dz)
+    ctx.set_slowness2d(s)
+    ends = np.array([(nx - 1) * dx, (nz - 1) * dz])
+    pos = np.concatenate([[[0.0, 0.0], ends], rng.uniform(0, 1, (3, 2)) * ends])
+    t = ctx.solve2d(pos, ex.Options(n_sweeps=3, tolerance=1e-9, factored_radius=2), precision)
+    for p, a in zip(pos, t):
+        cell = [min(n - 2, int(q / d)) for q, n, d in zip(p, grid, spacing)]
+        ref = oracle.solve2d(s, (nx, nz, dx, dz), cell, p, n_sweeps=3, radius=2, tol=1e-9)
         assert np.array_equal(_bits(a), _bits(ref)), (p, np.abs(a - ref).max())
