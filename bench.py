@@ -359,7 +359,7 @@ def run_gpu(args):
     peak, peak_kind = _peaks()
     tr = _traffic()
     shapes = {1: "8x4", 2: "4x8", 3: "16x2"}
-    # the default on a uniform grid is the wave-step kernel, which a tuning entry reports as the
+    # the default is the wave-step kernel, which a tuning entry reports as the
     # choice whose time is the default's
     wave = KERNEL[0] == 0 and not PAIR[0] and (not tuning or tuning["ms_per_sweep"] == tuning["default_ms_per_sweep"])
     if wave:

@@ -166,8 +166,8 @@ struct TuneKey {
         return std::tie(precision, uniform, nx, ny, nz, nsrc) < std::tie(o.precision, o.uniform, o.nx, o.ny, o.nz, o.nsrc);
     }
 };
-// A tuning entry: the reported choice, and whether it is the default step kernel of the class
-// (wave-step), which eikx_tuning has no value for (it then reads chunk-step, 8x4).
+// A tuning entry: the reported choice, and whether it is the default kernel (wave-step), which
+// eikx_tuning has no value for (it then reads chunk-step, 8x4).
 struct Tuned {
     eikx_tuning t{};
     bool wave = false;
@@ -501,7 +501,7 @@ eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std
     st.totalItems = nProgress - drop;
     const int spinLog2 = o.spin_limit_log2 > 0 ? std::min(o.spin_limit_log2, 40) : 22;
     st.spinLimit = 1ull << spinLog2;
-    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(false, near64)
+    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, false, near64)
                        : eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
     const int blocks = std::max(1, std::min(c->numSMs * perSM, (nProgress + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock));
@@ -604,11 +604,11 @@ eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std
             a.srcs64 = near64 ? w.srcs64.as<eikx::SourceFp64>() : nullptr;
             a.slots = w.slots.as<int2>();
             a.initSweeps = initSweeps;
-            if (wave || (uniform && sizeof(T) == 8)) {
+            if (uniform && (wave || sizeof(T) == 8)) {
                 a.hsPos = shad[0].as<T>(); a.hsNeg = shad[1].as<T>();
                 a.cells = c->slow3.p; a.cells64 = 1;
             }
-            if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, blocks, c->stream));
+            if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, uniform, blocks, c->stream));
             else EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
             EIKX_CUDA(eikx::launchCheckStream(st, w.slots.as<int2>(), S, sweepsRun, initSweeps, o.tolerance, c->stream));
             if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * profiled + 1], c->stream));
@@ -827,8 +827,8 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     }
     // FP32 uniform 3D batches run two fields per lane (the paired kernel) on request
     const bool paired = DIM == 3 && P == EIKX_F32 && uniform && nSrc >= 2 && o.pair_fields;
-    // the default on uniform grids is the wave-step kernel; a warp-block shape asks for chunk-step
-    const bool wave = DIM == 3 && uniform && !paired &&
+    // the default is the wave-step kernel; a warp-block shape asks for chunk-step
+    const bool wave = DIM == 3 && !paired &&
                         (o.sweep_kernel == eikx::kWaveStep || (o.sweep_kernel == 0 && o.block_shape == 0));
     const int variant = wave ? eikx::kWaveStep : o.sweep_kernel == eikx::kNodeStep ? eikx::kNodeStep : eikx::kChunkStep;
     const bool chunkStep = DIM == 3 && !paired && variant == eikx::kChunkStep;
@@ -976,7 +976,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
 
     int perSM = paired ? eikx::sweep3PairBlocksPerSM()
                 : DIM == 2 ? eikx::sweep2WaveBlocksPerSM<T>(uniform)
-                : wave ? eikx::sweep3WaveBlocksPerSM<T>(false, !srcT64.empty())
+                : wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, false, !srcT64.empty())
                 : chunkStep ? eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape)
                             : eikx::sweep3BlocksPerSM<T>(uniform);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
@@ -1064,7 +1064,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                 a.sweepIndex = sweepsLaunched;
                 a.sweep = e; a.init = init; a.radius = o.factored_radius; a.h = static_cast<T>(dx);
                 a.srcs64 = srcs64;
-                if (wave || (uniform && sizeof(T) == 8)) {
+                if (uniform && (wave || sizeof(T) == 8)) {
                     a.hsPos = shad[0].as<T>(); a.hsNeg = shad[1].as<T>();
                     a.cells = c->slow3.p; a.cells64 = 1;
                 }
@@ -1088,7 +1088,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                     }
                 }
                 if (!done) {
-                    if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, blocks, c->stream));
+                    if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, uniform, blocks, c->stream));
                     else if (chunkStep) EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
                     else EIKX_CUDA(eikx::launchSweep3<T>(a, uniform, blocks, c->stream));
                 }
@@ -1333,8 +1333,8 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     BatchWorkspace &w = c->bw;
     constexpr int V = 16 / sizeof(T);
     const int shape = o.block_shape > 0 ? o.block_shape - 1 : eikx::kShape8x4;
-    const bool wave = uniform && o.sweep_kernel == 0 && o.block_shape == 0;   // as solveImpl
-    const int nCopies = wave ? 4 : 2;   // padded slowness copies: shifted, unshifted, then both times h
+    const bool wave = o.sweep_kernel == 0 && o.block_shape == 0;   // as solveImpl
+    const int nCopies = wave && uniform ? 4 : 2;   // padded slowness copies: shifted, unshifted, then both times h
     const int nM = static_cast<int>(sel.size());
     struct Layout {
         int nx, ny, nz, Px, spPitch, tilesY, tilesZ, firstUnit, nSrc;
@@ -1482,8 +1482,8 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
             gu.tt = ttBase + l.ttOff + static_cast<size_t>(j) * l.fieldStride;
             gu.spPos = spBase + l.spOff;
             gu.spNeg = spBase + l.spOff + l.spElems;
-            gu.hsPos = wave ? spBase + l.spOff + 2 * l.spElems : nullptr;
-            gu.hsNeg = wave ? spBase + l.spOff + 3 * l.spElems : nullptr;
+            gu.hsPos = nCopies == 4 ? spBase + l.spOff + 2 * l.spElems : nullptr;
+            gu.hsNeg = nCopies == 4 ? spBase + l.spOff + 3 * l.spElems : nullptr;
             gu.mbox = mbBase + l.mboxOff + static_cast<size_t>(j) * l.tilesY * l.tilesZ * l.faceWords;
             gu.spPlane = l.spPlane;
             gu.spPitch = l.spPitch;
@@ -1579,7 +1579,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     st.totalItems = static_cast<int>(nItems);
     const int spinLog2 = o.spin_limit_log2 > 0 ? std::min(o.spin_limit_log2, 40) : 22;
     st.spinLimit = 1ull << spinLog2;
-    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(true, near64)
+    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, true, near64)
                        : eikx::sweep3ChunkBlocksPerSM<T>(uniform, true, shape);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
     const int blocks = std::max(1, static_cast<int>(std::min<size_t>(
@@ -1635,7 +1635,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
             a.sweep = e; a.init = init; a.radius = o.factored_radius;
             a.units = w.units.as<eikx::Grid3Unit<T>>();
             a.srcs64 = near64 ? w.srcs64.as<eikx::SourceFp64>() : nullptr;
-            if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, blocks, c->stream));
+            if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, uniform, blocks, c->stream));
             else EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
             if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * sweepsLaunched + 1], c->stream));
             buf ^= 1;
@@ -1806,8 +1806,8 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
         o.blocks_per_sm = perSM;
         cands.push_back(o);
     };
-    // the untuned default first: wave-step on uniform grids, else chunk-step 8x4
-    if (uniform) add(eikx::kWaveStep, 0, 0, eikx::sweep3WaveBlocksPerSM<T>(false, false));
+    // the untuned default first: wave-step
+    add(eikx::kWaveStep, 0, 0, eikx::sweep3WaveBlocksPerSM<T>(uniform, false, false));
     for (int shape = 0; shape < eikx::kNumShapes; ++shape) {
         const int mx = eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape);
         add(eikx::kChunkStep, 0, shape + 1, mx);

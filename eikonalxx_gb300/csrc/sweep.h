@@ -71,8 +71,7 @@ template <class T> struct Sweep3Args {
     // stream and `sweep` its ordering (sweepIndex mod 8).
     const int2 *slots;
     int initSweeps;           // 1 = a slot's first 8 sweeps are its initialisation pass
-    // Wave-step kernel, and FP64 chunk-step kernel on a uniform grid, one model (required
-    // there): the padded slowness copies multiplied by h (launchPadSlowness3 with h), laid out
+    // Uniform grids, one model: wave-step kernel and FP64 chunk-step kernel (required there): the padded slowness copies multiplied by h (launchPadSlowness3 with h), laid out
     // as spPos / spNeg; for the latter's factored branch also the model's natural-order cell
     // slowness (FP64 cells, or FP32 cells with cells64 = 0)
     const T *hsPos, *hsNeg;
@@ -144,15 +143,15 @@ template <class T> inline int sweep3ChunkBlocksPerSM(bool uniform, bool batch, i
     return sweep3ChunkBlocksPerSM_8x4<T>(uniform, batch);
 }
 // 3D sweep kernel variants (eikx_options.sweep_kernel; kWaveStep is not a value of the
-// option: it is what the default takes on uniform grids).
+// option: it is what the default takes).
 enum Sweep3Variant { kNodeStep = 1, kChunkStep = 2, kWaveStep = 3 };
-// Wave-step 3D kernel (sweep_wave.cu, uniform grids): a warp owns kWaveLY y'-rows x kWaveLZ
+// Wave-step 3D kernel (sweep_wave.cu): a warp owns kWaveLY y'-rows x kWaveLZ
 // z'-rows, the blocks starting at the first updated rows; its mailbox holds waveStepCap(Px)
 // steps of kWaveLY + kWaveLZ values per block.
 constexpr int kWaveLY = 8, kWaveLZ = 4;
 __host__ __device__ constexpr int waveStepCap(int Px) { return Px + 32; }
-template <class T> cudaError_t launchSweep3Wave(const Sweep3Args<T> &a, int blocks, cudaStream_t s);
-template <class T> int sweep3WaveBlocksPerSM(bool batch, bool near64);
+template <class T> cudaError_t launchSweep3Wave(const Sweep3Args<T> &a, bool uniform, int blocks, cudaStream_t s);
+template <class T> int sweep3WaveBlocksPerSM(bool uniform, bool batch, bool near64);
 // Warp blocks of one field, and the mailbox words each needs.
 struct Tiling3 {
     int ly, lz, tilesY, tilesZ;

@@ -71,10 +71,9 @@ typedef struct {
                               size (the paired kernel needs 168 registers per thread, which
                               leaves 12 resident warps per SM).  Both give identical times. */
     int sweep_kernel;      /* 3D sweep kernel: 0 (default) = the tuned kernel of this grid class
-                              if eikx_autotune3d ran, else wave-step on uniform grids (a lane
-                              updates one node per wavefront step, rows through a
-                              shared-memory ring) unless block_shape asks for chunk-step,
-                              and chunk-step on others; 1 = node-step (the earlier kernel of
+                              if eikx_autotune3d ran, else wave-step (a lane updates one node
+                              per wavefront step, rows through a shared-memory ring) unless
+                              block_shape asks for chunk-step; 1 = node-step (the earlier kernel of
                               one node per lane and step), 2 = chunk-step (a lane updates one
                               16-byte chunk, 4 FP32 / 2 FP64 nodes, per step).  2D: 0 and 1 =
                               wave-step warp blocks of 32 rows; 2 = one CTA per field, one
@@ -276,7 +275,7 @@ eikx_status eikx_trace_rays2d(eikx_ctx *ctx, int nx, int nz, double dx, double d
 /* The configuration eikx_autotune3d chose for one grid class. */
 typedef struct {
     int sweep_kernel;              /* 1 = node-step, 2 = chunk-step; where the untuned default
-                                      of a uniform grid (wave-step, no value here) is the
+                                      (wave-step, no value here) is the
                                       fastest, 2 with block_shape 1 and ms_per_sweep equal to
                                       default_ms_per_sweep */
     int pair_fields;               /* 1 = two FP32 fields per lane */

@@ -1,4 +1,4 @@
-"""The wave-step kernels (the 3D default on uniform grids, the 2D default) at the edges of their
+"""The wave-step kernels (the 3D and 2D defaults) at the edges of their
 warp blocks (8 x 4 rows, 32 rows), of their 4-node ring chunks and of their groups of four steps,
 against the oracle, bit for bit."""
 import numpy as np
@@ -21,22 +21,22 @@ GRIDS = [(3, 8, 4), (4, 9, 5), (5, 10, 6), (6, 18, 10), (31, 9, 10), (32, 10, 5)
 
 
 @pytest.mark.parametrize("precision,near", [(ex.F32, False), (ex.F32, True), (ex.F64, False)])
+@pytest.mark.parametrize("spacing", [(50.0, 50.0, 50.0), (50.0, 65.0, 8.0)])
 @pytest.mark.parametrize("grid", GRIDS)
-def test_wave_step_block_edges_match_the_oracle(ctx, oracle, grid, precision, near):
+def test_wave_step_block_edges_match_the_oracle(ctx, oracle, grid, spacing, precision, near):
     nx, ny, nz = grid
-    h = 50.0
     rng = np.random.default_rng(nx * 100 + ny * 10 + nz)
     dt = np.float32 if precision == ex.F32 else np.float64
     s = random_slowness(rng, (nz - 1) * (ny - 1) * (nx - 1), dtype=dt)
-    ctx.set_grid3d(nx, ny, nz, h, h, h)
+    ctx.set_grid3d(nx, ny, nz, *spacing)
     ctx.set_slowness3d(s)
-    ends = np.array([(nx - 1) * h, (ny - 1) * h, (nz - 1) * h])
+    ends = (np.array(grid) - 1) * spacing
     pos = np.concatenate([[[0.0, 0.0, 0.0], ends], rng.uniform(0, 1, (4, 3)) * ends])
     opt = ex.Options(n_sweeps=3, tolerance=1e-6, factored_radius=2, near_fp64=near)
     t = ctx.solve3d(pos, opt, precision)
     for p, a in zip(pos, t):
-        cell = [min(n - 2, int(q / h)) for q, n in zip(p, grid)]
-        ref = oracle.solve3d(s, (nx, ny, nz, h, h, h), cell, p, n_sweeps=3, radius=2, tol=1e-6, near_fp64=near)
+        cell = [min(n - 2, int(q / h)) for q, n, h in zip(p, grid, spacing)]
+        ref = oracle.solve3d(s, (nx, ny, nz, *spacing), cell, p, n_sweeps=3, radius=2, tol=1e-6, near_fp64=near)
         assert np.array_equal(_bits(a), _bits(ref)), (p, np.abs(a - ref).max())
 
 
