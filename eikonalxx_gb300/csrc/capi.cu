@@ -101,6 +101,31 @@ cudaError_t checkAfterSweep(const eikx::SolveState &st, int nFields, int nSweepK
                                         j >= nSweepKinds - 1 ? tol : -1.0, s);
 }
 
+// Whether a solve takes both orderings of a pair in one wave-step launch, for `items` warp blocks
+// (of all fields) on `warps` resident warps.  The second ordering starts in blocks that the first
+// is done with, so a pair costs one way through the blocks, not two: 256 x 256 x 128 nodes, us a
+// refinement sweep, one by one and both: 1 field (0.4 blocks a warp) 390, 274; 4 fields 526, 388;
+// 8 fields (3.4) 618, 540; 16 fields (6.7) 899, 882; 32 fields (13.5) 1546, 1578; 64 fields 2899,
+// 2985.  In double, 200 x 200 x 100: 4 fields (2.1) 2293, 1515; 32 fields (16) 5796, 5462.  With
+// many blocks a warp the way through them no longer counts, and the loop over the passes costs
+// 3 %.  The mailbox doubles, so the line also bounds that.
+bool bothSweeps(bool wave, size_t items, size_t warps) { return wave && items <= 10 * warps; }
+// The eight sweeps of a pass (initialisation, or a refinement iteration) as launches of pairs:
+// sweep(ordering, init, slot, mode) and check(refinement sweep, second).
+template <class Sweep, class Check>
+eikx_status sweepPairs(int pass, bool init, Sweep sweep, Check check) {
+    const int slot = 8 * pass, r0 = slot - 8;
+    for (int e = 0; e < 8; e += 2) {
+        if (eikx_status r = sweep(e, init ? 1 : 0, slot + e, eikx::kBothSweeps); r != EIKX_OK) return r;
+        if (init) continue;
+        if (eikx_status r = check(r0 + e, false); r != EIKX_OK) return r;
+        if (r0 + e < 8) continue;   // no field holds a sweep back before the ninth
+        if (eikx_status r = sweep(e + 1, 0, slot + e + 1, eikx::kSecondSweep); r != EIKX_OK) return r;
+        if (eikx_status r = check(r0 + e, true); r != EIKX_OK) return r;
+    }
+    return EIKX_OK;
+}
+
 // The host's copy of a workspace's sweep-tag base.  The device's reset kernel advances the
 // base by the previous solve's tag count at the start of every solve; the host repeats that
 // step and, before a solve whose 32-bit tags would wrap (and so could meet words an early
@@ -862,7 +887,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
 
     // workspace
     eikx::Tiling3 tl{1, eikx::kWaveRows2, 1, (nz - 1 + eikx::kWaveRows2 - 1) / eikx::kWaveRows2,
-                     static_cast<long long>(eikx::waveStepCap2(Px)) * (sizeof(T) / 4)};
+                     static_cast<long long>(eikx::waveStepCap2(Px)) * static_cast<int>(sizeof(T) / 4)};
     if (DIM == 3) tl = eikx::tiling3<T>(wave, shape, Px, ny, nz);
     if (paired) tl.faceWords *= 2;   // the two fields' values
     const int ly = tl.ly, lz = tl.lz, tilesY = tl.tilesY, tilesZ = tl.tilesZ;
@@ -871,8 +896,17 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     const int nSweeps = std::max(0, o.n_sweeps);
     const int resStride = nSweepKinds * (1 + nSweeps);
     Workspace &w = c->ws;
+    int perSM = paired ? eikx::sweep3PairBlocksPerSM()
+                : DIM == 2 ? eikx::sweep2WaveBlocksPerSM<T>(uniform)
+                : wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, false, !srcT64.empty())
+                : chunkStep ? eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape)
+                            : eikx::sweep3BlocksPerSM<T>(uniform);
+    if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
+    int blocks = std::min(c->numSMs * perSM, (nProgress + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock);
+    blocks = std::max(blocks, 1);
+    const bool both = bothSweeps(wave, nProgress, static_cast<size_t>(c->numSMs) * perSM * eikx::kWarpsPerBlock);
     const size_t ttBytes = static_cast<size_t>(fieldStride) * nSrc * sizeof(T);
-    const size_t mboxBytes = static_cast<size_t>(nProgress) * tl.faceWords * 8;
+    const size_t mboxBytes = static_cast<size_t>(nProgress) * tl.faceWords * 8 * (both ? 2 : 1);
     const void *before[] = {w.tt.p, w.mbox.p, w.epoch.p, w.residual.p, w.converged.p,
                             w.iterations.p, w.order.p, w.srcs.p, w.corners.p, w.srcs64.p, w.factor.p};
     EIKX_CUDA(w.tt.ensure(ttBytes));
@@ -887,7 +921,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     }
     EIKX_CUDA(w.queue.ensure(2 * sizeof(unsigned)));
     EIKX_CUDA(w.residual.ensure(static_cast<size_t>(nSrc) * resStride * 8));
-    EIKX_CUDA(w.converged.ensure(static_cast<size_t>(nSrc) * 4));
+    EIKX_CUDA(w.converged.ensure(static_cast<size_t>(nSrc) * 8));   // and the pair states
     EIKX_CUDA(w.iterations.ensure(static_cast<size_t>(nSrc) * 4));
     EIKX_CUDA(w.abortFlag.ensure(sizeof(int)));
     EIKX_CUDA(w.order.ensure(static_cast<size_t>(nProgress) * 16));
@@ -965,6 +999,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     st.residual = w.residual.as<unsigned long long>();
     st.residualStride = resStride;
     st.converged = w.converged.as<int>();
+    st.pairState = w.converged.as<int>() + nSrc;
     st.sweepsRun = w.iterations.as<int>();
     st.abortFlag = w.abortFlag.as<int>();
     // test hook: leave the first blocks of the queue out (their dependants time out)
@@ -973,15 +1008,6 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     st.totalItems = nProgress - drop;
     const int spinLog2 = o.spin_limit_log2 > 0 ? std::min(o.spin_limit_log2, 40) : 22;
     st.spinLimit = 1ull << spinLog2;
-
-    int perSM = paired ? eikx::sweep3PairBlocksPerSM()
-                : DIM == 2 ? eikx::sweep2WaveBlocksPerSM<T>(uniform)
-                : wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, false, !srcT64.empty())
-                : chunkStep ? eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape)
-                            : eikx::sweep3BlocksPerSM<T>(uniform);
-    if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
-    int blocks = std::min(c->numSMs * perSM, (nProgress + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock);
-    blocks = std::max(blocks, 1);
 
     // Host output: a field that has converged is not written again, so it is copied out on
     // a second stream at the end of the iteration in which it converged, while the sweeps
@@ -1005,7 +1031,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     sk.nSweeps = nSweeps; sk.radius = o.factored_radius; sk.initSweeps = o.init_sweeps ? 1 : 0;
     sk.initFp64 = o.init_fp64 ? 1 : 0; sk.uniform = uniform; sk.blocks = blocks; sk.tol = o.tolerance;
     sk.h = dx; sk.dx = dx; sk.dy = dy; sk.dz = dz; sk.spin = st.spinLimit; sk.dropBlocks = drop;
-    sk.paired = paired ? 1 : 0;
+    sk.paired = paired ? 1 : both ? 2 : 0;
     sk.warm = warm ? 1 : 0;
     sk.gate = gateTol;
     sk.nearFp64 = DIM == 3 && P == EIKX_F32 && o.near_fp64 ? 1 : 0;
@@ -1017,7 +1043,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     sk.flags = iterFlags;
 
     int launches = 0;
-    int sweepsLaunched = 0;
+    int sweepsLaunched = 0, profiled = 0;   // sweeps; sweep launches
     const bool profile = o.profile_sweeps != 0;
     if (profile) {
         while (static_cast<int>(c->sweepEv.size()) < 2 * nSweepLaunches) {
@@ -1028,7 +1054,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     }
     auto enqueue = [&]() -> eikx_status {
         launches = 0;
-        sweepsLaunched = 0;
+        sweepsLaunched = profiled = 0;
         int buf = 0;
         EIKX_CUDA(eikx::launchResetState(st, nSrc, buf, c->stream));
         ++launches;
@@ -1052,8 +1078,8 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                                            w.corners.as<eikx::Corner3>(), o.init_fp64 ? 1 : 0, c->stream));
         // 3D: the fill and the corner kernel; a warm start: its gate and the pitch padding
         launches += warm ? 1 + (Px > nx ? 1 : 0) : DIM == 3 ? 2 : 1;
-        auto sweep = [&](int e, int init, int slot) -> eikx_status {
-            if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * sweepsLaunched], c->stream));
+        auto sweep = [&](int e, int init, int slot, int mode) -> eikx_status {
+            if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * profiled], c->stream));
             if (DIM == 3) {
                 eikx::Sweep3Args<T> a{};
                 a.tt = w.tt.as<T>(); a.fieldStride = fieldStride; a.pitch = Px;
@@ -1061,9 +1087,11 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                 a.spPlane = static_cast<long long>(spPitch) * (ny + 1);
                 a.nx = nx; a.ny = ny; a.nz = nz; a.tilesY = tilesY; a.tilesZ = tilesZ;
                 a.srcs = w.srcs.as<eikx::SourceT<T>>(); a.st = st; a.buf = buf; a.residualSlot = slot;
-                a.sweepIndex = sweepsLaunched;
+                a.sweepIndex = mode == eikx::kSecondSweep ? sweepsLaunched - 1 : sweepsLaunched;
                 a.sweep = e; a.init = init; a.radius = o.factored_radius; a.h = static_cast<T>(dx);
                 a.srcs64 = srcs64;
+                a.passMode = mode;
+                a.nFields = nSrc;
                 if (uniform && (wave || sizeof(T) == 8)) {
                     a.hsPos = shad[0].as<T>(); a.hsNeg = shad[1].as<T>();
                     a.cells = c->slow3.p; a.cells64 = 1;
@@ -1114,18 +1142,27 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                     EIKX_CUDA(eikx::launchSweep2Wave<T>(a, uniform, blocks, c->stream));
                 }
             }
-            if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * sweepsLaunched + 1], c->stream));
+            if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * profiled + 1], c->stream));
+            ++profiled;
             buf ^= 1;
             ++launches;
-            ++sweepsLaunched;
+            sweepsLaunched += mode == eikx::kOneSweep ? 1 : mode == eikx::kBothSweeps ? 2 : 0;
             return EIKX_OK;
         };
-        if (o.init_sweeps)
-            for (int e = 0; e < nSweepKinds; ++e)
-                if (eikx_status r = sweep(e, 1, e); r != EIKX_OK) return r;
+        auto check = [&](int r, bool second) -> eikx_status {
+            EIKX_CUDA(eikx::launchCheckPair(st, nSrc, r, second, o.tolerance, c->stream));
+            ++launches;
+            return EIKX_OK;
+        };
+        if (o.init_sweeps && both)
+            if (eikx_status r = sweepPairs(0, true, sweep, check); r != EIKX_OK) return r;
+        for (int e = 0; e < nSweepKinds && o.init_sweeps && !both; ++e)
+            if (eikx_status r = sweep(e, 1, e, eikx::kOneSweep); r != EIKX_OK) return r;
         for (int k = 0; k < nSweeps; ++k) {
-            for (int e = 0; e < nSweepKinds; ++e) {
-                if (eikx_status r = sweep(e, 0, nSweepKinds * (1 + k) + e); r != EIKX_OK) return r;
+            if (both)
+                if (eikx_status r = sweepPairs(1 + k, false, sweep, check); r != EIKX_OK) return r;
+            for (int e = 0; e < nSweepKinds && !both; ++e) {
+                if (eikx_status r = sweep(e, 0, nSweepKinds * (1 + k) + e, eikx::kOneSweep); r != EIKX_OK) return r;
                 EIKX_CUDA(checkAfterSweep(st, nSrc, nSweepKinds, nSweepKinds * k + e, o.tolerance, c->stream));
                 ++launches;
             }
@@ -1263,7 +1300,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     s.sweep_ms = -1;
     if (profile) {
         double tot = 0;
-        for (int i = 0; i < sweepsLaunched; ++i) {
+        for (int i = 0; i < profiled; ++i) {
             float m = 0;
             cudaEventElapsedTime(&m, c->sweepEv[2 * i], c->sweepEv[2 * i + 1]);
             tot += m;
@@ -1379,6 +1416,14 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     const int resStride = nSweepKinds * (1 + nSweeps);
 
     const bool near64 = sizeof(T) == 4 && o.near_fp64;
+    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, true, near64)
+                       : eikx::sweep3ChunkBlocksPerSM<T>(uniform, true, shape);
+    if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
+    const int blocks = std::max(1, static_cast<int>(std::min<size_t>(
+                                       static_cast<size_t>(c->numSMs) * perSM,
+                                       (nItems + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock)));
+    const bool both = bothSweeps(wave, nItems, static_cast<size_t>(c->numSMs) * perSM * eikx::kWarpsPerBlock);
+    if (both) mboxWords *= 2;
     const void *before[] = {w.tt.p, w.sp.p, w.mbox.p, w.epoch.p, w.residual.p, w.converged.p, w.iterations.p,
                             w.order.p, w.srcs.p, w.corners.p, w.units.p, w.srcs64.p, w.factor.p};
     EIKX_CUDA(w.tt.ensure(ttElems * sizeof(T)));
@@ -1394,7 +1439,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     }
     EIKX_CUDA(w.queue.ensure(2 * sizeof(unsigned)));
     EIKX_CUDA(w.residual.ensure(static_cast<size_t>(nUnits) * resStride * 8));
-    EIKX_CUDA(w.converged.ensure(static_cast<size_t>(nUnits) * 4));
+    EIKX_CUDA(w.converged.ensure(static_cast<size_t>(nUnits) * 8));   // and the pair states
     EIKX_CUDA(w.iterations.ensure(static_cast<size_t>(nUnits) * 4));
     EIKX_CUDA(w.abortFlag.ensure(sizeof(int)));
     EIKX_CUDA(w.order.ensure(nItems * 16));
@@ -1484,7 +1529,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
             gu.spNeg = spBase + l.spOff + l.spElems;
             gu.hsPos = nCopies == 4 ? spBase + l.spOff + 2 * l.spElems : nullptr;
             gu.hsNeg = nCopies == 4 ? spBase + l.spOff + 3 * l.spElems : nullptr;
-            gu.mbox = mbBase + l.mboxOff + static_cast<size_t>(j) * l.tilesY * l.tilesZ * l.faceWords;
+            gu.mbox = mbBase + (l.mboxOff + static_cast<size_t>(j) * l.tilesY * l.tilesZ * l.faceWords) * (both ? 2 : 1);
             gu.spPlane = l.spPlane;
             gu.spPitch = l.spPitch;
             gu.Px = l.Px; gu.nx = m.nx; gu.ny = m.ny; gu.nz = m.nz;
@@ -1573,20 +1618,15 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     st.residual = w.residual.as<unsigned long long>();
     st.residualStride = resStride;
     st.converged = w.converged.as<int>();
+    st.pairState = w.converged.as<int>() + nUnits;
     st.sweepsRun = w.iterations.as<int>();
     st.abortFlag = w.abortFlag.as<int>();
     st.order = w.order.as<int4>();
     st.totalItems = static_cast<int>(nItems);
     const int spinLog2 = o.spin_limit_log2 > 0 ? std::min(o.spin_limit_log2, 40) : 22;
     st.spinLimit = 1ull << spinLog2;
-    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, true, near64)
-                       : eikx::sweep3ChunkBlocksPerSM<T>(uniform, true, shape);
-    if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
-    const int blocks = std::max(1, static_cast<int>(std::min<size_t>(
-                                       static_cast<size_t>(c->numSMs) * perSM,
-                                       (nItems + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock)));
 
-    int launches = 0, sweepsLaunched = 0;
+    int launches = 0, sweepsLaunched = 0, profiled = 0;   // kernels; sweeps; sweep launches
     const bool profile = o.profile_sweeps != 0;
     if (profile) {
         while (static_cast<int>(c->sweepEv.size()) < 2 * nSweepLaunches) {
@@ -1612,7 +1652,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     }
     auto enqueue = [&]() -> eikx_status {
         launches = 0;
-        sweepsLaunched = 0;
+        sweepsLaunched = profiled = 0;
         int buf = 0;
         EIKX_CUDA(eikx::launchResetState(st, nUnits, buf, c->stream));
         ++launches;
@@ -1627,28 +1667,39 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
                                            o.init_fp64 ? 1 : 0, c->stream));
             launches += 2;   // the fill and the corner kernel
         }
-        auto sweep = [&](int e, int init, int slot) -> eikx_status {
-            if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * sweepsLaunched], c->stream));
+        auto sweep = [&](int e, int init, int slot, int mode) -> eikx_status {
+            if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * profiled], c->stream));
             eikx::Sweep3Args<T> a{};
             a.srcs = w.srcs.as<eikx::SourceT<T>>(); a.st = st; a.buf = buf; a.residualSlot = slot;
-            a.sweepIndex = sweepsLaunched;
+            a.sweepIndex = mode == eikx::kSecondSweep ? sweepsLaunched - 1 : sweepsLaunched;
             a.sweep = e; a.init = init; a.radius = o.factored_radius;
+            a.passMode = mode;
+            a.nFields = nUnits;
             a.units = w.units.as<eikx::Grid3Unit<T>>();
             a.srcs64 = near64 ? w.srcs64.as<eikx::SourceFp64>() : nullptr;
             if (wave) EIKX_CUDA(eikx::launchSweep3Wave<T>(a, uniform, blocks, c->stream));
             else EIKX_CUDA(eikx::launchSweep3Chunk<T>(a, uniform, shape, blocks, c->stream));
-            if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * sweepsLaunched + 1], c->stream));
+            if (profile) EIKX_CUDA(cudaEventRecord(c->sweepEv[2 * profiled + 1], c->stream));
+            ++profiled;
             buf ^= 1;
             ++launches;
-            ++sweepsLaunched;
+            sweepsLaunched += mode == eikx::kOneSweep ? 1 : mode == eikx::kBothSweeps ? 2 : 0;
             return EIKX_OK;
         };
-        if (o.init_sweeps)
-            for (int e = 0; e < nSweepKinds; ++e)
-                if (eikx_status r = sweep(e, 1, e); r != EIKX_OK) return r;
+        auto check = [&](int r, bool second) -> eikx_status {
+            EIKX_CUDA(eikx::launchCheckPair(st, nUnits, r, second, o.tolerance, c->stream));
+            ++launches;
+            return EIKX_OK;
+        };
+        if (o.init_sweeps && both)
+            if (eikx_status r = sweepPairs(0, true, sweep, check); r != EIKX_OK) return r;
+        for (int e = 0; e < nSweepKinds && o.init_sweeps && !both; ++e)
+            if (eikx_status r = sweep(e, 1, e, eikx::kOneSweep); r != EIKX_OK) return r;
         for (int k = 0; k < nSweeps; ++k) {
-            for (int e = 0; e < nSweepKinds; ++e) {
-                if (eikx_status r = sweep(e, 0, nSweepKinds * (1 + k) + e); r != EIKX_OK) return r;
+            if (both)
+                if (eikx_status r = sweepPairs(1 + k, false, sweep, check); r != EIKX_OK) return r;
+            for (int e = 0; e < nSweepKinds && !both; ++e) {
+                if (eikx_status r = sweep(e, 0, nSweepKinds * (1 + k) + e, eikx::kOneSweep); r != EIKX_OK) return r;
                 EIKX_CUDA(checkAfterSweep(st, nUnits, nSweepKinds, nSweepKinds * k + e, o.tolerance, c->stream));
                 ++launches;
             }
@@ -1666,7 +1717,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
                                static_cast<double>(o.n_sweeps), static_cast<double>(o.factored_radius),
                                static_cast<double>(o.init_sweeps), static_cast<double>(o.init_fp64), o.tolerance,
                                static_cast<double>(st.spinLimit), static_cast<double>(blocks),
-                               static_cast<double>(wave ? -1 : shape), static_cast<double>(o.near_fp64 ? 1 : 0)};
+                               static_cast<double>(both ? -2 : wave ? -1 : shape), static_cast<double>(o.near_fp64 ? 1 : 0)};
     for (int i = 0; i < nM; ++i) {
         const eikx_model3d &m = models[sel[i]];
         for (double v : {static_cast<double>(m.nx), static_cast<double>(m.ny), static_cast<double>(m.nz), m.dx, m.dy,
@@ -1774,7 +1825,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     agg.device_ms += ms;
     if (profile) {
         double tot = 0;
-        for (int i = 0; i < sweepsLaunched; ++i) {
+        for (int i = 0; i < profiled; ++i) {
             float m = 0;
             cudaEventElapsedTime(&m, c->sweepEv[2 * i], c->sweepEv[2 * i + 1]);
             tot += m;

@@ -349,6 +349,7 @@ __global__ void resetKernel(SolveState st, int nFields, int buf) {
     for (int i = gtid; i < nFields; i += gthreads) {
         st.converged[i] = 0;
         st.sweepsRun[i] = 0;
+        if (st.pairState) st.pairState[i] = kPairRun;
     }
     if (gtid == 0) {
         *st.queue[buf] = 0u;
@@ -370,6 +371,30 @@ __global__ void checkKernel(SolveState st, int nFields, int firstSlot, int nSlot
                             st.residual[static_cast<long long>(f) * st.residualStride + firstSlot + k])));
         st.sweepsRun[f] = sweepsDone;
         if (m < tol) st.converged[f] = 1;
+    }
+}
+
+// The same test where a launch ran refinement sweeps r and r + 1 (slots 8 + r, 9 + r), or r alone
+// on the fields that held r + 1 back, and where it then ran r + 1 on those it left open (`second`).
+// A field holds the odd sweep back when it could end with the even one: when the seven sweeps
+// before that are below tol.
+__global__ void checkPairKernel(SolveState st, int nFields, int r, int second, double tol) {
+    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nFields; f += gridDim.x * blockDim.x) {
+        if (st.converged[f]) continue;
+        const int state = st.pairState[f];
+        if (second && state != kPairOpen) continue;
+        const unsigned long long *res = st.residual + static_cast<long long>(f) * st.residualStride + 8;
+        auto largest = [&](int first, int last) {
+            double m = 0;
+            for (int k = max(first, 0); k <= last; ++k) m = fmax(m, __longlong_as_double(static_cast<long long>(res[k])));
+            return m;
+        };
+        const bool held = !second && state == kPairHeld;
+        const int done = held ? r : r + 1;   // the last refinement sweep run
+        st.sweepsRun[f] = done + 1;
+        if (done >= 7 && largest(done - 7, done) < tol) st.converged[f] = 1;
+        else if (held) st.pairState[f] = kPairOpen;
+        else st.pairState[f] = r + 2 >= 7 && largest(r - 5, r + 1) < tol ? kPairHeld : kPairRun;
     }
 }
 
@@ -597,6 +622,10 @@ cudaError_t launchCheckPositive(const float *s, long long n, int *flag, cudaStre
 cudaError_t launchCheckConvergence(const SolveState &st, int nFields, int firstSlot, int nSlots, int sweepsDone,
                                    double tol, cudaStream_t s) {
     checkKernel<<<gridFor(nFields, 128), 128, 0, s>>>(st, nFields, firstSlot, nSlots, sweepsDone, tol);
+    return cudaGetLastError();
+}
+cudaError_t launchCheckPair(const SolveState &st, int nFields, int r, bool second, double tol, cudaStream_t s) {
+    checkPairKernel<<<gridFor(nFields, 128), 128, 0, s>>>(st, nFields, r, second ? 1 : 0, tol);
     return cudaGetLastError();
 }
 cudaError_t launchCheckStream(const SolveState &st, const int2 *slots, int nSlots, int sweepIndex, int initSweeps,

@@ -21,12 +21,21 @@ struct SolveState {
     unsigned long long *residual;   // [field][sweep slot] largest decrease (double bits)
     int residualStride;             // slots per field
     int *converged;                 // 1 once a field's iteration decrease fell below tol
+    int *pairState;                 // wave-step kernel, two orderings per launch: PairState per field
+                                    // (null otherwise)
     int *sweepsRun;                 // refinement sweeps each field ran
     int *abortFlag;                 // raised when a bounded wait ran out
     const int4 *order;              // work queue: (field, by, bz, 0) sorted by start step
     int totalItems;                 // fields * warp blocks per field
     unsigned long long spinLimit;   // polls before a wait gives up
 };
+
+// A wave-step launch runs one sweep, or the two orderings that differ in the direction of x' only
+// (even, odd: same blocks, same dependences between blocks): each block walks its rows forth and
+// back, which saves the second sweep's way through the blocks.  A field that could end with the
+// even one holds the odd one back, for a launch of its own (kSecondSweep).
+enum PassMode { kOneSweep = 0, kBothSweeps = 1, kSecondSweep = 2 };
+enum PairState { kPairRun = 0, kPairHeld = 1, kPairOpen = 2 };
 
 // Geometry of one work unit (one field on one model) of a multi-model batch: the grids of
 // a batch may differ in size and spacing; a warp reads its unit's entry per work item.
@@ -71,6 +80,9 @@ template <class T> struct Sweep3Args {
     // stream and `sweep` its ordering (sweepIndex mod 8).
     const int2 *slots;
     int initSweeps;           // 1 = a slot's first 8 sweeps are its initialisation pass
+    int passMode;             // PassMode (wave-step kernel); sweep, sweepIndex, residualSlot are the
+                              // launch's first sweep's
+    int nFields;              // fields (read unless passMode is kOneSweep)
     // Uniform grids, one model: wave-step kernel and FP64 chunk-step kernel (required there): the padded slowness copies multiplied by h (launchPadSlowness3 with h), laid out
     // as spPos / spNeg; for the latter's factored branch also the model's natural-order cell
     // slowness (FP64 cells, or FP32 cells with cells64 = 0)
@@ -152,6 +164,9 @@ constexpr int kWaveLY = 8, kWaveLZ = 4;
 __host__ __device__ constexpr int waveStepCap(int Px) { return Px + 32; }
 template <class T> cudaError_t launchSweep3Wave(const Sweep3Args<T> &a, bool uniform, int blocks, cudaStream_t s);
 template <class T> int sweep3WaveBlocksPerSM(bool uniform, bool batch, bool near64);
+// After a kBothSweeps launch whose first sweep was refinement sweep r (r even), and after the
+// kSecondSweep launch behind it: the convergence test, and which fields hold the next odd sweep.
+cudaError_t launchCheckPair(const SolveState &st, int nFields, int r, bool second, double tol, cudaStream_t s);
 // Warp blocks of one field, and the mailbox words each needs.
 struct Tiling3 {
     int ly, lz, tilesY, tilesZ;

@@ -65,3 +65,29 @@ def test_wave_step_2d_block_edges_match_the_oracle(ctx, oracle, grid, spacing, p
         cell = [min(n - 2, int(q / d)) for q, n, d in zip(p, grid, spacing)]
         ref = oracle.solve2d(s, (nx, nz, dx, dz), cell, p, n_sweeps=3, radius=2, tol=1e-9)
         assert np.array_equal(_bits(a), _bits(ref)), (p, np.abs(a - ref).max())
+
+
+# 160 fields of 5 x 8 warp blocks: on the warps of four (two in double) resident blocks per SM both
+# orderings of a pair share a launch, on those of one they don't
+@pytest.mark.parametrize("precision", [ex.F32, ex.F64])
+@pytest.mark.parametrize("spacing", [(50.0, 50.0, 50.0), (50.0, 65.0, 40.0)])
+@pytest.mark.parametrize("init,tol", [(True, 1e-2), (True, 1e-4), (True, 1e-5), (True, 1e-6), (False, 1e-4)])
+def test_both_orderings_in_one_launch_match_one_by_one(ctx, oracle, spacing, precision, init, tol):
+    grid = nx, ny, nz = 41, 34, 30
+    rng = np.random.default_rng(11)
+    dt = np.float32 if precision == ex.F32 else np.float64
+    s = random_slowness(rng, (nz - 1) * (ny - 1) * (nx - 1), dtype=dt)
+    ctx.set_grid3d(nx, ny, nz, *spacing)
+    ctx.set_slowness3d(s)
+    pos = rng.uniform(0, 1, (160, 3)) * (np.array(grid) - 1) * spacing
+    out = []
+    for per_sm in (0, 1):
+        t = ctx.solve3d(pos, ex.Options(n_sweeps=6, tolerance=tol, init_sweeps=init, blocks_per_sm=per_sm), precision)
+        st = ctx.stats()
+        out.append((t, [st[k] for k in ("iterations_max", "iterations_min", "sweeps_launched", "refine_node_updates")]))
+    assert out[0][1] == out[1][1]
+    assert np.array_equal(_bits(np.asarray(out[0][0])), _bits(np.asarray(out[1][0])))
+    for i in (0, 77, 159):
+        cell = [min(n - 2, int(q / h)) for q, n, h in zip(pos[i], grid, spacing)]
+        ref = oracle.solve3d(s, (nx, ny, nz, *spacing), cell, pos[i], n_sweeps=6, radius=3, tol=tol, init_sweeps=init)
+        assert np.array_equal(_bits(out[0][0][i]), _bits(ref))
