@@ -263,32 +263,17 @@ __global__ void __launch_bounds__(kThreads) wgradKernel(WGradArgs a) {
     }
 }
 
-__global__ void biasGradKernel(const bf16 *dy, int C, long long nodes, float *db) {
-    __shared__ float part[kThreads];
-    const int c = threadIdx.x % C, slot = threadIdx.x / C, slots = kThreads / C;
-    float s = 0.f;
-    for (long long v = static_cast<long long>(blockIdx.x) * slots + slot; v < nodes;
-         v += static_cast<long long>(gridDim.x) * slots)
-        s += __bfloat162float(dy[v * C + c]);
-    part[threadIdx.x] = s;
-    __syncthreads();
-    if (slot == 0) {
-        for (int k = 1; k < slots; ++k) s += part[k * C + c];
-        atomicAdd(db + c, s);
-    }
-}
-
 struct alignas(16) Vec8 {
     __nv_bfloat162 h[4];
 };
-__device__ __forceinline__ void load8(float (&f)[8], const bf16 *p) {
-    const Vec8 v = *reinterpret_cast<const Vec8 *>(p);
+__device__ __forceinline__ void unpack8(float (&f)[8], const Vec8 &v) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         f[2 * i] = __bfloat162float(v.h[i].x);
         f[2 * i + 1] = __bfloat162float(v.h[i].y);
     }
 }
+__device__ __forceinline__ void load8(float (&f)[8], const bf16 *p) { unpack8(f, *reinterpret_cast<const Vec8 *>(p)); }
 __device__ __forceinline__ void store8(bf16 *p, const float (&f)[8]) {
     Vec8 v;
 #pragma unroll
@@ -296,183 +281,273 @@ __device__ __forceinline__ void store8(bf16 *p, const float (&f)[8]) {
     *reinterpret_cast<Vec8 *>(p) = v;
 }
 
-__global__ void poolKernel(const bf16 *x, int C, int D, int H, int W, int B, bf16 *y) {
+// db[c] += sum over nodes of dy[.][c].  Bound by reading dy: a thread sums eight channels, 16 bytes
+// a node (8.4 M nodes of 16 channels: 131 us with one channel a thread, 61 now).
+__global__ void __launch_bounds__(kThreads) biasGradKernel(const bf16 *dy, int C, long long nodes, float *db) {
+    __shared__ float part[kThreads][9];   // 9: the sums below read 8 rows apart without bank conflicts
+    const int groups = C / 8, g = threadIdx.x % groups, slot = threadIdx.x / groups, slots = kThreads / groups;
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+    for (long long v = static_cast<long long>(blockIdx.x) * slots + slot; v < nodes;
+         v += static_cast<long long>(gridDim.x) * slots) {
+        float f[8];
+        load8(f, dy + v * C + 8 * g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += f[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part[threadIdx.x][j] = s[j];
+    __syncthreads();
+    if (threadIdx.x < C) {
+        float t = 0.f;
+        for (int k = 0; k < slots; ++k) t += part[k * groups + threadIdx.x / 8][threadIdx.x % 8];
+        atomicAdd(db + threadIdx.x, t);
+    }
+}
+
+// The element-wise kernels below move whole 16-byte pieces of 8 channels and are bound by memory.
+// A block takes pieces of one x-row of the tensor that it writes (grid: pieces of a row, rows of a
+// plane, planes of all samples), so that a thread needs one 32-bit division to find its place
+// (upsampling and concatenation at 8 x 64 x 128 x 128 nodes: 445 us with five 64-bit ones, 183 now).
+struct Piece {
+    int g, x, y, z, b;   // 8-channel group, node, sample
+};
+__device__ __forceinline__ bool pieceOf(Piece &p, int groups, int W, int D, long long plane) {
+    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+    p.x = static_cast<int>(i / static_cast<unsigned>(groups));
+    p.g = static_cast<int>(i - static_cast<unsigned>(p.x) * groups);
+    p.y = blockIdx.y;
+    p.b = static_cast<int>(plane / D);
+    p.z = static_cast<int>(plane - static_cast<long long>(p.b) * D);
+    return p.x < W;
+}
+
+__global__ void __launch_bounds__(kThreads) poolKernel(const bf16 *x, int C, int D, int H, int W, int B, bf16 *y) {
     const int Dl = D / 2, Hl = H / 2, Wl = W / 2, groups = C / 8;
-    const long long total = static_cast<long long>(B) * Dl * Hl * Wl * groups;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int g = i % groups;
-        long long u = i / groups;
-        const int ux = u % Wl, uy = (u / Wl) % Hl, uz = (u / (static_cast<long long>(Wl) * Hl)) % Dl;
-        const long long b = u / (static_cast<long long>(Wl) * Hl * Dl);
+    for (long long plane = blockIdx.z; plane < static_cast<long long>(B) * Dl; plane += gridDim.z) {
+        Piece p;
+        if (!pieceOf(p, groups, Wl, Dl, plane)) continue;
+        const bf16 *src = x + ((((static_cast<long long>(p.b) * D + 2 * p.z) * H + 2 * p.y) * W + 2 * p.x) * C + 8 * p.g);
         float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const int z = 2 * uz + (k >> 2), yy = 2 * uy + ((k >> 1) & 1), xx = 2 * ux + (k & 1);
             float f[8];
-            load8(f, x + ((b * D + z) * H * static_cast<long long>(W) + static_cast<long long>(yy) * W + xx) * C + 8 * g);
+            load8(f, src + ((static_cast<long long>(k >> 2) * H + ((k >> 1) & 1)) * W + (k & 1)) * C);
 #pragma unroll
             for (int j = 0; j < 8; ++j) s[j] += f[j];
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) s[j] *= 0.125f;
-        store8(y + u * C + 8 * g, s);
+        store8(y + ((plane * Hl + p.y) * Wl + p.x) * C + 8 * p.g, s);
     }
 }
 
-__global__ void upcatKernel(const bf16 *low, int c1, const bf16 *skip, int c2, int D, int H, int W, int B,
-                            bf16 *out) {
+// (kRowsEach rows a thread, their loads all in flight before the first store.)
+constexpr int kRowsEach = 4;
+__global__ void __launch_bounds__(kThreads) upcatKernel(const bf16 *low, int c1, const bf16 *skip, int c2, int D, int H, int W,
+                                                        int B, bf16 *out) {
     const int C = c1 + c2, groups = C / 8;
-    const long long total = static_cast<long long>(B) * D * H * W * groups;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int g = i % groups;
-        const long long v = i / groups;
-        const int x = v % W, y = (v / W) % H, z = (v / (static_cast<long long>(W) * H)) % D;
-        const long long b = v / (static_cast<long long>(W) * H * D);
-        const bf16 *src;
-        if (8 * g < c1) {
-            const long long u = ((b * (D / 2) + z / 2) * (H / 2) + y / 2) * (W / 2) + x / 2;
-            src = low + u * c1 + 8 * g;
-        } else {
-            src = skip + v * c2 + 8 * g - c1;
+    for (long long plane = blockIdx.z; plane < static_cast<long long>(B) * D; plane += gridDim.z) {
+        Piece p;
+        if (!pieceOf(p, groups, W, D, plane)) continue;
+        Vec8 v[kRowsEach];
+#pragma unroll
+        for (int k = 0; k < kRowsEach; ++k) {
+            const int y = kRowsEach * p.y + k;
+            if (y >= H) break;
+            const bf16 *src = skip + ((plane * H + y) * W + p.x) * c2 + 8 * p.g - c1;
+            if (8 * p.g < c1)
+                src = low + (((static_cast<long long>(p.b) * (D / 2) + p.z / 2) * (H / 2) + y / 2) * (W / 2) + p.x / 2) * c1 + 8 * p.g;
+            v[k] = *reinterpret_cast<const Vec8 *>(src);
         }
-        *reinterpret_cast<Vec8 *>(out + v * C + 8 * g) = *reinterpret_cast<const Vec8 *>(src);
+#pragma unroll
+        for (int k = 0; k < kRowsEach; ++k) {
+            const int y = kRowsEach * p.y + k;
+            if (y < H) *reinterpret_cast<Vec8 *>(out + ((plane * H + y) * W + p.x) * C + 8 * p.g) = v[k];
+        }
     }
 }
 
-__global__ void upSumMaskKernel(const bf16 *dcat, int ccat, const bf16 *act, int c1, int Dl, int Hl, int Wl, int B,
-                                bf16 *dpre) {
+__global__ void __launch_bounds__(kThreads) upSumMaskKernel(const bf16 *dcat, int ccat, const bf16 *act, int c1, int Dl, int Hl,
+                                                            int Wl, int B, bf16 *dpre) {
     const int groups = c1 / 8, D = 2 * Dl, H = 2 * Hl, W = 2 * Wl;
-    const long long total = static_cast<long long>(B) * Dl * Hl * Wl * groups;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int g = i % groups;
-        const long long u = i / groups;
-        const int ux = u % Wl, uy = (u / Wl) % Hl, uz = (u / (static_cast<long long>(Wl) * Hl)) % Dl;
-        const long long b = u / (static_cast<long long>(Wl) * Hl * Dl);
+    for (long long plane = blockIdx.z; plane < static_cast<long long>(B) * Dl; plane += gridDim.z) {
+        Piece p;
+        if (!pieceOf(p, groups, Wl, Dl, plane)) continue;
+        const bf16 *src = dcat + ((((static_cast<long long>(p.b) * D + 2 * p.z) * H + 2 * p.y) * W + 2 * p.x) * ccat + 8 * p.g);
+        const long long u = (plane * Hl + p.y) * Wl + p.x;
         float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const int z = 2 * uz + (k >> 2), yy = 2 * uy + ((k >> 1) & 1), xx = 2 * ux + (k & 1);
             float f[8];
-            load8(f, dcat + ((b * D + z) * H * static_cast<long long>(W) + static_cast<long long>(yy) * W + xx) * ccat +
-                         8 * g);
+            load8(f, src + ((static_cast<long long>(k >> 2) * H + ((k >> 1) & 1)) * W + (k & 1)) * ccat);
 #pragma unroll
             for (int j = 0; j < 8; ++j) s[j] += f[j];
         }
         float m[8];
-        load8(m, act + u * c1 + 8 * g);
+        load8(m, act + u * c1 + 8 * p.g);
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             if (!(m[j] > 0.f)) s[j] = 0.f;
-        store8(dpre + u * c1 + 8 * g, s);
+        store8(dpre + u * c1 + 8 * p.g, s);
     }
 }
 
-__global__ void combineSkipKernel(const bf16 *dcat, int ccat, int c1, const bf16 *dpool, const bf16 *skip, int c2,
-                                  int D, int H, int W, int B, bf16 *dpre) {
+__global__ void __launch_bounds__(kThreads) combineSkipKernel(const bf16 *dcat, int ccat, int c1, const bf16 *dpool,
+                                                              const bf16 *skip, int c2, int D, int H, int W, int B, bf16 *dpre) {
     const int groups = c2 / 8;
-    const long long total = static_cast<long long>(B) * D * H * W * groups;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int g = i % groups;
-        const long long v = i / groups;
-        const int x = v % W, y = (v / W) % H, z = (v / (static_cast<long long>(W) * H)) % D;
-        const long long b = v / (static_cast<long long>(W) * H * D);
-        const long long u = ((b * (D / 2) + z / 2) * (H / 2) + y / 2) * (W / 2) + x / 2;
-        float a[8], p[8], m[8];
-        load8(a, dcat + v * ccat + c1 + 8 * g);
-        load8(p, dpool + u * c2 + 8 * g);
-        load8(m, skip + v * c2 + 8 * g);
+    for (long long plane = blockIdx.z; plane < static_cast<long long>(B) * D; plane += gridDim.z) {
+        Piece q;
+        if (!pieceOf(q, groups, W, D, plane)) continue;
+        Vec8 a[kRowsEach], p[kRowsEach], m[kRowsEach];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) a[j] = (m[j] > 0.f) ? a[j] + 0.125f * p[j] : 0.f;
-        store8(dpre + v * c2 + 8 * g, a);
+        for (int k = 0; k < kRowsEach; ++k) {
+            const int y = kRowsEach * q.y + k;
+            if (y >= H) break;
+            const long long v = (plane * H + y) * W + q.x;
+            const long long u = ((static_cast<long long>(q.b) * (D / 2) + q.z / 2) * (H / 2) + y / 2) * (W / 2) + q.x / 2;
+            a[k] = *reinterpret_cast<const Vec8 *>(dcat + v * ccat + c1 + 8 * q.g);
+            p[k] = *reinterpret_cast<const Vec8 *>(dpool + u * c2 + 8 * q.g);
+            m[k] = *reinterpret_cast<const Vec8 *>(skip + v * c2 + 8 * q.g);
+        }
+#pragma unroll
+        for (int k = 0; k < kRowsEach; ++k) {
+            const int y = kRowsEach * q.y + k;
+            if (y >= H) break;
+            float f[8], g[8], r[8];
+            unpack8(f, a[k]);
+            unpack8(g, p[k]);
+            unpack8(r, m[k]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] = (r[j] > 0.f) ? f[j] + 0.125f * g[j] : 0.f;
+            store8(dpre + ((plane * H + y) * W + q.x) * c2 + 8 * q.g, f);
+        }
     }
 }
 
 // Per-node geometry, FP32: the offsets from the source are FP64 differences rounded to
 // FP32, the distance an FP32 square root; s_src is the slowness at the node nearest the
-// source.
-__device__ __forceinline__ long long nearestNode(const Sample &s, const Geometry &g) {
-    const int ix = min(g.nx - 1, max(0, __double2int_rn((s.xs - g.x0) / g.dx)));
-    const int iy = min(g.ny - 1, max(0, __double2int_rn((s.ys - g.y0) / g.dy)));
-    const int iz = min(g.nz - 1, max(0, __double2int_rn((s.zs - g.z0) / g.dz)));
-    return (static_cast<long long>(iz) * g.ny + iy) * g.nx + ix;
+// source.  An FP64 instruction takes 64 cycles a warp and scheduler here, so what is FP64 in them
+// is taken once per sample and axis position, into the sample's table (warmnet.h).
+__global__ void __launch_bounds__(kThreads) slownessKernel(const Sample *samples, Geometry g, float *slow, float *tables) {
+    const long long V = static_cast<long long>(g.nx) * g.ny * g.nz;
+    const Sample s = samples[blockIdx.y];
+    float *table = tables + blockIdx.y * tableLength(g);
+    const long long first = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x, step = static_cast<long long>(gridDim.x) * blockDim.x;
+    for (long long i = first; i < V; i += step) slow[blockIdx.y * V + i] = 1.f / s.velocity[i];
+    for (long long i = first; i < tableLength(g); i += step) {
+        float v;
+        if (i == 0) {
+            const int ix = min(g.nx - 1, max(0, __double2int_rn((s.xs - g.x0) / g.dx)));
+            const int iy = min(g.ny - 1, max(0, __double2int_rn((s.ys - g.y0) / g.dy)));
+            const int iz = min(g.nz - 1, max(0, __double2int_rn((s.zs - g.z0) / g.dz)));
+            v = 1.f / s.velocity[(static_cast<long long>(iz) * g.ny + iy) * g.nx + ix];
+        } else if (i < 4) {
+            v = static_cast<float>(i == 1 ? (s.xs - g.x0) / g.dx : i == 2 ? (s.ys - g.y0) / g.dy : (s.zs - g.z0) / g.dz);
+        } else {
+            const int k = static_cast<int>(i) - 4;
+            v = k < g.nx            ? static_cast<float>((g.x0 + k * g.dx) - s.xs)
+                : k < g.nx + g.ny ? static_cast<float>((g.y0 + (k - g.nx) * g.dy) - s.ys)
+                                  : static_cast<float>((g.z0 + (k - g.nx - g.ny) * g.dz) - s.zs);
+        }
+        table[i] = v;
+    }
 }
 struct NodeGeom {
     float ddx, ddy, ddz, dist;
 };
-__device__ __forceinline__ NodeGeom nodeGeom(long long v, const Sample &s, const Geometry &g) {
-    const int x = v % g.nx, y = (v / g.nx) % g.ny, z = v / (static_cast<long long>(g.nx) * g.ny);
+__device__ __forceinline__ NodeGeom nodeGeom(const float *table, const Geometry &g, int x, int y, int z) {
     NodeGeom n;
-    n.ddx = static_cast<float>((g.x0 + x * g.dx) - s.xs);
-    n.ddy = static_cast<float>((g.y0 + y * g.dy) - s.ys);
-    n.ddz = static_cast<float>((g.z0 + z * g.dz) - s.zs);
+    n.ddx = table[4 + x];
+    n.ddy = table[4 + g.nx + y];
+    n.ddz = table[4 + g.nx + g.ny + z];
     n.dist = sqrtf(n.ddx * n.ddx + n.ddy * n.ddy + n.ddz * n.ddz);
     return n;
 }
 
-__global__ void slownessKernel(const Sample *samples, Geometry g, int B, float *slow) {
-    const long long V = static_cast<long long>(g.nx) * g.ny * g.nz;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < B * V;
-         i += static_cast<long long>(gridDim.x) * blockDim.x)
-        slow[i] = 1.f / samples[i / V].velocity[i % V];
-}
-
 // Straight-ray estimate of tau - 1 at node (x, y, z): the mean of s/s_src - 1 over
 // kRaySamples midpoints of the segment from the source to the node, the slowness
-// trilinear in the nodal 1/v.  FP32, in an operation order the oracle repeats.
+// trilinear in the nodal 1/v.  FP32, in an operation order the oracle repeats.  What bounds it is
+// issue slots: two midpoints share packed FP32 additions, floor is an addition
+// rounded down (px + 2^23, whose low bits are the index; the conversions run at a quarter of the
+// rate), and the clamps to the grid are left out where the source lies inside (INSIDE: then so do
+// the rounded points of the segment: with w = RN(t e), |w| <= (63/64) |e| (1 + 2^-23) leaves s + w
+// between s and x, and rounding keeps that).
 constexpr int kRaySamples = 32;
-__device__ float straightRayContrast(const Sample &s, const float *sl, const Geometry &g, float sSrc, int x, int y,
-                                     int z) {
-    auto at = [&](int ix, int iy, int iz) { return sl[(static_cast<long long>(iz) * g.ny + iy) * g.nx + ix]; };
-    const float sx = static_cast<float>((s.xs - g.x0) / g.dx), sy = static_cast<float>((s.ys - g.y0) / g.dy),
-                sz = static_cast<float>((s.zs - g.z0) / g.dz);
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 r;
+    asm("{.reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+// (Scalar: the assembler fuses a packed product into a packed sum, .rn or not.)
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return add2(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 f) { return add2(a, mul2(f, sub2(b, a))); }
+template <bool INSIDE>
+__device__ __forceinline__ float straightRayContrast(const float *sl, const Geometry &g, const float *table, int x, int y, int z) {
+    const float sSrc = table[0], sx = table[1], sy = table[2], sz = table[3];
     const float ex = static_cast<float>(x) - sx, ey = static_cast<float>(y) - sy, ez = static_cast<float>(z) - sz;
+    constexpr float kTwo23 = 8388608.f;
+    // cell index along one axis (two midpoints), and the positions within the cells
+    auto cell = [&](float s, float e, float2 t, int n, int (&i)[2]) {
+        float2 p = add2(make_float2(s, s), mul2(t, make_float2(e, e)));
+        if (!INSIDE) {
+            p.x = fminf(fmaxf(p.x, 0.f), static_cast<float>(n - 1));
+            p.y = fminf(fmaxf(p.y, 0.f), static_cast<float>(n - 1));
+        }
+        const float top = kTwo23 + static_cast<float>(n - 2);   // exact: n <= 2^23
+        const float2 m = make_float2(fminf(__fadd_rd(p.x, kTwo23), top), fminf(__fadd_rd(p.y, kTwo23), top));
+        i[0] = __float_as_int(m.x) & 0x7fffff;
+        i[1] = __float_as_int(m.y) & 0x7fffff;
+        return sub2(p, sub2(m, make_float2(kTwo23, kTwo23)));
+    };
+    const int ny = g.nx, nz = g.nx * g.ny;   // strides (a sample holds fewer than 2^31 nodes)
+    const float *slY = sl + ny, *slZ = sl + nz, *slYZ = slY + nz;
     float acc = 0.f;
-    for (int k = 0; k < kRaySamples; ++k) {
-        const float t = (static_cast<float>(k) + 0.5f) / static_cast<float>(kRaySamples);
-        const float px = fminf(fmaxf(sx + t * ex, 0.f), static_cast<float>(g.nx - 1));
-        const float py = fminf(fmaxf(sy + t * ey, 0.f), static_cast<float>(g.ny - 1));
-        const float pz = fminf(fmaxf(sz + t * ez, 0.f), static_cast<float>(g.nz - 1));
-        const int ix = min(static_cast<int>(floorf(px)), g.nx - 2), iy = min(static_cast<int>(floorf(py)), g.ny - 2),
-                  iz = min(static_cast<int>(floorf(pz)), g.nz - 2);
-        const float fx = px - static_cast<float>(ix), fy = py - static_cast<float>(iy), fz = pz - static_cast<float>(iz);
-        const float s000 = at(ix, iy, iz), s100 = at(ix + 1, iy, iz);
-        const float s010 = at(ix, iy + 1, iz), s110 = at(ix + 1, iy + 1, iz);
-        const float s001 = at(ix, iy, iz + 1), s101 = at(ix + 1, iy, iz + 1);
-        const float s011 = at(ix, iy + 1, iz + 1), s111 = at(ix + 1, iy + 1, iz + 1);
-        const float c00 = s000 + fx * (s100 - s000), c10 = s010 + fx * (s110 - s010);
-        const float c01 = s001 + fx * (s101 - s001), c11 = s011 + fx * (s111 - s011);
-        const float c0 = c00 + fy * (c10 - c00), c1 = c01 + fy * (c11 - c01);
-        const float c = c0 + fz * (c1 - c0);
-        acc += c / sSrc - 1.f;
+#pragma unroll 2
+    for (int k = 0; k < kRaySamples; k += 2) {
+        const float2 t = make_float2((static_cast<float>(k) + 0.5f) / static_cast<float>(kRaySamples),
+                                     (static_cast<float>(k + 1) + 0.5f) / static_cast<float>(kRaySamples));
+        int ix[2], iy[2], iz[2];
+        const float2 fx = cell(sx, ex, t, g.nx, ix), fy = cell(sy, ey, t, g.ny, iy), fz = cell(sz, ez, t, g.nz, iz);
+        const int o = iz[0] * nz + iy[0] * ny + ix[0], q = iz[1] * nz + iy[1] * ny + ix[1];
+        const float2 c00 = lerp2(make_float2(sl[o], sl[q]), make_float2(sl[o + 1], sl[q + 1]), fx);
+        const float2 c10 = lerp2(make_float2(slY[o], slY[q]), make_float2(slY[o + 1], slY[q + 1]), fx);
+        const float2 c01 = lerp2(make_float2(slZ[o], slZ[q]), make_float2(slZ[o + 1], slZ[q + 1]), fx);
+        const float2 c11 = lerp2(make_float2(slYZ[o], slYZ[q]), make_float2(slYZ[o + 1], slYZ[q + 1]), fx);
+        const float2 c = lerp2(lerp2(c00, c10, fy), lerp2(c01, c11, fy), fz);
+        acc += c.x / sSrc - 1.f;
+        acc += c.y / sSrc - 1.f;
     }
     return acc / static_cast<float>(kRaySamples);
 }
 
-__global__ void featuresKernel(const Sample *samples, const float *slow, Geometry g, int B, bf16 *feat) {
+// Input features.  8 x 64 x 128 x 128 nodes: 1169 us with FP64 per node and one midpoint at a time,
+// 694 now; the 16 bytes a node reads and the 32 it writes would take 60.
+__global__ void __launch_bounds__(kThreads) featuresKernel(const float *slow, const float *tables, Geometry g, bf16 *feat) {
     const long long V = static_cast<long long>(g.nx) * g.ny * g.nz;
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    if (i >= B * V) return;
-    const int b = i / V;
-    const long long v = i % V;
-    const Sample s = samples[b];
-    const float *sl = slow + b * V;
-    const float sSrc = sl[nearestNode(s, g)];
-    const NodeGeom n = nodeGeom(v, s, g);
+    const int b = blockIdx.z, z = blockIdx.y;
+    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
+    const int y = static_cast<int>(p / static_cast<unsigned>(g.nx)), x = static_cast<int>(p - static_cast<unsigned>(y) * g.nx);
+    if (y >= g.ny) return;
+    const float *sl = slow + b * V, *table = tables + b * tableLength(g);
+    const long long v = static_cast<long long>(z) * g.nx * g.ny + p;
+    const NodeGeom n = nodeGeom(table, g, x, y, z);
     const float invL = static_cast<float>(g.invL);
-    float f[8] = {sl[v] / sSrc - 1.f,
+    const bool inside = table[1] >= 0.f && table[1] <= static_cast<float>(g.nx - 1) && table[2] >= 0.f &&
+                        table[2] <= static_cast<float>(g.ny - 1) && table[3] >= 0.f && table[3] <= static_cast<float>(g.nz - 1);
+    float f[8] = {sl[v] / table[0] - 1.f,
                   n.dist * invL,
                   n.ddx * invL,
                   n.ddy * invL,
                   n.ddz * invL,
-                  straightRayContrast(s, sl, g, sSrc, static_cast<int>(v % g.nx), static_cast<int>((v / g.nx) % g.ny),
-                                      static_cast<int>(v / (static_cast<long long>(g.nx) * g.ny))),
+                  inside ? straightRayContrast<true>(sl, g, table, x, y, z) : straightRayContrast<false>(sl, g, table, x, y, z),
                   0.f,
                   0.f};
-    store8(feat + i * 16, f);
-    const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    store8(feat + i * 16 + 8, z);
+    store8(feat + (b * V + v) * 16, f);
+    const float zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    store8(feat + (b * V + v) * 16 + 8, zero);
 }
 
 __device__ __forceinline__ float warpSum(float v) {
@@ -486,107 +561,130 @@ __device__ __forceinline__ double warpSumD(double v) {
     return v;
 }
 
-__device__ __forceinline__ float headOut(const float (&h)[16], const float *hw) {
+__device__ __forceinline__ float headOut(const float (&h)[16], const float (&hw)[17]) {
     float o = hw[16];
+#pragma unroll
     for (int c = 0; c < 16; ++c) o += hw[c] * h[c];
     return o;
 }
 
+// Nodes of sample blockIdx.y, strided over the sample's blocks: f(node, x, y, z).
+template <class F> __device__ __forceinline__ void forNodes(const Geometry &g, F f) {
+    const unsigned nx = g.nx, ny = g.ny, V = nx * ny * static_cast<unsigned>(g.nz);   // < 2^31
+    for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+        const unsigned r = v / nx, z = r / ny;
+        f(v, static_cast<int>(v - r * nx), static_cast<int>(r - z * ny), static_cast<int>(z));
+    }
+}
+
+// Head and loss.  Bound by the activations it reads and the gradients it writes (8 x 64 x 128 x 128
+// nodes, 537 MB: 885 us with the source's FP64 geometry per node and a block per 256 nodes, each
+// adding its 18 sums to the same words, 170 now): a thread sums over many nodes, a block adds once.
 __global__ void __launch_bounds__(kThreads) headLossKernel(const bf16 *h, const float *hw, const Sample *samples,
-                                                           const float *slow, Geometry g, int B, double invN,
-                                                           float *dhw, bf16 *dpre, double *lossSum) {
+                                                           const float *tables, Geometry g, double invN, float *dhw,
+                                                           bf16 *dpre, double *lossSum) {
     __shared__ float red[kThreads / 32][17];
     __shared__ double redL[kThreads / 32];
     const long long V = static_cast<long long>(g.nx) * g.ny * g.nz;
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    float hv[16];
-    float dout = 0.f;
+    const int b = blockIdx.y;
+    const float *table = tables + b * tableLength(g);
+    const float *travelTime = samples[b].travelTime;
+    float w[17], sum[17];
+#pragma unroll
+    for (int k = 0; k < 17; ++k) {
+        w[k] = hw[k];
+        sum[k] = 0.f;
+    }
     double l = 0.0;
-    if (i < B * V) {
-        const int b = i / V;
-        const long long v = i % V;
-        const Sample s = samples[b];
-        float a[8], c[8];
+    forNodes(g, [&](unsigned v, int x, int y, int z) {
+        const long long i = b * V + v;
+        float hv[16], a[8], c[8];
         load8(a, h + i * 16);
         load8(c, h + i * 16 + 8);
+#pragma unroll
         for (int k = 0; k < 8; ++k) {
             hv[k] = a[k];
             hv[8 + k] = c[k];
         }
-        const float o = headOut(hv, hw);
-        const float T0 = slow[b * V + nearestNode(s, g)] * nodeGeom(v, s, g).dist;
+        float dout = 0.f;
+        const float o = headOut(hv, w);
+        const float T0 = table[0] * nodeGeom(table, g, x, y, z).dist;
         if (T0 > 0.f) {
-            const float tgt = s.travelTime[v] / T0 - 1.f;
+            const float tgt = travelTime[v] / T0 - 1.f;
             const float diff = o - tgt;
-            l = static_cast<double>(diff) * diff;
-            dout = static_cast<float>(2.0 * diff * invN);
+            const double d = diff;
+            l = fma(d, d, l);
+            dout = static_cast<float>(2.0 * d * invN);
         }
-        float d[8], e[8];
+#pragma unroll
         for (int k = 0; k < 8; ++k) {
-            d[k] = hv[k] > 0.f ? dout * hw[k] : 0.f;
-            e[k] = hv[8 + k] > 0.f ? dout * hw[8 + k] : 0.f;
+            a[k] = hv[k] > 0.f ? dout * w[k] : 0.f;
+            c[k] = hv[8 + k] > 0.f ? dout * w[8 + k] : 0.f;
         }
-        store8(dpre + i * 16, d);
-        store8(dpre + i * 16 + 8, e);
-    } else {
-        for (int k = 0; k < 16; ++k) hv[k] = 0.f;
-    }
+        store8(dpre + i * 16, a);
+        store8(dpre + i * 16 + 8, c);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) sum[k] += dout * hv[k];
+        sum[16] += dout;
+    });
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = 0; k < 16; ++k) {
-        const float t = warpSum(dout * hv[k]);
+#pragma unroll
+    for (int k = 0; k < 17; ++k) {
+        const float t = warpSum(sum[k]);
         if (lane == 0) red[warp][k] = t;
     }
-    const float tb = warpSum(dout);
     const double tl = warpSumD(l);
-    if (lane == 0) {
-        red[warp][16] = tb;
-        redL[warp] = tl;
-    }
+    if (lane == 0) redL[warp] = tl;
     __syncthreads();
     if (threadIdx.x < 17) {
         float s = 0.f;
-        for (int w = 0; w < kThreads / 32; ++w) s += red[w][threadIdx.x];
+        for (int q = 0; q < kThreads / 32; ++q) s += red[q][threadIdx.x];
         atomicAdd(dhw + threadIdx.x, s);
     } else if (threadIdx.x == 32) {
         double s = 0.0;
-        for (int w = 0; w < kThreads / 32; ++w) s += redL[w];
+        for (int q = 0; q < kThreads / 32; ++q) s += redL[q];
         atomicAdd(lossSum, s);
     }
 }
 
+// Predicted times (4 x 64 x 128 x 128 nodes, 151 MB: 412 us with the FP64 geometry per node, 49 now).
 __global__ void __launch_bounds__(kThreads) predictKernel(const bf16 *h, const float *hw, const Sample *samples,
-                                                          const float *slow, Geometry g, int B, float inflate,
-                                                          float *out, double *lossSum) {
+                                                          const float *tables, Geometry g, float inflate, float *out,
+                                                          double *lossSum) {
     __shared__ double redL[kThreads / 32];
     const long long V = static_cast<long long>(g.nx) * g.ny * g.nz;
-    const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+    const int b = blockIdx.y;
+    const float *table = tables + b * tableLength(g);
+    const float *travelTime = samples[b].travelTime;
+    float w[17];
+#pragma unroll
+    for (int k = 0; k < 17; ++k) w[k] = hw[k];
     double l = 0.0;
-    if (i < B * V) {
-        const int b = i / V;
-        const long long v = i % V;
-        const Sample s = samples[b];
-        float a[8], c[8], hv[16];
+    forNodes(g, [&](unsigned v, int x, int y, int z) {
+        const long long i = b * V + v;
+        float hv[16], a[8], c[8];
         load8(a, h + i * 16);
         load8(c, h + i * 16 + 8);
+#pragma unroll
         for (int k = 0; k < 8; ++k) {
             hv[k] = a[k];
             hv[8 + k] = c[k];
         }
-        const float o = headOut(hv, hw);
-        const float T0 = slow[b * V + nearestNode(s, g)] * nodeGeom(v, s, g).dist;
+        const float o = headOut(hv, w);
+        const float T0 = table[0] * nodeGeom(table, g, x, y, z).dist;
         out[i] = T0 * (1.f + o) * inflate;
-        if (lossSum && s.travelTime && T0 > 0.f) {
-            const float diff = o - (s.travelTime[v] / T0 - 1.f);
-            l = static_cast<double>(diff) * diff;
+        if (lossSum && travelTime && T0 > 0.f) {
+            const double diff = o - (travelTime[v] / T0 - 1.f);
+            l = fma(diff, diff, l);
         }
-    }
+    });
     if (!lossSum) return;
     const double t = warpSumD(l);
     if ((threadIdx.x & 31) == 0) redL[threadIdx.x >> 5] = t;
     __syncthreads();
     if (threadIdx.x == 0) {
         double s = 0.0;
-        for (int w = 0; w < kThreads / 32; ++w) s += redL[w];
+        for (int q = 0; q < kThreads / 32; ++q) s += redL[q];
         atomicAdd(lossSum, s);
     }
 }
@@ -944,66 +1042,71 @@ cudaError_t launchWGrad(const WGradArgs &a, int numSMs, cudaStream_t s) {
 }
 
 cudaError_t launchBiasGrad(const bf16 *dy, int c, long long nodes, float *db, int numSMs, cudaStream_t s) {
-    if (c < 1 || c > kThreads || kThreads % c) return cudaErrorInvalidValue;
-    const long long slots = kThreads / c;
-    long long blocks = (nodes + slots * 64 - 1) / (slots * 64);
+    if (c < 8 || c > kThreads || kThreads % c) return cudaErrorInvalidValue;
+    const long long slots = kThreads / (c / 8);
+    long long blocks = (nodes + slots * 16 - 1) / (slots * 16);
     if (blocks > 4LL * numSMs) blocks = 4LL * numSMs;
     if (blocks < 1) blocks = 1;
     biasGradKernel<<<static_cast<int>(blocks), kThreads, 0, s>>>(dy, c, nodes, db);
     return cudaGetLastError();
 }
 
+namespace {
+// Grid of the kernels over 16-byte pieces (pieceOf): W x H rows, `planes` planes.
+dim3 pieceGrid(int W, int C, int H, long long planes) {
+    return dim3((W * (C / 8) + kThreads - 1) / kThreads, H, static_cast<unsigned>(planes < 65535 ? planes : 65535));
+}
+// Blocks of a sample in the kernels with sums (forNodes): eight per SM over all samples.
+dim3 nodeGrid(const Geometry &g, int B, int numSMs) {
+    const long long all = (static_cast<long long>(g.nx) * g.ny * g.nz + kThreads - 1) / kThreads, want = (8LL * numSMs + B - 1) / B;
+    return dim3(static_cast<unsigned>(all < want ? all : want), B);
+}
+}  // namespace
+
 cudaError_t launchPool(const bf16 *x, int C, int D, int H, int W, int B, bf16 *y, cudaStream_t s) {
-    poolKernel<<<gridFor(static_cast<long long>(B) * (D / 2) * (H / 2) * (W / 2) * (C / 8)), kThreads, 0, s>>>(
-        x, C, D, H, W, B, y);
+    poolKernel<<<pieceGrid(W / 2, C, H / 2, static_cast<long long>(B) * (D / 2)), kThreads, 0, s>>>(x, C, D, H, W, B, y);
     return cudaGetLastError();
 }
 
 cudaError_t launchUpcat(const bf16 *low, int c1, const bf16 *skip, int c2, int D, int H, int W, int B, bf16 *out,
                         cudaStream_t s) {
-    upcatKernel<<<gridFor(static_cast<long long>(B) * D * H * W * ((c1 + c2) / 8)), kThreads, 0, s>>>(
-        low, c1, skip, c2, D, H, W, B, out);
+    upcatKernel<<<pieceGrid(W, c1 + c2, (H + kRowsEach - 1) / kRowsEach, static_cast<long long>(B) * D), kThreads, 0, s>>>(low, c1, skip, c2, D, H, W, B, out);
     return cudaGetLastError();
 }
 
 cudaError_t launchUpSumMask(const bf16 *dcat, int ccat, const bf16 *act, int c1, int Dl, int Hl, int Wl, int B,
                             bf16 *dpre, cudaStream_t s) {
-    upSumMaskKernel<<<gridFor(static_cast<long long>(B) * Dl * Hl * Wl * (c1 / 8)), kThreads, 0, s>>>(
-        dcat, ccat, act, c1, Dl, Hl, Wl, B, dpre);
+    upSumMaskKernel<<<pieceGrid(Wl, c1, Hl, static_cast<long long>(B) * Dl), kThreads, 0, s>>>(dcat, ccat, act, c1, Dl, Hl, Wl, B, dpre);
     return cudaGetLastError();
 }
 
 cudaError_t launchCombineSkip(const bf16 *dcat, int ccat, int c1, const bf16 *dpool, const bf16 *skip, int c2,
                               int D, int H, int W, int B, bf16 *dpre, cudaStream_t s) {
-    combineSkipKernel<<<gridFor(static_cast<long long>(B) * D * H * W * (c2 / 8)), kThreads, 0, s>>>(
-        dcat, ccat, c1, dpool, skip, c2, D, H, W, B, dpre);
+    combineSkipKernel<<<pieceGrid(W, c2, (H + kRowsEach - 1) / kRowsEach, static_cast<long long>(B) * D), kThreads, 0, s>>>(dcat, ccat, c1, dpool, skip, c2, D, H, W,
+                                                                                             B, dpre);
     return cudaGetLastError();
 }
 
-cudaError_t launchSlowness(const Sample *samples, Geometry g, int B, float *slow, cudaStream_t s) {
-    slownessKernel<<<gridFor(static_cast<long long>(B) * g.nx * g.ny * g.nz), kThreads, 0, s>>>(samples, g, B, slow);
+cudaError_t launchSlowness(const Sample *samples, Geometry g, int B, float *slow, float *tables, cudaStream_t s) {
+    slownessKernel<<<dim3(gridFor(static_cast<long long>(g.nx) * g.ny * g.nz), B), kThreads, 0, s>>>(samples, g, slow, tables);
     return cudaGetLastError();
 }
 
-cudaError_t launchFeatures(const Sample *samples, const float *slow, Geometry g, int B, bf16 *feat, cudaStream_t s) {
-    const long long n = static_cast<long long>(B) * g.nx * g.ny * g.nz;
-    featuresKernel<<<static_cast<int>((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(samples, slow, g, B, feat);
+cudaError_t launchFeatures(const float *slow, const float *tables, Geometry g, int B, bf16 *feat, cudaStream_t s) {
+    const dim3 grid(static_cast<unsigned>((static_cast<long long>(g.nx) * g.ny + kThreads - 1) / kThreads), g.nz, B);
+    featuresKernel<<<grid, kThreads, 0, s>>>(slow, tables, g, feat);
     return cudaGetLastError();
 }
 
-cudaError_t launchHeadLoss(const bf16 *h, const float *hw, const Sample *samples, const float *slow, Geometry g,
-                           int B, double invN, float *dhw, bf16 *dpre, double *lossSum, cudaStream_t s) {
-    const long long n = static_cast<long long>(B) * g.nx * g.ny * g.nz;
-    headLossKernel<<<static_cast<int>((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(h, hw, samples, slow, g, B,
-                                                                                       invN, dhw, dpre, lossSum);
+cudaError_t launchHeadLoss(const bf16 *h, const float *hw, const Sample *samples, const float *tables, Geometry g,
+                           int B, double invN, float *dhw, bf16 *dpre, double *lossSum, int numSMs, cudaStream_t s) {
+    headLossKernel<<<nodeGrid(g, B, numSMs), kThreads, 0, s>>>(h, hw, samples, tables, g, invN, dhw, dpre, lossSum);
     return cudaGetLastError();
 }
 
-cudaError_t launchPredict(const bf16 *h, const float *hw, const Sample *samples, const float *slow, Geometry g, int B,
-                          double inflate, float *out, double *lossSum, cudaStream_t s) {
-    const long long n = static_cast<long long>(B) * g.nx * g.ny * g.nz;
-    predictKernel<<<static_cast<int>((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(
-        h, hw, samples, slow, g, B, static_cast<float>(inflate), out, lossSum);
+cudaError_t launchPredict(const bf16 *h, const float *hw, const Sample *samples, const float *tables, Geometry g, int B,
+                          double inflate, float *out, double *lossSum, int numSMs, cudaStream_t s) {
+    predictKernel<<<nodeGrid(g, B, numSMs), kThreads, 0, s>>>(h, hw, samples, tables, g, static_cast<float>(inflate), out, lossSum);
     return cudaGetLastError();
 }
 
