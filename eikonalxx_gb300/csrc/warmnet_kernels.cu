@@ -281,6 +281,30 @@ __device__ __forceinline__ void store8(bf16 *p, const float (&f)[8]) {
     *reinterpret_cast<Vec8 *>(p) = v;
 }
 
+// 16 channels, 32 bytes: a whole sector in one instruction.
+__device__ __forceinline__ unsigned pack2(float a, float b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const unsigned *>(&h);
+}
+__device__ __forceinline__ void store16(bf16 *p, const float (&f)[16]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(pack2(f[0], f[1])), "r"(pack2(f[2], f[3])),
+                 "r"(pack2(f[4], f[5])), "r"(pack2(f[6], f[7])), "r"(pack2(f[8], f[9])), "r"(pack2(f[10], f[11])),
+                 "r"(pack2(f[12], f[13])), "r"(pack2(f[14], f[15]))
+                 : "memory");
+}
+__device__ __forceinline__ void load16(float (&f)[16], const bf16 *p) {
+    unsigned u[8];
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "l"(p)
+                 : "memory");
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        f[2 * k] = __uint_as_float(u[k] << 16);
+        f[2 * k + 1] = __uint_as_float(u[k] & 0xffff0000u);
+    }
+}
+
 // db[c] += sum over nodes of dy[.][c].  Bound by reading dy: a thread sums eight channels, 16 bytes
 // a node (8.4 M nodes of 16 channels: 131 us with one channel a thread, 61 now).
 __global__ void __launch_bounds__(kThreads) biasGradKernel(const bf16 *dy, int C, long long nodes, float *db) {
@@ -942,6 +966,327 @@ __global__ void __launch_bounds__(128) convTcKernel(ConvArgs a, const __grid_con
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOL) : "memory");
 }
 
+// The same convolution as a persistent kernel, where all weights and a ring of four or more input
+// planes fit in shared memory: loads, MMAs and output run at the same time, in three roles (a
+// loading thread, an issuing thread, eight output warps).  A tile is four x-rows along y; a block
+// walks tiles along z (a segment), so that a plane of six haloed rows is loaded once for the three
+// tiles that read it.
+//
+// What bounds an MMA at few channels is reading A (128 nodes of 16 channels, 4 KB), so one takes an
+// input row's A for all output rows that it reaches: row r contributes through tap dy to row r - dy,
+// and with the accumulators of the output rows side by side and the weights ordered
+// [dz][dx][dy = 2, 1, 0][channel out], the two or three taps are one operand B of two or three times
+// N columns.  That is 54 MMAs a tile instead of 108; at 68 cycles each, whatever N is, they are what
+// bounds the kernel.  With several 16-channel chunks a segment is walked once per chunk, its tiles'
+// accumulators staying in TMEM.  The output warps free the accumulators once they are in registers
+// and store whole 32-byte sectors (with 16-byte stores before the arrival: 408 us where 222 is now,
+// and 1140 where 298 is).  Every output still sums its products in the order chunk, dz, dy, dx: the
+// results are those of convTcKernel, bit for bit.  8 x 64 x 128 x 128 nodes, us, convTcKernel and now:
+// 16 to 16 channels 530, 222; 48 to 16 1137, 606; 16 to 48 1448, 298.
+namespace rows {
+constexpr int kY = 4, kIn = kY + 2, kOutWarps = 8, kThreadsR = 64 + 32 * kOutWarps, kRing = 8;
+constexpr int kGroup = (kIn * kRowB + 127) / 128 * 128;   // one 8-channel group of a plane: 12,544
+constexpr int kPlane = 2 * kGroup;
+constexpr int kSmemMax = 232448, kBarB = 512;             // shared memory per block; barriers
+template <int N> __host__ __device__ constexpr int chunkWeights() { return 2 * 27 * N * 16; }
+// columns from one tile's accumulators to the next, and how many tiles TMEM holds
+template <int N> __host__ __device__ constexpr int accStep() { return N <= 16 ? 64 : N <= 32 ? 128 : 256; }
+template <int N> __host__ __device__ constexpr int accCount() { return 512 / accStep<N>(); }
+template <int N> __host__ int ringOf(int cin) {
+    const int r = (kSmemMax - kBarB - cin / 16 * chunkWeights<N>()) / kPlane;
+    return r < kRing ? r : kRing;
+}
+
+__device__ __forceinline__ void arrive(unsigned mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ void expect(unsigned mbar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void commit(unsigned mbar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+}
+// A bounded wait that also ends when another role has given up.
+__device__ __forceinline__ bool wait(unsigned mbar, unsigned parity, long long spin, volatile int *stop) {
+    for (long long it = 0; it < spin; ++it) {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred q;\n mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n selp.u32 %0, 1, 0, q;\n}\n"
+            : "=r"(done)
+            : "r"(mbar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (*stop) return false;
+    }
+    *stop = 1;
+    return false;
+}
+
+// The MMAs of one dz: the six input rows of a plane (A at `a`, group stride kGroup) with the weights
+// at `b` onto the accumulators at `acc`; FIRST: these are the first products of every output row.
+template <int N, bool FIRST>
+__device__ __forceinline__ void issuePlane(unsigned acc, unsigned long long a, unsigned long long b) {
+#pragma unroll
+    for (int r = 0; r < kIn; ++r)
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+            const int lo = r < 2 ? 0 : r - 2, hi = r < kY ? r : kY - 1;   // output rows reached
+            const unsigned long long ad = a + static_cast<unsigned long long>((r * kRowB + dx * 16) >> 4);
+            auto part = [&](int y0, int y1, unsigned accumulate) {
+                if (y1 < y0) return;
+                const int first = dx * 3 + 2 - (r - y0);   // [dx][dy = 2, 1, 0], dy = r - y0
+                const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                                       (static_cast<unsigned>((y1 - y0 + 1) * N >> 3) << 17) | ((128u >> 4) << 24);
+                mma(acc + static_cast<unsigned>(y0 * N), ad, b + static_cast<unsigned long long>(first * N), idesc, accumulate);
+            };
+            if (FIRST && dx == 0 && r < kY) {   // row r starts here
+                part(lo, r - 1, 1u);
+                part(r, r, 0u);
+            } else {
+                part(lo, hi, 1u);
+            }
+        }
+}
+
+// A slot of the ring and the parity of its barriers' present phase.
+struct Slot {
+    int at = 0, parity = 0;
+    __device__ __forceinline__ void next(int ring) {
+        if (++at == ring) {
+            at = 0;
+            parity ^= 1;
+        }
+    }
+};
+// Segment `s`: up to `len` tiles along z from z0, of rows y0 .. y0 + 3.
+struct Segment {
+    int b, y0, z0, n;
+    __device__ __forceinline__ Segment(int s, int len, const ConvArgs &a) {
+        const int tilesY = a.H / kY, segsZ = (a.D + len - 1) / len;
+        y0 = (s % tilesY) * kY;
+        z0 = (s / tilesY) % segsZ * len;
+        b = s / tilesY / segsZ;
+        n = a.D - z0 < len ? a.D - z0 : len;
+    }
+};
+
+template <int N>
+__global__ void __launch_bounds__(kThreadsR, 1) convRowsKernel(ConvArgs a, const __grid_constant__ CUtensorMap mapX,
+                                                            const __grid_constant__ CUtensorMap mapW, int segments, int len,
+                                                            int ring) {
+    constexpr int STEP = accStep<N>(), ACCS = accCount<N>(), WC = chunkWeights<N>(), WG = WC / 2;
+    static_assert(kY * N <= STEP && (ACCS & (ACCS - 1)) == 0, "TMEM layout");
+    extern __shared__ __align__(1024) unsigned char smemRaw[];
+    const int chunks = a.cin / 16;
+    unsigned char *wsm = smemRaw + ring * kPlane;   // [chunk][2 groups][dz][dx][dy = 2, 1, 0][N][16 B]
+    const unsigned full = smemAddr(wsm + chunks * WC), empty = full + 64, accFull = full + 128, accEmpty = full + 192,
+                   wFull = full + 256, drained = full + 264;
+    unsigned *tslot = reinterpret_cast<unsigned *>(wsm + chunks * WC + 272);
+    volatile int *stop = reinterpret_cast<volatile int *>(tslot + 1);
+    volatile int *issued = stop + 1;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int co0 = blockIdx.y * N;
+    const long long spin = a.spin > 0 ? a.spin : kSpin;
+    const unsigned hb = smemAddr(smemRaw), wb = smemAddr(wsm);
+
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smemAddr(tslot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < 34; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full + 8 * k), "r"(k >= 24 && k < 32 ? kOutWarps : 1) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        *stop = 0;
+        *issued = 0;
+    }
+    fenceBefore();
+    __syncthreads();
+    fenceAfter();
+    const unsigned tmem = *tslot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            expect(wFull, static_cast<unsigned>(chunks * WC));
+            for (int c = 0; c < chunks; ++c)
+                for (int g = 0; g < 2; ++g)
+                    for (int tap = 0; tap < 27; ++tap) {
+                        const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
+                        tma3(wb + c * WC + g * WG + ((dz * 3 + dx) * 3 + 2 - dy) * N * 16, &mapW, 16 * c + 8 * g, co0, tap, wFull);
+                    }
+            Slot slot;
+            int k = 0;   // planes loaded
+            bool ok = true;
+            for (int s = blockIdx.x; s < segments && ok; s += gridDim.x) {
+                const Segment sg(s, len, a);
+                for (int c = 0; c < chunks && ok; ++c)
+                    for (int p = 0; p < sg.n + 2; ++p) {
+                        if (k >= ring && !wait(empty + 8 * slot.at, slot.parity ^ 1, spin, stop)) {
+                            ok = false;
+                            break;
+                        }
+                        expect(full + 8 * slot.at, static_cast<unsigned>(2 * kIn * kRowB + (a.testLate == 1 && k == 0 ? 16 : 0)));
+                        for (int g = 0; g < 2; ++g)
+                            tma5(hb + slot.at * kPlane + g * kGroup, &mapX, 16 * c + 8 * g, -1, sg.y0 - 1, sg.z0 - 1 + p, sg.b,
+                                 full + 8 * slot.at);
+                        *issued = ++k;
+                        slot.next(ring);
+                    }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            bool ok = wait(wFull, 0, spin, stop);
+            Slot slot;     // the next plane to arrive
+            int first = 0;   // tiles of the segments before
+            for (int s = blockIdx.x; s < segments && ok; s += gridDim.x) {
+                const Segment sg(s, len, a);
+                for (int c = 0; c < chunks && ok; ++c) {
+                    const unsigned long long bd = sdesc(wb + c * WC, WG, 128);
+                    constexpr unsigned long long bPlane = 9 * N;
+                    int s0 = 0, s1 = slot.at;   // the slots of the tile's planes z - 1 and z
+                    ok = wait(full + 8 * slot.at, slot.parity, spin, stop);
+                    slot.next(ring);
+                    int s2 = slot.at;
+                    ok = ok && wait(full + 8 * slot.at, slot.parity, spin, stop);
+                    slot.next(ring);
+                    for (int j = 0; j < sg.n && ok; ++j) {
+                        s0 = s1;
+                        s1 = s2;
+                        s2 = slot.at;
+                        ok = wait(full + 8 * slot.at, slot.parity, spin, stop);
+                        slot.next(ring);
+                        const int t = first + j, at = t & (ACCS - 1);
+                        if (ok && c == 0 && t >= ACCS) ok = wait(accEmpty + 8 * at, (t / ACCS + 1) & 1, spin, stop);
+                        if (!ok) break;
+                        fenceAfter();
+                        const unsigned acc = tmem + static_cast<unsigned>(at * STEP);
+                        const unsigned long long d0 = sdesc(hb + s0 * kPlane, kGroup, 128);
+                        if (c == 0) issuePlane<N, true>(acc, d0, bd);
+                        else issuePlane<N, false>(acc, d0, bd);
+#pragma unroll 1
+                        for (int dz = 1; dz < 3; ++dz)
+                            issuePlane<N, false>(acc, sdesc(hb + (dz == 1 ? s1 : s2) * kPlane, kGroup, 128), bd + dz * bPlane);
+                        commit(empty + 8 * s0);   // once they have read it
+                        if (j == sg.n - 1) {
+                            commit(empty + 8 * s1);
+                            commit(empty + 8 * s2);
+                        }
+                        if (c == chunks - 1 && !(a.testLate == 2 && t == 0)) commit(accFull + 8 * at);
+                    }
+                }
+                first += sg.n;
+            }
+        }
+    } else {
+        // warp w reads TMEM lanes 32 (w & 3) .., the first four warps rows 0 and 1, the others 2 and 3
+        const int q = warp & 3, x = q * 32 + lane, yFirst = warp < 6 ? 0 : 2;
+        float bias[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) bias[j] = a.bias ? a.bias[co0 + j] : 0.f;
+        int t = 0;
+        bool ok = true;
+        for (int s = blockIdx.x; s < segments && ok; s += gridDim.x) {
+            const Segment sg(s, len, a);
+            for (int j = 0; j < sg.n; ++j, ++t) {
+                const int at = t & (ACCS - 1);
+                ok = __all_sync(0xffffffffu, wait(accFull + 8 * at, (t / ACCS) & 1, spin, stop));
+                if (!ok) break;
+                fenceAfter();
+                // both rows into registers, the accumulators free at once, then the output
+                unsigned r[2 * N];
+#pragma unroll
+                for (int c0 = 0; c0 < 2 * N; c0 += 16)
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                        : "=r"(r[c0]), "=r"(r[c0 + 1]), "=r"(r[c0 + 2]), "=r"(r[c0 + 3]), "=r"(r[c0 + 4]), "=r"(r[c0 + 5]),
+                          "=r"(r[c0 + 6]), "=r"(r[c0 + 7]), "=r"(r[c0 + 8]), "=r"(r[c0 + 9]), "=r"(r[c0 + 10]), "=r"(r[c0 + 11]),
+                          "=r"(r[c0 + 12]), "=r"(r[c0 + 13]), "=r"(r[c0 + 14]), "=r"(r[c0 + 15])
+                        : "r"(tmem + ((static_cast<unsigned>(q) * 32u) << 16) + static_cast<unsigned>(at * STEP + yFirst * N + c0))
+                        : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                fenceBefore();
+                __syncwarp();
+                if (lane == 0) arrive(accEmpty + 8 * at);
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    const long long node = ((static_cast<long long>(sg.b) * a.D + sg.z0 + j) * a.H + sg.y0 + yFirst + y) * 128 + x;
+#pragma unroll
+                    for (int c0 = 0; c0 < N; c0 += 16) {
+                        float v[16];
+#pragma unroll
+                        for (int k = 0; k < 16; ++k) {
+                            v[k] = __uint_as_float(r[y * N + c0 + k]);
+                            if (a.bias) v[k] += bias[c0 + k];
+                            if (a.relu) v[k] = fmaxf(v[k], 0.f);
+                        }
+                        if (a.mask) {
+                            float m[16];
+                            load16(m, a.mask + node * a.cout + co0 + c0);
+#pragma unroll
+                            for (int k = 0; k < 16; ++k)
+                                if (!(m[k] > 0.f)) v[k] = 0.f;
+                        }
+                        store16(a.y + node * a.cout + co0 + c0, v);
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();
+    __syncthreads();
+    if (*stop) {
+        // A wait ran out: the block leaves only when its copies have landed and its MMAs are done
+        // (waits again, kDrain times as long; the test hook's late bytes and completion come now).
+        constexpr long long kDrain = 64;
+        if (tid == 0) {
+            if (a.testLate == 1)
+                asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(full), "r"(16u) : "memory");
+            waitParity(wFull, 0, kDrain * spin);
+            const int n = *issued;
+            for (int k = n > ring ? n - ring : 0; k < n; ++k) waitParity(full + 8 * (k % ring), (k / ring) & 1, kDrain * spin);
+            if (a.status) atomicExch(a.status, 1);
+        } else if (tid == 32) {
+            commit(drained);
+            waitParity(drained, 0, kDrain * spin);
+        }
+    }
+    fenceBefore();
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+template <int N>
+cudaError_t launch(const ConvArgs &a, const CUtensorMap &mapX, const CUtensorMap &mapW, cudaStream_t s) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int ring = ringOf<N>(a.cin), smem = ring * kPlane + a.cin / 16 * chunkWeights<N>() + kBarB;
+    // the shared-memory limit is a per-device attribute: set it for the current device
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(convRowsKernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    // Tiles per segment: with several chunks as many as TMEM holds; with one, what leaves the blocks
+    // least to do (two planes more per segment, about half a tile's time each).
+    auto segmentsOf = [&](int len) { return static_cast<long long>(a.B) * (a.H / kY) * ((a.D + len - 1) / len); };
+    int len = accCount<N>();
+    if (a.cin == 16) {
+        long long best = 0;
+        for (int l = 4; l <= 64; l += 4) {
+            const long long cost = (segmentsOf(l) + sms - 1) / sms * (l + 1);
+            if (!best || cost < best) {
+                best = cost;
+                len = l;
+            }
+        }
+    }
+    const long long segments = segmentsOf(len);
+    if (segments > 2147483647LL - 65536) return cudaErrorInvalidValue;
+    const dim3 grid(static_cast<unsigned>(segments < sms ? segments : sms), a.cout / N);
+    convRowsKernel<N><<<grid, kThreadsR, smem, s>>>(a, mapX, mapW, static_cast<int>(segments), len, ring);
+    return cudaGetLastError();
+}
+}  // namespace rows
+
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -962,26 +1307,29 @@ template <int N>
 cudaError_t launchTc(const ConvArgs &a, cudaStream_t s) {
     EncodeTiled enc = encodeTiled();
     if (!enc) return cudaErrorNotSupported;
-    // activations [B][D][H][128][cin] BF16: box of 8 channels x 130 nodes x 6 rows x 4 planes x 1 sample
+    const bool rowsFit = rows::ringOf<N>(a.cin) >= 4;
+    // activations [B][D][H][128][cin] BF16: box of 8 channels x 130 nodes x 6 rows x 4 planes (1) x 1 sample
     CUtensorMap mapX, mapW;
     const cuuint64_t dimX[5] = {static_cast<cuuint64_t>(a.cin), 128, static_cast<cuuint64_t>(a.H),
                                 static_cast<cuuint64_t>(a.D), static_cast<cuuint64_t>(a.B)};
     const cuuint64_t strideX[4] = {static_cast<cuuint64_t>(a.cin) * 2, 128ull * a.cin * 2,
                                    static_cast<cuuint64_t>(a.H) * 128 * a.cin * 2,
                                    static_cast<cuuint64_t>(a.D) * a.H * 128 * a.cin * 2};
-    const cuuint32_t boxX[5] = {8, kXN, kHY, kHZ, 1}, ones[5] = {1, 1, 1, 1, 1};
+    const cuuint32_t boxX[5] = {8, kXN, kHY, static_cast<cuuint32_t>(rowsFit ? 1 : kHZ), 1}, ones[5] = {1, 1, 1, 1, 1};
+    static_assert(kHY == rows::kIn, "one box height");
     if (enc(&mapX, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16 *>(a.x), dimX, strideX, boxX, ones,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    // weights [27][cout][cin] BF16: box of 8 channels in x N channels out x 27 taps
+    // weights [27][cout][cin] BF16: box of 8 channels in x N channels out x 27 taps (1 tap)
     const cuuint64_t dimW[3] = {static_cast<cuuint64_t>(a.cin), static_cast<cuuint64_t>(a.cout), 27};
     const cuuint64_t strideW[2] = {static_cast<cuuint64_t>(a.cin) * 2, static_cast<cuuint64_t>(a.cout) * a.cin * 2};
-    const cuuint32_t boxW[3] = {8, static_cast<cuuint32_t>(N), 27};
+    const cuuint32_t boxW[3] = {8, static_cast<cuuint32_t>(N), rowsFit ? 1u : 27u};
     if (enc(&mapW, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16 *>(a.w), dimW, strideW, boxW, ones,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
+    if (rowsFit) return rows::launch<N>(a, mapX, mapW, s);
     // the shared-memory limit is a per-device attribute: set it for the current device
     cudaError_t e = cudaFuncSetAttribute(convTcKernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes<N>());
     if (e != cudaSuccess) return e;
