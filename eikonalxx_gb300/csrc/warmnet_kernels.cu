@@ -2,17 +2,17 @@
 //
 // The 3x3x3 convolutions are implicit GEMMs on the BF16 tensor cores with FP32
 // accumulation.  Levels whose x-rows hold 128 nodes run on tcgen05 (TMA staging, TMEM
-// accumulators; convTcKernel below); the others on mma.sync m16n8k16:
+// accumulators; convRowsKernel and convTcKernel below); the others on mma.sync m16n8k16:
 //   * forward and input-gradient: M = output nodes (one 16-node x-row per MMA row block),
 //     N = output channels, K = 27 taps x input channels.  A block stages a haloed
 //     4 x 10 x 18-node tile of 16 input channels and the 27-tap weight slice of its
 //     output channels in shared memory (cp.async, zero fill outside the grid); every
 //     tap's A operand is an ldmatrix from the shifted halo, so each input value is read
 //     from global memory once per block;
-//   * weight gradient: M = output channels, N = 16 input channels, K = nodes; the A
+//   * weight gradient: M = 16 output channels, N = 16 input channels, K = nodes; the A
 //     operand (dy transposed) and the B operand (shifted input) come from the same two
 //     tiles through ldmatrix.trans; each block loops over node tiles and adds its partial
-//     sums to the FP32 gradient with one atomic per element at the end.
+//     sums to the FP32 gradient with one atomic per warp and element at the end.
 // Shared-memory rows are 48 bytes (an odd number of 16-byte segments), so the eight row
 // addresses of every ldmatrix phase fall in distinct banks.
 #include <cuda.h>
@@ -44,12 +44,6 @@ __device__ __forceinline__ void ldsm4(unsigned (&r)[4], const void *p) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(smemAddr(p)));
 }
-__device__ __forceinline__ void ldsm4t(unsigned (&r)[4], const void *p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(smemAddr(p)));
-}
-
 __device__ __forceinline__ void mma16816(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
@@ -175,92 +169,133 @@ __global__ void __launch_bounds__(kThreads) convKernel(ConvArgs a) {
     }
 }
 
-// Weight gradient.  A warp owns one 16-channel block cb of dy and 4 consecutive taps:
-// its 4 accumulators are 16 (co) x 16 (ci) blocks of dw that share the dy^T operand, so
-// each 16-node row loads it once for 4 taps.  Warp w of block y is warp group
-// g = y * 8 + w: cb = g / kTapGroups, taps 4 * (g % kTapGroups) + 0..3 (< 27).  grid.z
-// walks the 16-channel input chunks, grid.x strides over the node tiles of all samples.
-constexpr int kUnitsPerWarp = 4;
-constexpr int kTapGroups = (27 + kUnitsPerWarp - 1) / kUnitsPerWarp;   // 7
-__global__ void __launch_bounds__(kThreads) wgradKernel(WGradArgs a) {
-    extern __shared__ __align__(16) unsigned char smemRaw[];
-    bf16 *xs = reinterpret_cast<bf16 *>(smemRaw);
-    bf16 *dys = xs + kHaloNodes * kRowHalfs;
+// Weight gradient.  A block sums, over its share of the node tiles, the 27 x 16 (co) x 16 (ci) values
+// of one block of output channels (blockIdx.y) and one of input channels (blockIdx.z).  Warp w takes
+// the taps of one dz = w % 3 on the tile's plane tz = w / 3: nine accumulators of 16 x 16.  Down the
+// plane's rows along y a row of dy (operand A, transposed) meets three rows of x at three shifts along
+// x (operand B), and two of those rows were there for the row of dy before: three new fragments of x
+// and one of dy for 18 MMAs.  What bounds it is shared memory (ldmatrix) with the copies' latency, so
+// a tile's copies run while the one before is worked on.  8 x 64 x 128 x 128 nodes, 16 to 16 and 48
+// to 16 channels: 620 and 2134 us with four taps a warp (five fragments for eight MMAs), their
+// addresses formed per tap and row and more blocks than fit; 450 and 1355 with constant offsets and
+// the resident blocks; 354 and 1044 now.
+constexpr int kWgThreads = 192;
+constexpr int kWgRowB = kRowHalfs * 2, kWgXB = kHaloNodes * kWgRowB, kWgBufB = kWgXB + 256 * kWgRowB;
+constexpr int kWgX = (2 * kHaloNodes + kWgThreads - 1) / kWgThreads, kWgDy = (512 + kWgThreads - 1) / kWgThreads;   // 16-byte pieces a thread
+__device__ __forceinline__ void ldsm4tAt(unsigned (&r)[4], unsigned a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a)
+                 : "memory");
+}
+__device__ __forceinline__ void cpAsync16At(unsigned dst, const void *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__global__ void __launch_bounds__(kWgThreads, 2) wgradKernel(WGradArgs a) {
+    extern __shared__ __align__(16) unsigned char smemRaw[];   // two buffers: [x halo][dy]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int li = lane >> 3, lj = lane & 7;
-    const int ci0 = blockIdx.z * 16;
-    const int group = blockIdx.y * (kThreads / 32) + warp;
-    const int cb = group / kTapGroups, tap0 = kUnitsPerWarp * (group % kTapGroups);
-    const bool warpActive = cb < a.cout / 16;
-    const int dyRow = a.cout + 8;   // halfs; an odd number of 16-byte segments
+    const int co0 = blockIdx.y * 16, ci0 = blockIdx.z * 16;
+    const int dz = warp % 3, tz = warp / 3;
     const long long V = static_cast<long long>(a.D) * a.H * a.W;
     const int tps = tilesPerSample(a.D, a.H, a.W);
     const int nTiles = tps * a.B;
+    const unsigned smem = smemAddr(smemRaw);
 
-    float acc[kUnitsPerWarp][2][4];
+    float acc[9][2][4];
 #pragma unroll
-    for (int i = 0; i < kUnitsPerWarp; ++i)
+    for (int i = 0; i < 9; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.f;
 
-    for (int t = blockIdx.x; t < nTiles; t += gridDim.x) {
+    // the halo nodes that this thread copies one half of: x, y, z in bytes
+    const int half = threadIdx.x & 1;
+    int place[kWgX];
+#pragma unroll
+    for (int i = 0; i < kWgX; ++i) {
+        const int hv = (threadIdx.x + i * kWgThreads) >> 1;
+        place[i] = hv % kHaloX | (hv / kHaloX % kHaloY) << 8 | hv / (kHaloX * kHaloY) << 16;
+    }
+    const unsigned xTo = smem + (threadIdx.x >> 1) * kWgRowB + 16 * half, dyTo = xTo + kWgXB;
+    auto stage = [&](int t, unsigned buf) {
         const int b = t / tps;
         const TileCoord c = tileOf(t % tps, a.D, a.H, a.W);
-        stageHalo(xs, a.x + b * V * a.cin, a.cin, ci0, c, a.D, a.H, a.W, a.x);
-        const int pieces = a.cout / 8;
-        for (int p = threadIdx.x; p < 256 * pieces; p += kThreads) {
-            const int node = p / pieces, piece = p % pieces;
-            const int r = node >> 4, xx = node & 15;
-            const int gz = c.gz0 + (r >> 3), gy = c.gy0 + (r & 7), gx = c.gx0 + xx;
-            const bool in = gz < a.D && gy < a.H && gx < a.W;
-            const bf16 *src =
-                in ? a.dy + (b * V + (static_cast<long long>(gz) * a.H + gy) * a.W + gx) * a.cout + 8 * piece : a.dy;
-            cpAsync16(dys + node * dyRow + 8 * piece, src, in);
-        }
-        cpAsyncCommitWaitAll();
-        __syncthreads();
-        if (warpActive) {
-#pragma unroll 2
-            for (int r = 0; r < 16; ++r) {
-                const int tz = r >> 3, ty = r & 7;
-                // A = dy^T: matrix li = (co 16cb + 8*(li&1) .., nodes 16r + 8*(li>>1) ..)
-                unsigned afr[4];
-                ldsm4t(afr, dys + (16 * r + lj + 8 * (li >> 1)) * dyRow + 16 * cb + 8 * (li & 1));
+        const bf16 *xb = a.x + (b * V + (static_cast<long long>(c.gz0 - 1) * a.H + c.gy0 - 1) * a.W + c.gx0 - 1) * a.cin + ci0 + 8 * half;
 #pragma unroll
-                for (int kk = 0; kk < kUnitsPerWarp; ++kk) {
-                    const int tap = tap0 + kk;
-                    if (tap >= 27) continue;
-                    const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-                    // B = shifted input: matrix li = (nodes 8*(li&1) .., channels 8*(li>>1) ..)
-                    unsigned bfr[4];
-                    ldsm4t(bfr, xs + (((tz + dz) * kHaloY + ty + dy) * kHaloX + lj + 8 * (li & 1) + dx) * kRowHalfs +
-                                    8 * (li >> 1));
-                    mma16816(acc[kk][0], afr, bfr[0], bfr[1]);
-                    mma16816(acc[kk][1], afr, bfr[2], bfr[3]);
+        for (int i = 0; i < kWgX; ++i) {
+            const int hx = place[i] & 255, hy = place[i] >> 8 & 255, hz = place[i] >> 16;
+            const bool in = static_cast<unsigned>(c.gx0 - 1 + hx) < static_cast<unsigned>(a.W) &&
+                            static_cast<unsigned>(c.gy0 - 1 + hy) < static_cast<unsigned>(a.H) &&
+                            static_cast<unsigned>(c.gz0 - 1 + hz) < static_cast<unsigned>(a.D);
+            if (i + 1 < kWgX || threadIdx.x < 2 * kHaloNodes - (kWgX - 1) * kWgThreads)
+                cpAsync16At(xTo + buf + i * (kWgThreads / 2) * kWgRowB,
+                            in ? xb + ((static_cast<long long>(hz) * a.H + hy) * a.W + hx) * a.cin : a.x, in);
+        }
+        const bf16 *db = a.dy + (b * V + (static_cast<long long>(c.gz0) * a.H + c.gy0) * a.W + c.gx0) * a.cout + co0 + 8 * half;
+#pragma unroll
+        for (int i = 0; i < kWgDy; ++i) {
+            const int node = (threadIdx.x + i * kWgThreads) >> 1, z = node >> 7, y = node >> 4 & 7, x = node & 15;
+            const bool in = c.gz0 + z < a.D && c.gy0 + y < a.H && c.gx0 + x < a.W;
+            if (node < 256)
+                cpAsync16At(dyTo + buf + i * (kWgThreads / 2) * kWgRowB,
+                            in ? db + ((static_cast<long long>(z) * a.H + y) * a.W + x) * a.cout : a.dy, in);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    // B: matrix li = (nodes 8*(li&1) .., channels 8*(li>>1) ..); A: (co 8*(li&1) .., nodes 8*(li>>1) ..)
+    const unsigned bAt = smem + (((tz + dz) * kHaloY * kHaloX + lj + 8 * (li & 1)) * kWgRowB + 16 * (li >> 1));
+    const unsigned aAt = smem + kWgXB + (128 * tz + lj + 8 * (li >> 1)) * kWgRowB + 16 * (li & 1);
+
+    unsigned buf = 0;
+    if (static_cast<int>(blockIdx.x) < nTiles) stage(blockIdx.x, 0);
+    for (int t = blockIdx.x; t < nTiles; t += gridDim.x) {
+        const int next = t + gridDim.x;
+        if (next < nTiles) {
+            stage(next, kWgBufB - buf);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        __syncthreads();
+        unsigned x[3][3][4];   // [row mod 3][dx]
+        auto row = [&](int hy) {
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) ldsm4tAt(x[hy % 3][dx], bAt + buf + (hy * kHaloX + dx) * kWgRowB);
+        };
+        row(0);
+        row(1);
+#pragma unroll
+        for (int ty = 0; ty < kTileY; ++ty) {
+            row(ty + 2);
+            unsigned d[4];
+            ldsm4tAt(d, aAt + buf + 16 * ty * kWgRowB);
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx) {
+                    const unsigned(&f)[4] = x[(ty + dy) % 3][dx];
+                    mma16816(acc[3 * dy + dx][0], d, f[0], f[1]);
+                    mma16816(acc[3 * dy + dx][1], d, f[2], f[3]);
                 }
-            }
         }
         __syncthreads();
+        buf = kWgBufB - buf;
     }
-    if (!warpActive) return;
 #pragma unroll
-    for (int kk = 0; kk < kUnitsPerWarp; ++kk) {
-        const int tap = tap0 + kk;
-        if (tap >= 27) continue;
+    for (int k = 0; k < 9; ++k)
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
             const int ci = ci0 + 8 * nt + 2 * (lane & 3);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int co = 16 * cb + (lane >> 2) + 8 * h;
-                float *d = a.dw + (static_cast<long long>(tap) * a.cout + co) * a.cin + ci;
-                atomicAdd(d, acc[kk][nt][2 * h]);
-                atomicAdd(d + 1, acc[kk][nt][2 * h + 1]);
+                const int co = co0 + (lane >> 2) + 8 * h;
+                float *d = a.dw + (static_cast<long long>(9 * dz + k) * a.cout + co) * a.cin + ci;
+                atomicAdd(d, acc[k][nt][2 * h]);
+                atomicAdd(d + 1, acc[k][nt][2 * h + 1]);
             }
         }
-    }
 }
 
 struct alignas(16) Vec8 {
@@ -1376,16 +1411,17 @@ cudaError_t launchConv(const ConvArgs &a, cudaStream_t s) {
 
 cudaError_t launchWGrad(const WGradArgs &a, int numSMs, cudaStream_t s) {
     if (a.cin % 16 || a.cout % 16 || a.B < 1) return cudaErrorInvalidValue;
-    const int smem = (kHaloNodes * kRowHalfs + 256 * (a.cout + 8)) * static_cast<int>(sizeof(bf16));
+    const int smem = 2 * kWgBufB;
     // the shared-memory limit is a per-device attribute: set it for the current device
     cudaError_t e = cudaFuncSetAttribute(wgradKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const int warpsPerBlock = kThreads / 32;
-    const int gy = (kTapGroups * (a.cout / 16) + warpsPerBlock - 1) / warpsPerBlock, gz = a.cin / 16;
+    const int gy = a.cout / 16, gz = a.cin / 16;
     const int nTiles = tilesPerSample(a.D, a.H, a.W) * a.B;
-    int gx = (4 * numSMs + gy * gz - 1) / (gy * gz);
+    // as many blocks as are resident (two per SM): a block's share of the tiles is fixed, so a second
+    // wave takes as long as the first
+    int gx = 2 * numSMs / (gy * gz);
     gx = gx < 1 ? 1 : (gx > nTiles ? nTiles : gx);
-    wgradKernel<<<dim3(gx, gy, gz), kThreads, smem, s>>>(a);
+    wgradKernel<<<dim3(gx, gy, gz), kWgThreads, smem, s>>>(a);
     return cudaGetLastError();
 }
 
