@@ -6,15 +6,15 @@
 //   * forward and input-gradient: M = output nodes (one 16-node x-row per MMA row block),
 //     N = output channels, K = 27 taps x input channels.  A block stages a haloed
 //     4 x 10 x 18-node tile of 16 input channels and the 27-tap weight slice of its
-//     output channels in shared memory (cp.async, zero fill outside the grid); every
-//     tap's A operand is an ldmatrix from the shifted halo, so each input value is read
-//     from global memory once per block;
+//     output channels in shared memory (cp.async, zero fill outside the grid), and the A
+//     operands are ldmatrix loads from the shifted halo, so each input value is read from
+//     global memory once per block;
 //   * weight gradient: M = 16 output channels, N = 16 input channels, K = nodes; the A
 //     operand (dy transposed) and the B operand (shifted input) come from the same two
 //     tiles through ldmatrix.trans; each block loops over node tiles and adds its partial
 //     sums to the FP32 gradient with one atomic per warp and element at the end.
-// Shared-memory rows are 48 bytes (an odd number of 16-byte segments), so the eight row
-// addresses of every ldmatrix phase fall in distinct banks.
+// Shared-memory rows are 48 bytes (an odd number of 16-byte segments) or 32 bytes with their halves
+// swapped in turn, so the eight row addresses of every ldmatrix phase fall in distinct banks.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -29,21 +29,10 @@ __device__ __forceinline__ unsigned smemAddr(const void *p) {
 }
 
 // 16-byte global -> shared copy; zero fill when !valid (src is then not read).
-__device__ __forceinline__ void cpAsync16(void *dst, const void *src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smemAddr(dst)), "l"(src),
-                 "r"(valid ? 16 : 0));
-}
-__device__ __forceinline__ void cpAsyncCommitWaitAll() {
-    asm volatile("cp.async.commit_group;\n" ::);
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+__device__ __forceinline__ void cpAsync16At(unsigned dst, const void *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-
-__device__ __forceinline__ void ldsm4(unsigned (&r)[4], const void *p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(smemAddr(p)));
-}
 __device__ __forceinline__ void mma16816(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
@@ -69,78 +58,101 @@ __host__ __device__ inline int tilesPerSample(int D, int H, int W) {
     return ((D + kTileZ - 1) / kTileZ) * ((H + kTileY - 1) / kTileY) * ((W + kTileX - 1) / kTileX);
 }
 
-// Stage 16 channels (ci0..ci0+15) of the haloed input tile: node (hz, hy, hx) of the
-// halo at row (hz*kHaloY + hy)*kHaloX + hx, zero outside the grid.
-__device__ __forceinline__ void stageHalo(bf16 *xs, const bf16 *xb, int cin, int ci0, TileCoord c, int D, int H,
-                                          int W, const bf16 *anyValid) {
-    for (int p = threadIdx.x; p < kHaloNodes * 2; p += kThreads) {
-        const int hv = p >> 1, half = p & 1;
-        const int hx = hv % kHaloX, hy = (hv / kHaloX) % kHaloY, hz = hv / (kHaloX * kHaloY);
-        const int gx = c.gx0 - 1 + hx, gy = c.gy0 - 1 + hy, gz = c.gz0 - 1 + hz;
-        const bool in = gx >= 0 && gx < W && gy >= 0 && gy < H && gz >= 0 && gz < D;
-        const bf16 *src = in ? xb + ((static_cast<long long>(gz) * H + gy) * W + gx) * cin + ci0 + 8 * half : anyValid;
-        cpAsync16(xs + hv * kRowHalfs + 8 * half, src, in);
-    }
+// Forward and input-gradient convolution on mma.sync.  A warp owns four x-rows of the tile along y.
+// Per dz it loads the six haloed rows that they read, at three shifts along x, as 18 A fragments, and
+// every tap's weights (operand B) meet four of them: 18 fragments of x and 18 of weights (N = 32) for
+// 144 MMAs, where a warp of two rows loading A anew for every tap took 108 of each kind.  Rows of 16
+// channels are 32 bytes in shared memory, the two halves swapped where bit 2 of the node (weights:
+// channel) is set, so that eight consecutive rows fall in distinct banks at any shift; haloed rows
+// are 24 nodes apart.  Sums run over chunk, dz, dy, dx.  8 x 32 x 64 x 64 nodes, us: 32 to 32 channels
+// 216, 155 now; 96 to 32 611, 419 now.
+constexpr int kCvThreads = 128, kCvRow = 24 * 32, kCvHaloB = kHaloZ * kHaloY * kCvRow;
+__device__ __forceinline__ void ldsm4At(unsigned (&r)[4], unsigned a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a)
+                 : "memory");
 }
-
 template <int NB>
-__global__ void __launch_bounds__(kThreads) convKernel(ConvArgs a) {
-    extern __shared__ __align__(16) unsigned char smemRaw[];
-    bf16 *xs = reinterpret_cast<bf16 *>(smemRaw);
-    bf16 *wsm = xs + kHaloNodes * kRowHalfs;
+__global__ void __launch_bounds__(kCvThreads, 3) convKernel(ConvArgs a) {
+    extern __shared__ __align__(128) unsigned char smemRaw[];   // [halo][weights: tap, channel out]
+    const unsigned xAt = smemAddr(smemRaw), wAt = xAt + kCvHaloB;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const TileCoord c = tileOf(blockIdx.x, a.D, a.H, a.W);
     const int b = blockIdx.z, co0 = blockIdx.y * NB;
     const long long V = static_cast<long long>(a.D) * a.H * a.W;
-    const bf16 *xb = a.x + b * V * a.cin;
+    const bf16 *xb = a.x + (b * V + (static_cast<long long>(c.gz0 - 1) * a.H + c.gy0 - 1) * a.W + c.gx0 - 1) * a.cin;
 
-    float acc[2][NB / 8][4];
+    float acc[4][NB / 8][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < NB / 8; ++j)
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.f;
 
     const int li = lane >> 3, lj = lane & 7;
+    const int tz = warp >> 1, ty0 = 4 * (warp & 1);
+    // A: matrix li = (nodes 8*(li&1) .. of the shifted row, k half li>>1)
+    unsigned aAt[3];
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx) {
+        const int hx = lj + 8 * (li & 1) + dx;
+        aAt[dx] = xAt + (tz * kHaloY + ty0) * kCvRow + hx * 32 + 16 * ((li >> 1) ^ (hx >> 2 & 1));
+    }
+    // B: matrix li = (channels 16p + 8*(li>>1) .. +7, k half li&1)
+    const unsigned bAt = wAt + (lj + 8 * (li >> 1)) * 32 + 16 * ((li & 1) ^ (lj >> 2 & 1));
+    const int half = threadIdx.x & 1;
     for (int ci0 = 0; ci0 < a.cin; ci0 += 16) {
-        stageHalo(xs, xb, a.cin, ci0, c, a.D, a.H, a.W, a.x);
-        for (int p = threadIdx.x; p < 27 * NB * 2; p += kThreads) {
-            const int row = p >> 1, half = p & 1;   // row = tap * NB + co
-            const int tap = row / NB, co = row % NB;
-            cpAsync16(wsm + row * kRowHalfs + 8 * half,
-                      a.w + (static_cast<long long>(tap) * a.cout + co0 + co) * a.cin + ci0 + 8 * half, true);
+#pragma unroll
+        for (int i = 0; i < (2 * kHaloNodes + kCvThreads - 1) / kCvThreads; ++i) {
+            const int hv = (threadIdx.x + i * kCvThreads) >> 1;
+            const int hx = hv % kHaloX, hr = hv / kHaloX, hy = hr % kHaloY, hz = hr / kHaloY;
+            const bool in = static_cast<unsigned>(c.gx0 - 1 + hx) < static_cast<unsigned>(a.W) &&
+                            static_cast<unsigned>(c.gy0 - 1 + hy) < static_cast<unsigned>(a.H) &&
+                            static_cast<unsigned>(c.gz0 - 1 + hz) < static_cast<unsigned>(a.D);
+            if (hv < kHaloNodes)
+                cpAsync16At(xAt + hr * kCvRow + hx * 32 + 16 * (half ^ (hx >> 2 & 1)),
+                            in ? xb + ((static_cast<long long>(hz) * a.H + hy) * a.W + hx) * a.cin + ci0 + 8 * half : a.x, in);
         }
-        cpAsyncCommitWaitAll();
+#pragma unroll
+        for (int i = 0; i < (27 * NB * 2 + kCvThreads - 1) / kCvThreads; ++i) {
+            const int row = (threadIdx.x + i * kCvThreads) >> 1, tap = row / NB, co = row % NB;   // row = tap * NB + co
+            if (row < 27 * NB)
+                cpAsync16At(wAt + row * 32 + 16 * (half ^ (row >> 2 & 1)),
+                            a.w + (static_cast<long long>(tap) * a.cout + co0 + co) * a.cin + ci0 + 8 * half, true);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();
 #pragma unroll 1
-        for (int tap = 0; tap < 27; ++tap) {
-            const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-            // B fragments: matrix li of ldmatrix.x4 = (channels 16p + 8*(li>>1) .. +7, k half li&1)
-            unsigned bfr[NB / 16][4];
+        for (int dz = 0; dz < 3; ++dz) {
+            unsigned x[6][3][4];   // [row][dx]
 #pragma unroll
-            for (int p = 0; p < NB / 16; ++p)
-                ldsm4(bfr[p], wsm + (tap * NB + 16 * p + lj + 8 * (li >> 1)) * kRowHalfs + 8 * (li & 1));
+            for (int r = 0; r < 6; ++r)
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                const int r = warp * 2 + mt, tz = r >> 3, ty = r & 7;
-                // A fragment: matrix li = (nodes 8*(li&1) .. +7 of the x-row, k half li>>1)
-                unsigned afr[4];
-                ldsm4(afr, xs + (((tz + dz) * kHaloY + ty + dy) * kHaloX + lj + 8 * (li & 1) + dx) * kRowHalfs +
-                               8 * (li >> 1));
+                for (int dx = 0; dx < 3; ++dx) ldsm4At(x[r][dx], aAt[dx] + (dz * kHaloY + r) * kCvRow);
 #pragma unroll
-                for (int nt = 0; nt < NB / 8; ++nt)
-                    mma16816(acc[mt][nt], afr, bfr[nt >> 1][(nt & 1) * 2], bfr[nt >> 1][(nt & 1) * 2 + 1]);
-            }
+            for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+                for (int dx = 0; dx < 3; ++dx) {
+                    unsigned w[NB / 16][4];
+#pragma unroll
+                    for (int p = 0; p < NB / 16; ++p) ldsm4At(w[p], bAt + ((9 * dz + 3 * dy + dx) * NB + 16 * p) * 32);
+#pragma unroll
+                    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+                        for (int nt = 0; nt < NB / 8; ++nt)
+                            mma16816(acc[mt][nt], x[mt + dy][dx], w[nt >> 1][(nt & 1) * 2], w[nt >> 1][(nt & 1) * 2 + 1]);
+                }
         }
         __syncthreads();
     }
 
     // Epilogue: accumulator (row lane/4 [+8], columns 2*(lane%4), +1) of each 16x8 block.
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-        const int r = warp * 2 + mt;
-        const int gz = c.gz0 + (r >> 3), gy = c.gy0 + (r & 7);
+    for (int mt = 0; mt < 4; ++mt) {
+        const int gz = c.gz0 + tz, gy = c.gy0 + ty0 + mt;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int gx = c.gx0 + (lane >> 2) + 8 * h;
@@ -188,11 +200,8 @@ __device__ __forceinline__ void ldsm4tAt(unsigned (&r)[4], unsigned a) {
                  : "r"(a)
                  : "memory");
 }
-__device__ __forceinline__ void cpAsync16At(unsigned dst, const void *src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
 __global__ void __launch_bounds__(kWgThreads, 2) wgradKernel(WGradArgs a) {
-    extern __shared__ __align__(16) unsigned char smemRaw[];   // two buffers: [x halo][dy]
+    extern __shared__ __align__(128) unsigned char smemRaw[];   // two buffers: [x halo][dy]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int li = lane >> 3, lj = lane & 7;
     const int co0 = blockIdx.y * 16, ci0 = blockIdx.z * 16;
@@ -1382,12 +1391,12 @@ int gridFor(long long n, int cap = 1 << 20) {
 
 template <int NB>
 cudaError_t convOne(const ConvArgs &a, cudaStream_t s) {
-    const int smem = (kHaloNodes + 27 * NB) * kRowHalfs * static_cast<int>(sizeof(bf16));
+    const int smem = kCvHaloB + 27 * NB * 32;
     // the shared-memory limit is a per-device attribute: set it for the current device
     cudaError_t e = cudaFuncSetAttribute(convKernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(tilesPerSample(a.D, a.H, a.W), a.cout / NB, a.B);
-    convKernel<NB><<<grid, kThreads, smem, s>>>(a);
+    convKernel<NB><<<grid, kCvThreads, smem, s>>>(a);
     return cudaGetLastError();
 }
 
