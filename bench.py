@@ -544,8 +544,8 @@ def run_models(args):
                                  else "fp32 sweeps, fp64 source init"), "factored_radius": RADIUS, "tolerance_s": TOL,
                    "max_iterations": N_SWEEPS_MAX, "l2": "flushed (write of 2x L2) between timed steps",
                    "parallelism": f"replicas x{world} (models split by estimated cost, no collective)"},
-        "roofline": {"bound": "hbm", "kernel": ("sweep3ChunkNear64Kernel<float,uniform,batch>" if NEAR64[0] else
-                                                "sweep3ChunkKernel<float,uniform,batch>"), "achieved": achieved,
+        "roofline": {"bound": "hbm", "kernel": ("sweep3WaveKernel<float,near64,batch>" if NEAR64[0] else
+                                                "sweep3WaveKernel<float,batch>"), "achieved": achieved,
                      "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                      "algorithmic_bytes": rl["algorithmic_bytes"], "node_updates": rl["node_updates"],
                      "refine_ms": rl["refine_ms"], "launch_ms": rl["launch_ms"], "traffic": None,
@@ -633,7 +633,7 @@ def run_2d(args):
                                f"{fields} field(s) per step", "factored_radius": 3, "n_sweeps": 2, "tolerance_s": 1e-8,
                    "l2": "flushed (write of 2x L2) between timed steps"},
         "roofline": {"bound": "hbm", "kernel": ("sweep2BlockKernel<double,uniform>" if KERNEL[0] == 2 and nz <= 512
-                                                else "sweep2Kernel<double,uniform>"),
+                                                else "sweep2WaveKernel<double,uniform>"),
                      "achieved": rl["achieved"], "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": rl["achieved"] / peak, "algorithmic_bytes": rl["algorithmic_bytes"],
                      "node_updates": rl["node_updates"], "refine_ms": rl["refine_ms"], "launch_ms": rl["launch_ms"],
@@ -1074,9 +1074,9 @@ def main():
     ap.add_argument("--skip-cpu", action="store_true")
     ap.add_argument("--skip-accuracy", action="store_true")
     ap.add_argument("--sweep-kernel", type=int, default=0, choices=[0, 1, 2],
-                    help="3D sweep kernel: 0 default (chunk-step), 1 node-step, 2 chunk-step")
+                    help="3D sweep kernel: 0 default (wave-step), 1 node-step, 2 chunk-step")
     ap.add_argument("--no-autotune", action="store_true",
-                    help="skip eikx_autotune3d before timing (default chunk-step 8x4 configuration)")
+                    help="skip eikx_autotune3d before timing (the default kernel, full occupancy)")
     ap.add_argument("--fp32-near", action="store_true",
                     help="3D: factored (near-source) updates in FP32 too, instead of FP64")
     ap.add_argument("--pair-fields", action="store_true",

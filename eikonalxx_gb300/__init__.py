@@ -221,7 +221,7 @@ class Options:
     test_drop_blocks: int = 0   # test hook only (see eikx_options.test_drop_blocks)
     profile_sweeps: bool = False  # time each sweep kernel with CUDA events (no graph)
     pair_fields: bool = False     # two fields per GPU lane for FP32 uniform batches
-    sweep_kernel: int = 0         # 3D: 0 = tuned or chunk-step, 1 = node-step, 2 = chunk-step
+    sweep_kernel: int = 0         # 3D: 0 = tuned or wave-step, 1 = node-step, 2 = chunk-step
     block_shape: int = 0          # 3D chunk-step warp block: 0 = tuned or 8x4, 1 = 8x4, 2 = 4x8, 3 = 16x2
     blocks_per_sm: int = 0        # persistent grid: 0 = as many as fit (or tuned)
     test_tag_margin: int = 0      # test hook only (see eikx_options.test_tag_margin)

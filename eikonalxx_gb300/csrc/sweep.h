@@ -71,10 +71,10 @@ template <class T> struct Sweep3Args {
     T h;                      // uniform spacing
     Spacing3<T> sp3;          // non-uniform constants
     const int2 *pairs;        // field pairs of the paired kernel (work items index pairs)
-    const Grid3Unit<T> *units;  // multi-model batch: per-unit geometry (chunk-step kernel only)
-    const SourceFp64 *srcs64; // per field, FP32 chunk-step only: set = the FP64 factored branch
+    const Grid3Unit<T> *units;  // multi-model batch: per-unit geometry (wave-step and chunk-step kernels)
+    const SourceFp64 *srcs64; // per field, FP32 wave-step and chunk-step: set = the FP64 factored branch
                               // (eikx_options.near_fp64), its own kernel instances
-    // A stream of sources through slots (chunk-step, one model; eikx_options.max_in_flight):
+    // A stream of sources through slots (wave-step or chunk-step, one model; eikx_options.max_in_flight):
     // set = field f is a slot whose current source started at sweep slots[f].x of the stream
     // (-1 = idle) in field buffer slots[f].y; sweepIndex is this sweep's position in the
     // stream and `sweep` its ordering (sweepIndex mod 8).
@@ -83,7 +83,8 @@ template <class T> struct Sweep3Args {
     int passMode;             // PassMode (wave-step kernel); sweep, sweepIndex, residualSlot are the
                               // launch's first sweep's
     int nFields;              // fields (read unless passMode is kOneSweep)
-    // Uniform grids, one model: wave-step kernel and FP64 chunk-step kernel (required there): the padded slowness copies multiplied by h (launchPadSlowness3 with h), laid out
+    // Uniform grids, one model: wave-step kernel and FP64 chunk-step kernel (required there): the
+    // padded slowness copies multiplied by h (launchPadSlowness3 with h), laid out
     // as spPos / spNeg; for the latter's factored branch also the model's natural-order cell
     // slowness (FP64 cells, or FP32 cells with cells64 = 0)
     const T *hsPos, *hsNeg;

@@ -326,7 +326,8 @@ enum { EIKX_CELL_SLOWNESS = 0, EIKX_NODAL_VELOCITY = 1 };
  * schedule.  Every (model, source) field of the batch is a work unit of the same
  * persistent sweep launches, whatever the grid sizes; models with uniform spacing and
  * models with non-uniform spacing run as two schedules.  Fields are identical to
- * eikx_solve3d on each model alone.  Uses the chunk-step sweep kernel; the context's own
+ * eikx_solve3d on each model alone.  Uses the wave-step sweep kernel, or chunk-step where
+ * sweep_kernel or block_shape ask for it; the context's own
  * model (eikx_set_slowness3d) is not touched.  eikx_get_stats reports the batch. */
 eikx_status eikx_solve3d_batch(eikx_ctx *ctx, const eikx_model3d *models, int n_models,
                                const eikx_options *opt, int precision);
