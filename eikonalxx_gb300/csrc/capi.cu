@@ -106,20 +106,21 @@ cudaError_t checkAfterSweep(const eikx::SolveState &st, int nFields, int nSweepK
 // is done with, so a pair costs one way through the blocks, not two: 256 x 256 x 128 nodes, us a
 // refinement sweep, one by one and both: 1 field (0.4 blocks a warp) 390, 274; 4 fields 526, 388;
 // 8 fields (3.4) 618, 540; 16 fields (6.7) 899, 882; 32 fields (13.5) 1546, 1578; 64 fields 2899,
-// 2985.  In double, 200 x 200 x 100: 4 fields (2.1) 2293, 1515; 32 fields (16) 5796, 5462.  With
+// 2985.  In double, 200 x 200 x 100: 4 fields (2.1) 2293, 1515; 32 fields (16) 5796, 5462.  2D in
+// double, 501 x 251: 1 field 807, 699; 64 fields (0.2) 1089, 761; 512 fields (1.7) 2145, 2061.  With
 // many blocks a warp the way through them no longer counts, and the loop over the passes costs
 // 3 %.  The mailbox doubles, so the line also bounds that.
 bool bothSweeps(bool wave, size_t items, size_t warps) { return wave && items <= 10 * warps; }
-// The eight sweeps of a pass (initialisation, or a refinement iteration) as launches of pairs:
+// The `kinds` sweeps of a pass (initialisation, or a refinement iteration) as launches of pairs:
 // sweep(ordering, init, slot, mode) and check(refinement sweep, second).
 template <class Sweep, class Check>
-eikx_status sweepPairs(int pass, bool init, Sweep sweep, Check check) {
-    const int slot = 8 * pass, r0 = slot - 8;
-    for (int e = 0; e < 8; e += 2) {
+eikx_status sweepPairs(int kinds, int pass, bool init, Sweep sweep, Check check) {
+    const int slot = kinds * pass, r0 = slot - kinds;
+    for (int e = 0; e < kinds; e += 2) {
         if (eikx_status r = sweep(e, init ? 1 : 0, slot + e, eikx::kBothSweeps); r != EIKX_OK) return r;
         if (init) continue;
         if (eikx_status r = check(r0 + e, false); r != EIKX_OK) return r;
-        if (r0 + e < 8) continue;   // no field holds a sweep back before the ninth
+        if (r0 + e < kinds) continue;   // no field holds a sweep back before the second iteration
         if (eikx_status r = sweep(e + 1, 0, slot + e + 1, eikx::kSecondSweep); r != EIKX_OK) return r;
         if (eikx_status r = check(r0 + e, true); r != EIKX_OK) return r;
     }
@@ -907,7 +908,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
     int blocks = std::min(c->numSMs * perSM, (nProgress + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock);
     blocks = std::max(blocks, 1);
-    const bool both = bothSweeps(wave, nProgress, static_cast<size_t>(c->numSMs) * perSM * eikx::kWarpsPerBlock);
+    const bool both = bothSweeps(DIM == 2 ? !block2 : wave, nProgress, static_cast<size_t>(c->numSMs) * perSM * eikx::kWarpsPerBlock);
     const size_t ttBytes = static_cast<size_t>(fieldStride) * nSrc * sizeof(T);
     const size_t mboxBytes = static_cast<size_t>(nProgress) * tl.faceWords * 8 * (both ? 2 : 1);
     const void *before[] = {w.tt.p, w.mbox.p, w.epoch.p, w.residual.p, w.converged.p,
@@ -1129,8 +1130,10 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                 a.spPos = spad[0].as<T>(); a.spNeg = spad[1].as<T>(); a.spPitch = spPitch;
                 a.nx = nx; a.nz = nz; a.tilesZ = tilesZ;
                 a.srcs = w.srcs.as<eikx::SourceT<T>>(); a.st = st; a.buf = buf; a.residualSlot = slot;
-                a.sweepIndex = sweepsLaunched;
+                a.sweepIndex = mode == eikx::kSecondSweep ? sweepsLaunched - 1 : sweepsLaunched;
                 a.sweep = e; a.init = init; a.radius = o.factored_radius; a.h = static_cast<T>(dx);
+                a.passMode = mode;
+                a.nFields = nSrc;
                 eikx::Spacing2<T> g;
                 g.dx = static_cast<T>(dx); g.dz = static_cast<T>(dz);
                 g.dx_dz = static_cast<T>(dx / dz); g.dz_dx = static_cast<T>(dz / dx);
@@ -1153,17 +1156,17 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
             return EIKX_OK;
         };
         auto check = [&](int r, bool second) -> eikx_status {
-            EIKX_CUDA(eikx::launchCheckPair(st, nSrc, r, second, o.tolerance, c->stream));
+            EIKX_CUDA(eikx::launchCheckPair(st, nSrc, nSweepKinds, r, second, o.tolerance, c->stream));
             ++launches;
             return EIKX_OK;
         };
         if (o.init_sweeps && both)
-            if (eikx_status r = sweepPairs(0, true, sweep, check); r != EIKX_OK) return r;
+            if (eikx_status r = sweepPairs(nSweepKinds, 0, true, sweep, check); r != EIKX_OK) return r;
         for (int e = 0; e < nSweepKinds && o.init_sweeps && !both; ++e)
             if (eikx_status r = sweep(e, 1, e, eikx::kOneSweep); r != EIKX_OK) return r;
         for (int k = 0; k < nSweeps; ++k) {
             if (both)
-                if (eikx_status r = sweepPairs(1 + k, false, sweep, check); r != EIKX_OK) return r;
+                if (eikx_status r = sweepPairs(nSweepKinds, 1 + k, false, sweep, check); r != EIKX_OK) return r;
             for (int e = 0; e < nSweepKinds && !both; ++e) {
                 if (eikx_status r = sweep(e, 0, nSweepKinds * (1 + k) + e, eikx::kOneSweep); r != EIKX_OK) return r;
                 EIKX_CUDA(checkAfterSweep(st, nSrc, nSweepKinds, nSweepKinds * k + e, o.tolerance, c->stream));
@@ -1690,17 +1693,17 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
             return EIKX_OK;
         };
         auto check = [&](int r, bool second) -> eikx_status {
-            EIKX_CUDA(eikx::launchCheckPair(st, nUnits, r, second, o.tolerance, c->stream));
+            EIKX_CUDA(eikx::launchCheckPair(st, nUnits, nSweepKinds, r, second, o.tolerance, c->stream));
             ++launches;
             return EIKX_OK;
         };
         if (o.init_sweeps && both)
-            if (eikx_status r = sweepPairs(0, true, sweep, check); r != EIKX_OK) return r;
+            if (eikx_status r = sweepPairs(nSweepKinds, 0, true, sweep, check); r != EIKX_OK) return r;
         for (int e = 0; e < nSweepKinds && o.init_sweeps && !both; ++e)
             if (eikx_status r = sweep(e, 1, e, eikx::kOneSweep); r != EIKX_OK) return r;
         for (int k = 0; k < nSweeps; ++k) {
             if (both)
-                if (eikx_status r = sweepPairs(1 + k, false, sweep, check); r != EIKX_OK) return r;
+                if (eikx_status r = sweepPairs(nSweepKinds, 1 + k, false, sweep, check); r != EIKX_OK) return r;
             for (int e = 0; e < nSweepKinds && !both; ++e) {
                 if (eikx_status r = sweep(e, 0, nSweepKinds * (1 + k) + e, eikx::kOneSweep); r != EIKX_OK) return r;
                 EIKX_CUDA(checkAfterSweep(st, nUnits, nSweepKinds, nSweepKinds * k + e, o.tolerance, c->stream));

@@ -374,16 +374,16 @@ __global__ void checkKernel(SolveState st, int nFields, int firstSlot, int nSlot
     }
 }
 
-// The same test where a launch ran refinement sweeps r and r + 1 (slots 8 + r, 9 + r), or r alone
+// The same test where a launch ran refinement sweeps r and r + 1 (slots kinds + r and on), or r alone
 // on the fields that held r + 1 back, and where it then ran r + 1 on those it left open (`second`).
-// A field holds the odd sweep back when it could end with the even one: when the seven sweeps
+// A field holds the odd sweep back when it could end with the even one: when the kinds - 1 sweeps
 // before that are below tol.
-__global__ void checkPairKernel(SolveState st, int nFields, int r, int second, double tol) {
+__global__ void checkPairKernel(SolveState st, int nFields, int kinds, int r, int second, double tol) {
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nFields; f += gridDim.x * blockDim.x) {
         if (st.converged[f]) continue;
         const int state = st.pairState[f];
         if (second && state != kPairOpen) continue;
-        const unsigned long long *res = st.residual + static_cast<long long>(f) * st.residualStride + 8;
+        const unsigned long long *res = st.residual + static_cast<long long>(f) * st.residualStride + kinds;
         auto largest = [&](int first, int last) {
             double m = 0;
             for (int k = max(first, 0); k <= last; ++k) m = fmax(m, __longlong_as_double(static_cast<long long>(res[k])));
@@ -392,9 +392,9 @@ __global__ void checkPairKernel(SolveState st, int nFields, int r, int second, d
         const bool held = !second && state == kPairHeld;
         const int done = held ? r : r + 1;   // the last refinement sweep run
         st.sweepsRun[f] = done + 1;
-        if (done >= 7 && largest(done - 7, done) < tol) st.converged[f] = 1;
+        if (done >= kinds - 1 && largest(done - kinds + 1, done) < tol) st.converged[f] = 1;
         else if (held) st.pairState[f] = kPairOpen;
-        else st.pairState[f] = r + 2 >= 7 && largest(r - 5, r + 1) < tol ? kPairHeld : kPairRun;
+        else st.pairState[f] = r + 2 >= kinds - 1 && largest(r + 3 - kinds, r + 1) < tol ? kPairHeld : kPairRun;
     }
 }
 
@@ -624,8 +624,8 @@ cudaError_t launchCheckConvergence(const SolveState &st, int nFields, int firstS
     checkKernel<<<gridFor(nFields, 128), 128, 0, s>>>(st, nFields, firstSlot, nSlots, sweepsDone, tol);
     return cudaGetLastError();
 }
-cudaError_t launchCheckPair(const SolveState &st, int nFields, int r, bool second, double tol, cudaStream_t s) {
-    checkPairKernel<<<gridFor(nFields, 128), 128, 0, s>>>(st, nFields, r, second ? 1 : 0, tol);
+cudaError_t launchCheckPair(const SolveState &st, int nFields, int kinds, int r, bool second, double tol, cudaStream_t s) {
+    checkPairKernel<<<gridFor(nFields, 128), 128, 0, s>>>(st, nFields, kinds, r, second ? 1 : 0, tol);
     return cudaGetLastError();
 }
 cudaError_t launchCheckStream(const SolveState &st, const int2 *slots, int nSlots, int sweepIndex, int initSweeps,

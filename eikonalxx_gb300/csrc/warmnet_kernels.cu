@@ -536,20 +536,14 @@ __device__ __forceinline__ NodeGeom nodeGeom(const float *table, const Geometry 
 // Straight-ray estimate of tau - 1 at node (x, y, z): the mean of s/s_src - 1 over
 // kRaySamples midpoints of the segment from the source to the node, the slowness
 // trilinear in the nodal 1/v.  FP32, in an operation order the oracle repeats.  What bounds it is
-// issue slots: two midpoints share packed FP32 additions, floor is an addition
+// issue slots (72 % taken): two midpoints are in flight together, floor is an addition
 // rounded down (px + 2^23, whose low bits are the index; the conversions run at a quarter of the
 // rate), and the clamps to the grid are left out where the source lies inside (INSIDE: then so do
 // the rounded points of the segment: with w = RN(t e), |w| <= (63/64) |e| (1 + 2^-23) leaves s + w
 // between s and x, and rounding keeps that).
 constexpr int kRaySamples = 32;
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 r;
-    asm("{.reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-// (Scalar: the assembler fuses a packed product into a packed sum, .rn or not.)
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return add2(a, make_float2(-b.x, -b.y)); }
 __device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 f) { return add2(a, mul2(f, sub2(b, a))); }
 template <bool INSIDE>

@@ -91,3 +91,28 @@ def test_both_orderings_in_one_launch_match_one_by_one(ctx, oracle, spacing, pre
         cell = [min(n - 2, int(q / h)) for q, n, h in zip(pos[i], grid, spacing)]
         ref = oracle.solve3d(s, (nx, ny, nz, *spacing), cell, pos[i], n_sweeps=6, radius=3, tol=tol, init_sweeps=init)
         assert np.array_equal(_bits(out[0][0][i]), _bits(ref))
+
+
+# 2100 fields of 3 warp blocks, likewise
+@pytest.mark.parametrize("precision", [ex.F32, ex.F64])
+@pytest.mark.parametrize("spacing", [(10.0, 10.0), (10.0, 12.5)])
+@pytest.mark.parametrize("init,tol", [(True, 1e-3), (True, 1e-5), (True, 1e-7), (False, 1e-5)])
+def test_both_orderings_in_one_launch_match_one_by_one_2d(ctx, oracle, spacing, precision, init, tol):
+    grid = nx, nz = 23, 66
+    rng = np.random.default_rng(12)
+    dt = np.float32 if precision == ex.F32 else np.float64
+    s = random_slowness(rng, (nz - 1) * (nx - 1), dtype=dt)
+    ctx.set_grid2d(nx, nz, *spacing)
+    ctx.set_slowness2d(s)
+    pos = rng.uniform(0, 1, (2100, 2)) * (np.array(grid) - 1) * spacing
+    out = []
+    for per_sm in (0, 1):
+        t = ctx.solve2d(pos, ex.Options(n_sweeps=6, tolerance=tol, init_sweeps=init, blocks_per_sm=per_sm), precision)
+        st = ctx.stats()
+        out.append((t, [st[k] for k in ("iterations_max", "iterations_min", "sweeps_launched", "refine_node_updates")]))
+    assert out[0][1] == out[1][1]
+    assert np.array_equal(_bits(np.asarray(out[0][0])), _bits(np.asarray(out[1][0])))
+    for i in (0, 1033, 2099):
+        cell = [min(n - 2, int(q / h)) for q, n, h in zip(pos[i], grid, spacing)]
+        ref = oracle.solve2d(s, (nx, nz, *spacing), cell, pos[i], n_sweeps=6, radius=3, tol=tol, init_sweeps=init)
+        assert np.array_equal(_bits(out[0][0][i]), _bits(ref))
