@@ -104,8 +104,8 @@ cudaError_t checkAfterSweep(const eikx::SolveState &st, int nFields, int nSweepK
 // Whether a solve takes both orderings of a pair in one wave-step launch, for `items` warp blocks
 // (of all fields) on `warps` resident warps.  The second ordering starts in blocks that the first
 // is done with, so a pair costs one way through the blocks, not two: 256 x 256 x 128 nodes, us a
-// refinement sweep, one by one and both: 1 field (0.4 blocks a warp) 390, 274; 4 fields 526, 388;
-// 8 fields (3.4) 618, 540; 16 fields (6.7) 899, 882; 32 fields (13.5) 1546, 1578; 64 fields 2899,
+// refinement sweep, one by one and both: 1 field (0.4 blocks a warp) 390, 257; 4 fields 526, 364;
+// 8 fields (3.4) 618, 516; 16 fields (6.7) 899, 868; 32 fields (13.5) 1546, 1578; 64 fields 2899,
 // 2985.  In double, 200 x 200 x 100: 4 fields (2.1) 2293, 1515; 32 fields (16) 5796, 5462.  2D in
 // double, 501 x 251: 1 field 807, 699; 64 fields (0.2) 1089, 761; 512 fields (1.7) 2145, 2061.  With
 // many blocks a warp the way through them no longer counts, and the loop over the passes costs
@@ -855,8 +855,8 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     const bool paired = DIM == 3 && P == EIKX_F32 && uniform && nSrc >= 2 && o.pair_fields;
     // The default is the wave-step kernel on every grid; a warp-block shape asks for chunk-step.
     // Measured, us a refinement sweep, chunk-step and wave-step: 256 x 256 x 128 FP32, 1 field 915,
-    // 275; 16 fields 1383, 885; 64 fields 3301, 2900; 64 x 64 x 32, 1 field 264, 79; 200 x 200 x 100 in
-    // double, 4 fields 4691, 1524; flat cells (non-uniform), 151 x 131 x 87, 8 fields 811, 295.
+    // 257; 16 fields 1383, 866; 64 fields 3301, 2892; 64 x 64 x 32, 1 field 264, 76; 200 x 200 x 100 in
+    // double, 4 fields 4691, 1519; flat cells (non-uniform), 151 x 131 x 87, 8 fields 811, 288.
     const bool wave = DIM == 3 && !paired &&
                         (o.sweep_kernel == eikx::kWaveStep || (o.sweep_kernel == 0 && o.block_shape == 0));
     const int variant = wave ? eikx::kWaveStep : o.sweep_kernel == eikx::kNodeStep ? eikx::kNodeStep : eikx::kChunkStep;
