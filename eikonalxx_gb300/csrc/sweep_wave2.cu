@@ -17,8 +17,8 @@
 // What bounds a field is that chain (issue slots 14 % taken, DRAM idle); many fields share its latency
 // until the FP64 pipe is full.  Measured, a solve of 4 + 8 sweeps of 501 x 251 nodes in double, ms, the
 // kernel before (32-row blocks, the whole operator in FP64) and this one: 1 field 26.3, 7.8 (8.8 with
-// one ordering per launch); 64 fields 32.2, 9.2 (13.5).  With non-uniform spacing only the exit test
-// is FP32: 2673 to 2034 us a refinement sweep.
+// one ordering per launch); 64 fields 32.2, 9.2 (13.5).  With non-uniform spacing 2673 to 1244 us a
+// refinement sweep (2034 with the exit test alone in FP32).
 #include <algorithm>
 #include "sweep.h"
 #include "wave.cuh"
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kThreads2) sweep2WaveKernel(const Sweep2Args<T
     const T huge = static_cast<T>(1.e10);
     const int Px = a.pitch, nx = a.nx, nz = a.nz, nChunks = Px / kG;
     const long long fieldWords = static_cast<long long>(a.tilesZ) * waveStepCap2(Px) * W;
-    const float hF = view(a.h);
+    const float hF = view(a.h), dxF = view(a.sp2.dx), dzF = view(a.sp2.dz), dMinF = fminf(dxF, dzF);
     bool ok = true;
 
     while (ok) {
@@ -238,12 +238,13 @@ __global__ void __launch_bounds__(kThreads2) sweep2WaveKernel(const Sweep2Args<T
                     float low;
                     // A 1D operator or one of a cell edge is >= t1 or >= t3; the diagonal one, its window
                     // open, is >= t2 + h s0 less the rounding (the 3D planes' bound, sweep_wave.cu), and on a
-                    // non-uniform grid >= t2 less a rounding error below 64 u max(t1, t2, t3): with d = t1 - t3
-                    // between -dx s0 and dz s0, the exact operator is concave in d and dx s0, dz s0 above t2 at
-                    // the ends, and each of its terms is at most 3 max(t1, t2, t3).
+                    // non-uniform grid >= t2 + min(dx s0, dz s0) less a rounding error below 64 u
+                    // max(t1, t2, t3): with d = t1 - t3 between -dx s0 and dz s0, the exact operator is concave
+                    // in d and dx s0, dz s0 above t2 at the ends, and each of its terms is at most
+                    // 3 max(t1, t2, t3) there.
                     if (UNIFORM && SCALED) low = vnP + __fmaf_rn(view(snP), kC20, -E);
                     else if (UNIFORM) low = vnP - E;
-                    else low = vnP - fmaxf(mx, vnP) * 1.52587890625e-5f;   // 2^-16
+                    else low = vnP + __fmaf_rn(dMinF * view(snP), kC20, -fmaxf(mx, vnP) * 1.52587890625e-5f);   // 2^-16
                     bool need = upd & !(v0 <= fminf(fminf(vo, vN), low));
                     T v = t0;
                     if (tileNear) {
@@ -297,6 +298,52 @@ __global__ void __launch_bounds__(kThreads2) sweep2WaveKernel(const Sweep2Args<T
                             const bool again = need & (edge(vo, !above(nP, o1)) | edge(vN, !above(nP, N)));
                             if (__any_sync(kFull, again)) {
                                 if (again) best = dmin(best, node2<T, UNIFORM, false>(a.h, a.sp2, src, sg, xa, za, o1, nP, N, a.spNeg, a.spPitch));
+                            }
+                            if (need) v = best;
+                        } else if constexpr (!UNIFORM && sizeof(T) == 8) {
+                            // fd2NonUniformFar, each operator only where FP32 cannot rule it out
+                            const Spacing2<T> &g2 = a.sp2;
+                            T best = t0;
+                            const float f0 = view(snP), big = fmaxf(mx, vnP) * (1.0f / 1048576.0f);
+                            constexpr float kUp = 1.0f + 1.0f / 65536.0f;
+                            const bool outX = !above(nP, o1), outZ = !above(nP, N);   // t1 >= t2, t3 >= t2
+                            bool c3 = need & outX & outZ & (low <= v0) & (vo - vN <= f0 * dzF * kUp + big) & (vN - vo <= f0 * dxF * kUp + big);
+                            if (__any_sync(kFull, c3)) {
+                                const T hx = g2.dx * snP, hz = g2.dz * snP, d = o1 - N, det = hx * hx + hz * hz - d * d;
+                                c3 = c3 & above(det, T(0)) & above(N + hz, o1) & above(o1 + hx, N);
+                                const T tx = o1 - N + nP, tz = N - o1 + nP, dxdz = g2.cosTheta * g2.sinTheta;
+                                const T u = dxdz * (tx * g2.dz_dx + tz * g2.dx_dz + 2 * dsqrt(c3 ? det : T(1)));
+                                if (c3 && !(u < 0) && u < best) best = u;
+                            }
+                            const bool gx = need & (vo + __fmaf_rn(dxF * fminf(f0, view(soP)), kC20, -E) <= Bounds<T>::upper(view(best)));
+                            if (__any_sync(kFull, gx)) {
+                                const T u = o1 + g2.dx * pmin(snP, soP);
+                                if (gx & above(best, u)) best = u;
+                            }
+                            const bool gz = need & (vN + __fmaf_rn(dzF * fminf(f0, view(sN)), kC20, -E) <= Bounds<T>::upper(view(best)));
+                            if (__any_sync(kFull, gz)) {
+                                const T u = N + g2.dz * pmin(snP, sN);
+                                if (gz & above(best, u)) best = u;
+                            }
+                            // t1 + dx / dz sqrt((dz s0)^2 - (t1 - t2)^2) where 0 <= t1 - t2 <= dz sin s0; t3 likewise
+                            auto edge = [&](float va, float dF, float ratio, float sine) {
+                                const float hi = fmaxf(va - vnP, 0.f) + big, lo = va - vnP - big, h = dF * f0;
+                                const float w = __fmaf_rn(h * (1.0f - 1.0f / 131072.0f), h, -(hi * hi));
+                                float root;
+                                asm("sqrt.approx.f32 %0, %1;" : "=f"(root) : "f"(fmaxf(w, 0.f)));
+                                return (lo <= h * sine * kUp) & (va + ratio * root * (1.0f - 1.0f / 1024.0f) - E <= Bounds<T>::upper(view(best)));
+                            };
+                            const bool ea = need & outX & edge(vo, dzF, view(g2.dx_dz), view(g2.sinTheta));
+                            if (__any_sync(kFull, ea)) {
+                                const T hz = g2.dz * snP, d = o1 - nP, det = hz * hz - d * d;
+                                const T u = o1 + g2.dx_dz * dsqrt(ea && det >= 0 ? det : T(1));
+                                if (ea && det >= 0 && d <= g2.dz * (g2.sinTheta * snP) && u < best) best = u;
+                            }
+                            const bool eb = need & outZ & edge(vN, dxF, view(g2.dz_dx), view(g2.cosTheta));
+                            if (__any_sync(kFull, eb)) {
+                                const T hx = g2.dx * snP, d = N - nP, det = hx * hx - d * d;
+                                const T u = N + g2.dz_dx * dsqrt(eb && det >= 0 ? det : T(1));
+                                if (eb && det >= 0 && d <= g2.dx * (g2.cosTheta * snP) && u < best) best = u;
                             }
                             if (need) v = best;
                         } else {
