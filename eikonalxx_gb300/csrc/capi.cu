@@ -925,7 +925,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     }
     EIKX_CUDA(w.queue.ensure(2 * sizeof(unsigned)));
     EIKX_CUDA(w.residual.ensure(static_cast<size_t>(nSrc) * resStride * 8));
-    EIKX_CUDA(w.converged.ensure(static_cast<size_t>(nSrc) * 8));   // and the pair states
+    EIKX_CUDA(w.converged.ensure(static_cast<size_t>(nSrc) * 12));   // and the pair states, and anyTimes
     EIKX_CUDA(w.iterations.ensure(static_cast<size_t>(nSrc) * 4));
     EIKX_CUDA(w.abortFlag.ensure(sizeof(int)));
     EIKX_CUDA(w.order.ensure(static_cast<size_t>(nProgress) * 16));
@@ -1004,6 +1004,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     st.residualStride = resStride;
     st.converged = w.converged.as<int>();
     st.pairState = w.converged.as<int>() + nSrc;
+    st.anyTimes = warm && wave ? w.converged.as<int>() + 2 * static_cast<size_t>(nSrc) : nullptr;
     st.sweepsRun = w.iterations.as<int>();
     st.abortFlag = w.abortFlag.as<int>();
     // test hook: leave the first blocks of the queue out (their dependants time out)
@@ -1073,7 +1074,7 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                                                c->slow3.as<double>(), o.factored_radius, uniform, static_cast<T>(dx),
                                                spacing3<T>(dx, dy, dz), gateTol, o.warm_gate == 1 ? 1 : 0,
                                                o.init_fp64 ? 1 : 0, srcs64,
-                                               w.resetCount.as<unsigned long long>(), c->stream));
+                                               w.resetCount.as<unsigned long long>(), st.anyTimes, c->stream));
         } else if (DIM == 3)
             EIKX_CUDA(eikx::launchInit3<T>(w.tt.as<T>(), nSrc, fieldStride, Px, nx, ny, nz, dx, dy, dz,
                                            w.corners.as<eikx::Corner3>(), o.init_fp64 ? 1 : 0, c->stream));

@@ -85,7 +85,7 @@ __global__ void warmInit3Kernel(T *tt, const T *init, int nFields, long long fie
                                 int nz, double dx, double dy, double dz, const Corner3 *corners,
                                 const SourceT<T> *srcs, const double *slow, int radius, T h, Spacing3<T> g,
                                 double gateTol, int twoSided, int fp64, const SourceFp64 *srcs64,
-                                unsigned long long *nReset) {
+                                unsigned long long *nReset, int *anyTimes) {
     const long long perField = static_cast<long long>(nx) * ny * nz;
     const long long n = perField * nFields;
     const int ncx = nx - 1, ncy = ny - 1, ncz = nz - 1;
@@ -155,6 +155,7 @@ __global__ void warmInit3Kernel(T *tt, const T *init, int nFields, long long fie
             }
             if (under) ++resets;
         }
+        if (anyTimes && !(v >= 0 && v <= static_cast<T>(kTimeMax))) anyTimes[f] = 1;
         tt[static_cast<long long>(f) * fieldStride + (static_cast<long long>(iz) * ny + iy) * pitch + ix] = v;
     }
     if (resets) atomicAdd(nReset, resets);
@@ -350,6 +351,7 @@ __global__ void resetKernel(SolveState st, int nFields, int buf) {
         st.converged[i] = 0;
         st.sweepsRun[i] = 0;
         if (st.pairState) st.pairState[i] = kPairRun;
+        if (st.anyTimes) st.anyTimes[i] = 0;
     }
     if (gtid == 0) {
         *st.queue[buf] = 0u;
@@ -580,16 +582,16 @@ cudaError_t launchWarmInit3(T *tt, const T *init, int nFields, long long fieldSt
                             double dx, double dy, double dz, const Corner3 *corners, const SourceT<T> *srcs,
                             const double *slow, int radius, bool uniform, T h, const Spacing3<T> &g, double gateTol,
                             int twoSided, int fp64, const SourceFp64 *srcs64, unsigned long long *nReset,
-                            cudaStream_t s) {
+                            int *anyTimes, cudaStream_t s) {
     const long long n = static_cast<long long>(nx) * ny * nz * nFields;
     if (uniform)
         warmInit3Kernel<T, true><<<gridFor(n), kThreads, 0, s>>>(tt, init, nFields, fieldStride, pitch, nx, ny, nz, dx,
                                                                  dy, dz, corners, srcs, slow, radius, h, g, gateTol,
-                                                                 twoSided, fp64, srcs64, nReset);
+                                                                 twoSided, fp64, srcs64, nReset, anyTimes);
     else
         warmInit3Kernel<T, false><<<gridFor(n), kThreads, 0, s>>>(tt, init, nFields, fieldStride, pitch, nx, ny, nz, dx,
                                                                   dy, dz, corners, srcs, slow, radius, h, g, gateTol,
-                                                                  twoSided, fp64, srcs64, nReset);
+                                                                  twoSided, fp64, srcs64, nReset, anyTimes);
     if (pitch > nx) {
         const long long np = static_cast<long long>(nFields) * ny * nz * (pitch - nx);
         fillPadKernel<T><<<gridFor(np), kThreads, 0, s>>>(tt, nFields, fieldStride, pitch, nx, ny * nz);
@@ -599,11 +601,11 @@ cudaError_t launchWarmInit3(T *tt, const T *init, int nFields, long long fieldSt
 template cudaError_t launchWarmInit3<float>(float *, const float *, int, long long, int, int, int, int, double, double,
                                             double, const Corner3 *, const SourceT<float> *, const double *, int, bool,
                                             float, const Spacing3<float> &, double, int, int, const SourceFp64 *,
-                                            unsigned long long *, cudaStream_t);
+                                            unsigned long long *, int *, cudaStream_t);
 template cudaError_t launchWarmInit3<double>(double *, const double *, int, long long, int, int, int, int, double,
                                              double, double, const Corner3 *, const SourceT<double> *, const double *,
                                              int, bool, double, const Spacing3<double> &, double, int, int,
-                                             const SourceFp64 *, unsigned long long *, cudaStream_t);
+                                             const SourceFp64 *, unsigned long long *, int *, cudaStream_t);
 
 cudaError_t launchFactorTables(const SourceFp64 *srcs, int nFields, cudaStream_t s) {
     factorTableKernel<<<nFields, 256, 0, s>>>(srcs);

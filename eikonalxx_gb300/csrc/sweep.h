@@ -23,12 +23,18 @@ struct SolveState {
     int *converged;                 // 1 once a field's iteration decrease fell below tol
     int *pairState;                 // wave-step kernel, two orderings per launch: PairState per field
                                     // (null otherwise)
+    int *anyTimes;                  // wave-step kernel, warm starts: 1 = the field's start holds times
+                                    // outside [0, kTimeMax] (null otherwise)
     int *sweepsRun;                 // refinement sweeps each field ran
     int *abortFlag;                 // raised when a bounded wait ran out
     const int4 *order;              // work queue: (field, by, bz, 0) sorted by start step
     int totalItems;                 // fields * warp blocks per field
     unsigned long long spinLimit;   // polls before a wait gives up
 };
+
+// The bounds of the wave-step kernel take times to lie in [0, kTimeMax], as a solve's own always do
+// (1e10 is the largest), with room for their squares in FP32.
+constexpr float kTimeMax = 1e18f;
 
 // A wave-step launch runs one sweep, or the two orderings that differ in the direction of x' only
 // (even, odd: same blocks, same dependences between blocks): each block walks its rows forth and
@@ -229,7 +235,7 @@ cudaError_t launchWarmInit3(T *tt, const T *init, int nFields, long long fieldSt
                             double dx, double dy, double dz, const Corner3 *corners, const SourceT<T> *srcs,
                             const double *slow, int radius, bool uniform, T h, const Spacing3<T> &g, double gateTol,
                             int twoSided, int fp64, const SourceFp64 *srcs64, unsigned long long *nReset,
-                            cudaStream_t s);
+                            int *anyTimes, cudaStream_t s);
 // Fills the FP64 analytic-factor table of each field whose SourceFp64 has one.
 cudaError_t launchFactorTables(const SourceFp64 *srcs, int nFields, cudaStream_t s);
 // Box of a field's factor table: the nodes within `radius` of the source cell along every

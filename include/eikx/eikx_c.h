@@ -192,7 +192,9 @@ eikx_status eikx_solve3d(eikx_ctx *ctx, const eikx_source3d *src, int n_src,
  * below the analytic value, so a converged field is a fixed point of the warm start), or
  * takes the analytic value when the gate rejects it; then refinement iterations run to
  * the tolerance without the initialisation pass.  eikx_stats.reset_nodes counts the
- * resets.  Note: the reference's local solver is not monotone in its neighbours (the
+ * resets.  What the gate keeps need not be a time: negative, not-a-number and infinite values enter the
+ * operators as they are, and a field that starts from any takes every operator at every node (slower).
+ * Note: the reference's local solver is not monotone in its neighbours (the
  * causality windows of the 2D and 3D operators, the factored branch): raising a
  * neighbour can lower a node.  Sweeps started from any field other than the cold
  * start's own result -- even that result inflated by 0.1 % -- can settle on a different
