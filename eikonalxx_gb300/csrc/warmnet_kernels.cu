@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(kThreads) biasGradKernel(const bf16 *dy, int C
 
 // The element-wise kernels below move whole 16-byte pieces of 8 channels and are bound by memory.
 // A block takes pieces of one x-row of the tensor that it writes (grid: pieces of a row, rows of a
-// plane, planes of all samples), so that a thread needs one 32-bit division to find its place
+// plane, planes of all samples, the latter two up to what a launch takes and in steps of it), so that a thread needs one 32-bit division to find its place
 // (upsampling and concatenation at 8 x 64 x 128 x 128 nodes: 445 us with five 64-bit ones, 183 now).
 struct Piece {
     int g, x, y, z, b;   // 8-channel group, node, sample
@@ -395,18 +395,20 @@ __global__ void __launch_bounds__(kThreads) poolKernel(const bf16 *x, int C, int
     for (long long plane = blockIdx.z; plane < static_cast<long long>(B) * Dl; plane += gridDim.z) {
         Piece p;
         if (!pieceOf(p, groups, Wl, Dl, plane)) continue;
-        const bf16 *src = x + ((((static_cast<long long>(p.b) * D + 2 * p.z) * H + 2 * p.y) * W + 2 * p.x) * C + 8 * p.g);
-        float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        for (; p.y < Hl; p.y += gridDim.y) {
+            const bf16 *src = x + ((((static_cast<long long>(p.b) * D + 2 * p.z) * H + 2 * p.y) * W + 2 * p.x) * C + 8 * p.g);
+            float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            float f[8];
-            load8(f, src + ((static_cast<long long>(k >> 2) * H + ((k >> 1) & 1)) * W + (k & 1)) * C);
+            for (int k = 0; k < 8; ++k) {
+                float f[8];
+                load8(f, src + ((static_cast<long long>(k >> 2) * H + ((k >> 1) & 1)) * W + (k & 1)) * C);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s[j] += f[j];
+                for (int j = 0; j < 8; ++j) s[j] += f[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[j] *= 0.125f;
+            store8(y + ((plane * Hl + p.y) * Wl + p.x) * C + 8 * p.g, s);
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s[j] *= 0.125f;
-        store8(y + ((plane * Hl + p.y) * Wl + p.x) * C + 8 * p.g, s);
     }
 }
 
@@ -415,23 +417,26 @@ constexpr int kRowsEach = 4;
 __global__ void __launch_bounds__(kThreads) upcatKernel(const bf16 *low, int c1, const bf16 *skip, int c2, int D, int H, int W,
                                                         int B, bf16 *out) {
     const int C = c1 + c2, groups = C / 8;
+    const int rows = (H + kRowsEach - 1) / kRowsEach;
     for (long long plane = blockIdx.z; plane < static_cast<long long>(B) * D; plane += gridDim.z) {
         Piece p;
         if (!pieceOf(p, groups, W, D, plane)) continue;
-        Vec8 v[kRowsEach];
+        for (; p.y < rows; p.y += gridDim.y) {
+            Vec8 v[kRowsEach];
 #pragma unroll
-        for (int k = 0; k < kRowsEach; ++k) {
-            const int y = kRowsEach * p.y + k;
-            if (y >= H) break;
-            const bf16 *src = skip + ((plane * H + y) * W + p.x) * c2 + 8 * p.g - c1;
-            if (8 * p.g < c1)
-                src = low + (((static_cast<long long>(p.b) * (D / 2) + p.z / 2) * (H / 2) + y / 2) * (W / 2) + p.x / 2) * c1 + 8 * p.g;
-            v[k] = *reinterpret_cast<const Vec8 *>(src);
-        }
+            for (int k = 0; k < kRowsEach; ++k) {
+                const int y = kRowsEach * p.y + k;
+                if (y >= H) break;
+                const bf16 *src = skip + ((plane * H + y) * W + p.x) * c2 + 8 * p.g - c1;
+                if (8 * p.g < c1)
+                    src = low + (((static_cast<long long>(p.b) * (D / 2) + p.z / 2) * (H / 2) + y / 2) * (W / 2) + p.x / 2) * c1 + 8 * p.g;
+                v[k] = *reinterpret_cast<const Vec8 *>(src);
+            }
 #pragma unroll
-        for (int k = 0; k < kRowsEach; ++k) {
-            const int y = kRowsEach * p.y + k;
-            if (y < H) *reinterpret_cast<Vec8 *>(out + ((plane * H + y) * W + p.x) * C + 8 * p.g) = v[k];
+            for (int k = 0; k < kRowsEach; ++k) {
+                const int y = kRowsEach * p.y + k;
+                if (y < H) *reinterpret_cast<Vec8 *>(out + ((plane * H + y) * W + p.x) * C + 8 * p.g) = v[k];
+            }
         }
     }
 }
@@ -442,53 +447,58 @@ __global__ void __launch_bounds__(kThreads) upSumMaskKernel(const bf16 *dcat, in
     for (long long plane = blockIdx.z; plane < static_cast<long long>(B) * Dl; plane += gridDim.z) {
         Piece p;
         if (!pieceOf(p, groups, Wl, Dl, plane)) continue;
-        const bf16 *src = dcat + ((((static_cast<long long>(p.b) * D + 2 * p.z) * H + 2 * p.y) * W + 2 * p.x) * ccat + 8 * p.g);
-        const long long u = (plane * Hl + p.y) * Wl + p.x;
-        float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        for (; p.y < Hl; p.y += gridDim.y) {
+            const bf16 *src = dcat + ((((static_cast<long long>(p.b) * D + 2 * p.z) * H + 2 * p.y) * W + 2 * p.x) * ccat + 8 * p.g);
+            const long long u = (plane * Hl + p.y) * Wl + p.x;
+            float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            float f[8];
-            load8(f, src + ((static_cast<long long>(k >> 2) * H + ((k >> 1) & 1)) * W + (k & 1)) * ccat);
+            for (int k = 0; k < 8; ++k) {
+                float f[8];
+                load8(f, src + ((static_cast<long long>(k >> 2) * H + ((k >> 1) & 1)) * W + (k & 1)) * ccat);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s[j] += f[j];
+                for (int j = 0; j < 8; ++j) s[j] += f[j];
+            }
+            float m[8];
+            load8(m, act + u * c1 + 8 * p.g);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (!(m[j] > 0.f)) s[j] = 0.f;
+            store8(dpre + u * c1 + 8 * p.g, s);
         }
-        float m[8];
-        load8(m, act + u * c1 + 8 * p.g);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (!(m[j] > 0.f)) s[j] = 0.f;
-        store8(dpre + u * c1 + 8 * p.g, s);
     }
 }
 
 __global__ void __launch_bounds__(kThreads) combineSkipKernel(const bf16 *dcat, int ccat, int c1, const bf16 *dpool,
                                                               const bf16 *skip, int c2, int D, int H, int W, int B, bf16 *dpre) {
     const int groups = c2 / 8;
+    const int rows = (H + kRowsEach - 1) / kRowsEach;
     for (long long plane = blockIdx.z; plane < static_cast<long long>(B) * D; plane += gridDim.z) {
         Piece q;
         if (!pieceOf(q, groups, W, D, plane)) continue;
-        Vec8 a[kRowsEach], p[kRowsEach], m[kRowsEach];
+        for (; q.y < rows; q.y += gridDim.y) {
+            Vec8 a[kRowsEach], p[kRowsEach], m[kRowsEach];
 #pragma unroll
-        for (int k = 0; k < kRowsEach; ++k) {
-            const int y = kRowsEach * q.y + k;
-            if (y >= H) break;
-            const long long v = (plane * H + y) * W + q.x;
-            const long long u = ((static_cast<long long>(q.b) * (D / 2) + q.z / 2) * (H / 2) + y / 2) * (W / 2) + q.x / 2;
-            a[k] = *reinterpret_cast<const Vec8 *>(dcat + v * ccat + c1 + 8 * q.g);
-            p[k] = *reinterpret_cast<const Vec8 *>(dpool + u * c2 + 8 * q.g);
-            m[k] = *reinterpret_cast<const Vec8 *>(skip + v * c2 + 8 * q.g);
-        }
+            for (int k = 0; k < kRowsEach; ++k) {
+                const int y = kRowsEach * q.y + k;
+                if (y >= H) break;
+                const long long v = (plane * H + y) * W + q.x;
+                const long long u = ((static_cast<long long>(q.b) * (D / 2) + q.z / 2) * (H / 2) + y / 2) * (W / 2) + q.x / 2;
+                a[k] = *reinterpret_cast<const Vec8 *>(dcat + v * ccat + c1 + 8 * q.g);
+                p[k] = *reinterpret_cast<const Vec8 *>(dpool + u * c2 + 8 * q.g);
+                m[k] = *reinterpret_cast<const Vec8 *>(skip + v * c2 + 8 * q.g);
+            }
 #pragma unroll
-        for (int k = 0; k < kRowsEach; ++k) {
-            const int y = kRowsEach * q.y + k;
-            if (y >= H) break;
-            float f[8], g[8], r[8];
-            unpack8(f, a[k]);
-            unpack8(g, p[k]);
-            unpack8(r, m[k]);
+            for (int k = 0; k < kRowsEach; ++k) {
+                const int y = kRowsEach * q.y + k;
+                if (y >= H) break;
+                float f[8], g[8], r[8];
+                unpack8(f, a[k]);
+                unpack8(g, p[k]);
+                unpack8(r, m[k]);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] = (r[j] > 0.f) ? f[j] + 0.125f * g[j] : 0.f;
-            store8(dpre + ((plane * H + y) * W + q.x) * c2 + 8 * q.g, f);
+                for (int j = 0; j < 8; ++j) f[j] = (r[j] > 0.f) ? f[j] + 0.125f * g[j] : 0.f;
+                store8(dpre + ((plane * H + y) * W + q.x) * c2 + 8 * q.g, f);
+            }
         }
     }
 }
@@ -589,27 +599,29 @@ __device__ __forceinline__ float straightRayContrast(const float *sl, const Geom
 // 694 now; the 16 bytes a node reads and the 32 it writes would take 60.
 __global__ void __launch_bounds__(kThreads) featuresKernel(const float *slow, const float *tables, Geometry g, bf16 *feat) {
     const long long V = static_cast<long long>(g.nx) * g.ny * g.nz;
-    const int b = blockIdx.z, z = blockIdx.y;
+    const int b = blockIdx.z;
     const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = static_cast<int>(p / static_cast<unsigned>(g.nx)), x = static_cast<int>(p - static_cast<unsigned>(y) * g.nx);
     if (y >= g.ny) return;
     const float *sl = slow + b * V, *table = tables + b * tableLength(g);
-    const long long v = static_cast<long long>(z) * g.nx * g.ny + p;
-    const NodeGeom n = nodeGeom(table, g, x, y, z);
     const float invL = static_cast<float>(g.invL);
     const bool inside = table[1] >= 0.f && table[1] <= static_cast<float>(g.nx - 1) && table[2] >= 0.f &&
                         table[2] <= static_cast<float>(g.ny - 1) && table[3] >= 0.f && table[3] <= static_cast<float>(g.nz - 1);
-    float f[8] = {sl[v] / table[0] - 1.f,
-                  n.dist * invL,
-                  n.ddx * invL,
-                  n.ddy * invL,
-                  n.ddz * invL,
-                  inside ? straightRayContrast<true>(sl, g, table, x, y, z) : straightRayContrast<false>(sl, g, table, x, y, z),
-                  0.f,
-                  0.f};
-    store8(feat + (b * V + v) * 16, f);
-    const float zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    store8(feat + (b * V + v) * 16 + 8, zero);
+    for (int z = blockIdx.y; z < g.nz; z += gridDim.y) {   // one plane, unless there are more than a launch takes
+        const long long v = static_cast<long long>(z) * g.nx * g.ny + p;
+        const NodeGeom n = nodeGeom(table, g, x, y, z);
+        float f[8] = {sl[v] / table[0] - 1.f,
+                      n.dist * invL,
+                      n.ddx * invL,
+                      n.ddy * invL,
+                      n.ddz * invL,
+                      inside ? straightRayContrast<true>(sl, g, table, x, y, z) : straightRayContrast<false>(sl, g, table, x, y, z),
+                      0.f,
+                      0.f};
+        store8(feat + (b * V + v) * 16, f);
+        const float zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        store8(feat + (b * V + v) * 16 + 8, zero);
+    }
 }
 
 __device__ __forceinline__ float warpSum(float v) {
@@ -1439,9 +1451,12 @@ cudaError_t launchBiasGrad(const bf16 *dy, int c, long long nodes, float *db, in
 }
 
 namespace {
+// The y or z extent of a launch grid for n of something that the kernel steps through by it: a
+// launch takes up to 65535.
+unsigned gridYZ(long long n) { return static_cast<unsigned>(n < 65535 ? n : 65535); }
 // Grid of the kernels over 16-byte pieces (pieceOf): W x H rows, `planes` planes.
 dim3 pieceGrid(int W, int C, int H, long long planes) {
-    return dim3((W * (C / 8) + kThreads - 1) / kThreads, H, static_cast<unsigned>(planes < 65535 ? planes : 65535));
+    return dim3((W * (C / 8) + kThreads - 1) / kThreads, gridYZ(H), gridYZ(planes));
 }
 // Blocks of a sample in the kernels with sums (forNodes): eight per SM over all samples.
 dim3 nodeGrid(const Geometry &g, int B, int numSMs) {
@@ -1480,7 +1495,7 @@ cudaError_t launchSlowness(const Sample *samples, Geometry g, int B, float *slow
 }
 
 cudaError_t launchFeatures(const float *slow, const float *tables, Geometry g, int B, bf16 *feat, cudaStream_t s) {
-    const dim3 grid(static_cast<unsigned>((static_cast<long long>(g.nx) * g.ny + kThreads - 1) / kThreads), g.nz, B);
+    const dim3 grid(static_cast<unsigned>((static_cast<long long>(g.nx) * g.ny + kThreads - 1) / kThreads), gridYZ(g.nz), B);
     featuresKernel<<<grid, kThreads, 0, s>>>(slow, tables, g, feat);
     return cudaGetLastError();
 }
