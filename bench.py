@@ -359,9 +359,8 @@ def run_gpu(args):
     peak, peak_kind = _peaks()
     tr = _traffic()
     shapes = {1: "8x4", 2: "4x8", 3: "16x2"}
-    # the default is the wave-step kernel, which a tuning entry reports as the
-    # choice whose time is the default's
-    wave = KERNEL[0] == 0 and not PAIR[0] and (not tuning or tuning["ms_per_sweep"] == tuning["default_ms_per_sweep"])
+    # the default is the wave-step kernel
+    wave = KERNEL[0] == 0 and not PAIR[0] and (not tuning or tuning["wave_step"] == 1)
     if wave:
         kernel_name = "sweep3WaveKernel<float,near64>" if NEAR64[0] else "sweep3WaveKernel<float>"
     elif NEAR64[0]:

@@ -115,7 +115,7 @@ class _Src2(ctypes.Structure):
 class _Tuning(ctypes.Structure):
     _fields_ = [("sweep_kernel", ctypes.c_int), ("pair_fields", ctypes.c_int), ("block_shape", ctypes.c_int),
                 ("blocks_per_sm", ctypes.c_int), ("ms_per_sweep", ctypes.c_double),
-                ("default_ms_per_sweep", ctypes.c_double), ("candidates", ctypes.c_int)]
+                ("default_ms_per_sweep", ctypes.c_double), ("candidates", ctypes.c_int), ("wave_step", ctypes.c_int)]
 
 
 class _Model3(ctypes.Structure):
@@ -433,7 +433,8 @@ class Context:
     def autotune3d(self, sources, precision=F32):
         """Time the kernel variants, warp-block shapes and grid sizes on this model and these
         sources; later solves of the same grid class with default options use the fastest.
-        Returns the choice as a dict."""
+        Returns the choice as a dict; where its wave_step is 1, the options that ask for it are
+        blocks_per_sm alone (see eikx_tuning)."""
         src = np.atleast_2d(np.asarray(sources, dtype=np.float64))
         arr = (_Src3 * len(src))(*[_Src3(*map(float, q)) for q in src])
         t = _Tuning()

@@ -192,12 +192,6 @@ struct TuneKey {
         return std::tie(precision, uniform, nx, ny, nz, nsrc) < std::tie(o.precision, o.uniform, o.nx, o.ny, o.nz, o.nsrc);
     }
 };
-// A tuning entry: the reported choice, and whether it is the default kernel (wave-step), which
-// eikx_tuning has no value for (it then reads chunk-step, 8x4).
-struct Tuned {
-    eikx_tuning t{};
-    bool wave = false;
-};
 TuneKey tuneKey(int precision, bool uniform, int nx, int ny, int nz, int nSrc) {
     int p2 = 1;
     while (p2 < nSrc) p2 <<= 1;
@@ -247,7 +241,7 @@ struct eikx_ctx {
     DevBuf scratch;                // staging for host inputs and analytic fields
     Workspace ws;
     BatchWorkspace bw;
-    std::map<TuneKey, Tuned> tuning;   // eikx_autotune3d results per grid class
+    std::map<TuneKey, eikx_tuning> tuning;   // eikx_autotune3d results per grid class
     // the last eikx_solve3d / eikx_solve2d: its fields stay in ws.tt (row pitch Px)
     struct {
         bool valid = false;
@@ -833,10 +827,10 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
         const int perLaunch = o.max_in_flight > 0 && o.max_in_flight < nSrc ? o.max_in_flight : nSrc;
         auto it = c->tuning.find(tuneKey(P, uniform, nx, ny, nz, perLaunch));
         if (it != c->tuning.end()) {
-            o.sweep_kernel = it->second.wave ? eikx::kWaveStep : it->second.t.sweep_kernel;
-            o.pair_fields = it->second.t.pair_fields;
-            o.block_shape = it->second.wave ? 0 : it->second.t.block_shape;
-            o.blocks_per_sm = it->second.t.blocks_per_sm;
+            o.sweep_kernel = it->second.wave_step ? eikx::kWaveStep : it->second.sweep_kernel;
+            o.pair_fields = it->second.pair_fields;
+            o.block_shape = it->second.wave_step ? 0 : it->second.block_shape;
+            o.blocks_per_sm = it->second.blocks_per_sm;
         }
     }
     // the FP64 factored branch runs in the wave-step and chunk-step kernels (their own instances)
@@ -1874,8 +1868,7 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
     add(eikx::kNodeStep, 0, 1, eikx::sweep3BlocksPerSM<T>(uniform));
     if (std::is_same<T, float>::value && uniform && nSrc >= 2) add(eikx::kChunkStep, 1, 1, eikx::sweep3PairBlocksPerSM());
     double best = 1e300, dflt = -1;
-    Tuned entry;
-    eikx_tuning &pick = entry.t;
+    eikx_tuning pick{};
     for (size_t i = 0; i < cands.size(); ++i) {
         double ms = 0;
         for (int rep = 0; rep < 2; ++rep) {
@@ -1886,17 +1879,17 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
         if (i == 0) dflt = ms;
         if (ms < best) {
             best = ms;
-            entry.wave = cands[i].sweep_kernel == eikx::kWaveStep;
-            pick.sweep_kernel = entry.wave ? eikx::kChunkStep : cands[i].sweep_kernel;
+            pick.wave_step = cands[i].sweep_kernel == eikx::kWaveStep;
+            pick.sweep_kernel = pick.wave_step ? eikx::kChunkStep : cands[i].sweep_kernel;
             pick.pair_fields = cands[i].pair_fields;
-            pick.block_shape = entry.wave ? 1 : cands[i].block_shape;
+            pick.block_shape = pick.wave_step ? 1 : cands[i].block_shape;
             pick.blocks_per_sm = cands[i].blocks_per_sm;
         }
     }
     pick.ms_per_sweep = best;
     pick.default_ms_per_sweep = dflt;
     pick.candidates = static_cast<int>(cands.size());
-    c->tuning[tuneKey(P, uniform, c->nx, c->ny, c->nz, nSrc)] = entry;
+    c->tuning[tuneKey(P, uniform, c->nx, c->ny, c->nz, nSrc)] = pick;
     if (res) *res = pick;
     return EIKX_OK;
 }
@@ -2184,13 +2177,13 @@ eikx_status eikx_tuning_save(const eikx_ctx *c, const char *path) {
     if (!f) return fail(EIKX_ERR_INVALID, std::string("cannot write ") + path);
     for (const auto &kv : c->tuning) {
         const TuneKey &k = kv.first;
-        const eikx_tuning &t = kv.second.t;
+        const eikx_tuning &t = kv.second;
         f << "{\"precision\": " << k.precision << ", \"uniform\": " << k.uniform << ", \"nx\": " << k.nx
           << ", \"ny\": " << k.ny << ", \"nz\": " << k.nz << ", \"nsrc\": " << k.nsrc
           << ", \"sweep_kernel\": " << t.sweep_kernel << ", \"pair_fields\": " << t.pair_fields
           << ", \"block_shape\": " << t.block_shape << ", \"blocks_per_sm\": " << t.blocks_per_sm
           << ", \"ms_per_sweep\": " << t.ms_per_sweep << ", \"default_ms_per_sweep\": " << t.default_ms_per_sweep
-          << ", \"candidates\": " << t.candidates << (kv.second.wave ? ", \"wave\": 1" : "") << "}\n";
+          << ", \"candidates\": " << t.candidates << ", \"wave\": " << t.wave_step << "}\n";
     }
     return f ? EIKX_OK : fail(EIKX_ERR_INVALID, std::string("cannot write ") + path);
 }
@@ -2202,13 +2195,12 @@ eikx_status eikx_tuning_load(eikx_ctx *c, const char *path) {
     if (!f) return fail(EIKX_ERR_INVALID, std::string("cannot read ") + path);
     std::string line;
     int lineNo = 0;
-    std::map<TuneKey, Tuned> add;
+    std::map<TuneKey, eikx_tuning> add;
     while (std::getline(f, line)) {
         ++lineNo;
         if (line.find_first_not_of(" \t\r") == std::string::npos) continue;
         TuneKey k{};
-        Tuned entry;
-        eikx_tuning &t = entry.t;
+        eikx_tuning t{};
         const int got = std::sscanf(line.c_str(),
                                     " {\"precision\": %d, \"uniform\": %d, \"nx\": %d, \"ny\": %d, \"nz\": %d, "
                                     "\"nsrc\": %d, \"sweep_kernel\": %d, \"pair_fields\": %d, \"block_shape\": %d, "
@@ -2220,8 +2212,11 @@ eikx_status eikx_tuning_load(eikx_ctx *c, const char *path) {
         if (got != 13 || t.sweep_kernel < 1 || t.sweep_kernel > 2 || t.block_shape < 1 ||
             t.block_shape > eikx::kNumShapes || t.blocks_per_sm < 0)
             return fail(EIKX_ERR_INVALID, std::string(path) + ":" + std::to_string(lineNo) + ": not a tuning entry");
-        entry.wave = line.find("\"wave\": 1") != std::string::npos;
-        add[k] = entry;
+        // an entry without the mark was chosen before wave-step was a candidate
+        const size_t wave = line.find("\"wave\": ");
+        if (wave == std::string::npos) continue;
+        t.wave_step = line[wave + 8] == '1';
+        add[k] = t;
     }
     for (const auto &kv : add) c->tuning[kv.first] = kv.second;
     return EIKX_OK;

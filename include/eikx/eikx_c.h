@@ -276,16 +276,16 @@ eikx_status eikx_trace_rays2d(eikx_ctx *ctx, int nx, int nz, double dx, double d
 
 /* The configuration eikx_autotune3d chose for one grid class. */
 typedef struct {
-    int sweep_kernel;              /* 1 = node-step, 2 = chunk-step; where the untuned default
-                                      (wave-step, no value here) is the
-                                      fastest, 2 with block_shape 1 and ms_per_sweep equal to
-                                      default_ms_per_sweep */
+    int sweep_kernel;              /* 1 = node-step, 2 = chunk-step (also where wave_step is 1) */
     int pair_fields;               /* 1 = two FP32 fields per lane */
-    int block_shape;               /* 1 = 8x4, 2 = 4x8, 3 = 16x2 (chunk-step) */
+    int block_shape;               /* 1 = 8x4, 2 = 4x8, 3 = 16x2 (chunk-step; 1 where wave_step is 1) */
     int blocks_per_sm;             /* resident blocks per SM of the persistent grid */
     double ms_per_sweep;           /* measured mean sweep launch of the choice */
     double default_ms_per_sweep;   /* the untuned default, full grid */
     int candidates;                /* configurations timed */
+    int wave_step;                 /* 1 = the choice is wave-step, which eikx_options has no value for:
+                                      to ask for it, leave sweep_kernel, block_shape and pair_fields 0
+                                      and copy blocks_per_sm alone */
 } eikx_tuning;
 
 /* No counterpart in the reference.  Times the sweep kernels, warp-block shapes and grid
@@ -299,7 +299,8 @@ typedef struct {
 eikx_status eikx_autotune3d(eikx_ctx *ctx, const eikx_source3d *src, int n_src, int precision,
                             eikx_tuning *out);
 /* Writes the context's tuning table to `path` (one JSON object per line) / merges the
- * table at `path` into the context. */
+ * table at `path` into the context.  Entries of a table written before wave-step was among the
+ * candidates (without its mark) are left out: what they chose was not timed against it. */
 eikx_status eikx_tuning_save(const eikx_ctx *ctx, const char *path);
 eikx_status eikx_tuning_load(eikx_ctx *ctx, const char *path);
 
