@@ -72,7 +72,7 @@ class _Options(ctypes.Structure):
                 ("pair_fields", ctypes.c_int), ("sweep_kernel", ctypes.c_int),
                 ("block_shape", ctypes.c_int), ("blocks_per_sm", ctypes.c_int),
                 ("test_tag_margin", ctypes.c_int), ("near_fp64", ctypes.c_int), ("warm_gate", ctypes.c_int),
-                ("max_in_flight", ctypes.c_int), ("reserved", ctypes.c_int)]
+                ("max_in_flight", ctypes.c_int), ("test_alloc_fail", ctypes.c_int)]
 
 
 class _Stats(ctypes.Structure):
@@ -228,6 +228,7 @@ class Options:
     near_fp64: bool = False       # 3D FP32: factored (near-source) updates in FP64
     warm_gate: int = 0            # solve3d_warm residual gate: 0 one-sided, 1 two-sided
     max_in_flight: int = 0        # solve3d: > 0 = a stream of the sources through this many slots
+    test_alloc_fail: int = 0      # test hook only (see eikx_options.test_alloc_fail)
 
     def _c(self):
         o = _Options()
@@ -247,6 +248,7 @@ class Options:
         o.near_fp64 = int(bool(self.near_fp64))
         o.warm_gate = int(self.warm_gate)
         o.max_in_flight = int(self.max_in_flight)
+        o.test_alloc_fail = int(self.test_alloc_fail)
         return o
 
 

@@ -51,7 +51,12 @@ struct DevBuf {
         if (n <= bytes && p) return cudaSuccess;
         release();
         cudaError_t e = cudaMalloc(&p, n ? n : 16);
-        if (e == cudaSuccess) bytes = n; else p = nullptr;
+        if (e == cudaSuccess) {
+            bytes = n;
+        } else {
+            p = nullptr;
+            cudaGetLastError();   // reported here; the next launch check is not to find it
+        }
         return e;
     }
     void release() {
@@ -180,7 +185,7 @@ struct ScheduleKey {
         warm = 0, early = 0, nearFp64 = 0, warmGate = 0;
     double tol = 0, h = 0, dx = 0, dy = 0, dz = 0, gate = 0;
     unsigned long long spin = 0;
-    const void *tt = nullptr, *sp = nullptr, *hs = nullptr, *srcs = nullptr, *corners = nullptr, *flags = nullptr;
+    const void *tt = nullptr, *sp[2] = {}, *hs[2] = {}, *srcs = nullptr, *corners = nullptr, *flags = nullptr;
     bool operator==(const ScheduleKey &o) const { return std::memcmp(this, &o, sizeof(*this)) == 0; }
 };
 
@@ -221,9 +226,9 @@ struct eikx_ctx {
     mutable std::vector<double> hostSlow3;   // host copy, fetched when first asked for
     mutable bool hostSlow3Valid = false;
     DevBuf spad3[2][2];            // [precision][0: shifted for +x sweeps, 1: unshifted]
-    bool spadValid3[2] = {false, false};
+    bool spadValid3[2][2] = {};
     DevBuf shad3[2][2];            // the same multiplied by h (uniform grids; wave-step and FP64 chunk-step)
-    bool shadValid3[2] = {false, false};
+    bool shadValid3[2][2] = {};
     // 2D model
     int nx2 = 0, nz2 = 0;
     double dx2 = 0, dz2 = 0, x02 = 0, z02 = 0;
@@ -235,9 +240,9 @@ struct eikx_ctx {
     DevBuf rayGrad, raySlow, raySt, rayPos, raySeg, rayCnt;   // eikx_trace_rays2d buffers
     PinnedBuf srcSlow;             // source-cell slownesses of a solve, read from the device
     DevBuf spad2[2][2];
-    bool spadValid2[2] = {false, false};
+    bool spadValid2[2][2] = {};
     DevBuf shad2[2];               // FP64, the same multiplied by h (uniform grids)
-    bool shadValid2 = false;
+    bool shadValid2[2] = {};
     DevBuf scratch;                // staging for host inputs and analytic fields
     Workspace ws;
     BatchWorkspace bw;
@@ -281,6 +286,16 @@ void dropGraph(eikx_ctx *c) {
     if (c->graphExec) cudaGraphExecDestroy(c->graphExec);
     c->graphExec = nullptr;
     c->graphKey = ScheduleKey{};
+}
+
+// A new model or grid: the padded copies are made again when a solve reads them.
+void dropPads(eikx_ctx *c, int dim) {
+    if (dim == 3) {
+        for (auto *v : {c->spadValid3, c->shadValid3}) v[0][0] = v[0][1] = v[1][0] = v[1][1] = false;
+    } else {
+        c->spadValid2[0][0] = c->spadValid2[0][1] = c->spadValid2[1][0] = c->spadValid2[1][1] = false;
+        c->shadValid2[0] = c->shadValid2[1] = false;
+    }
 }
 
 // Work-queue order: warp blocks of all fields sorted by the step at which they can start
@@ -342,12 +357,11 @@ eikx_status finishModel(eikx_ctx *c, int dim) {
     if (dim == 3) {
         c->haveSlow3 = false;
         c->hostSlow3Valid = false;
-        c->spadValid3[0] = c->spadValid3[1] = false;
-        c->shadValid3[0] = c->shadValid3[1] = false;
+        dropPads(c, 3);
     } else {
         c->haveSlow2 = false;
         c->hostSlow2Valid = false;
-        c->spadValid2[0] = c->spadValid2[1] = c->shadValid2 = false;
+        dropPads(c, 2);
     }
     if (bad) return fail(EIKX_ERR_INVALID, "Non-positive velocities detected");
     (dim == 3 ? c->haveSlow3 : c->haveSlow2) = true;
@@ -450,6 +464,7 @@ eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std
     // buffers
     const size_t mboxBytes = static_cast<size_t>(nProgress) * tl.faceWords * 8;
     EIKX_CUDA(w.tt.ensure(static_cast<size_t>(fieldStride) * nBufs * sizeof(T)));
+    if (o.test_alloc_fail == 1 && wave) return fail(EIKX_ERR_ALLOC, "test hook: the buffers do not fit");
     if (w.mbox.bytes < mboxBytes || !w.mbox.p) {
         EIKX_CUDA(w.mbox.ensure(mboxBytes));
         EIKX_CUDA(cudaMemsetAsync(w.mbox.p, 0, w.mbox.bytes, c->stream));
@@ -717,11 +732,12 @@ eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std
     return EIKX_OK;
 }
 
-// Shared solve driver for 2D and 3D.
+// Shared solve driver for 2D and 3D.  `lean`: the form that needs the least memory, for a solve by
+// default options whose buffers did not fit (solveImpl).
 
 template <class T, int DIM>
-eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options o, void *tOut,
-                      int where, const void *tInit = nullptr, int initWhere = EIKX_HOST, double gateTol = 0) {
+eikx_status solveOnce(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options o, void *tOut, int where, const void *tInit,
+                      int initWhere, double gateTol, bool lean) {
     const bool warm = DIM == 3 && tInit != nullptr;
     if (warm) o.init_sweeps = 0;   // the initial field replaces the initialisation pass
     const int P = precOf<T>();
@@ -778,49 +794,9 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                                    static_cast<double>(static_cast<T>(s))};
     }
 
-    // edge-replicated slowness in the sweep precision: one copy shifted by V-1 columns
-    // (16-byte chunks of V elements) for +x sweeps, one unshifted for -x sweeps
-    DevBuf *spad = DIM == 3 ? c->spad3[P] : c->spad2[P];
-    bool &spadValid = DIM == 3 ? c->spadValid3[P] : c->spadValid2[P];
-    const size_t spElems = static_cast<size_t>(spPitch) * (DIM == 3 ? ny + 1 : 1) * (nz + 1);
-    if (!spadValid || spad[0].bytes < spElems * sizeof(T)) {
-        if (spad[0].bytes < spElems * sizeof(T)) dropGraph(c);
-        for (int k = 0; k < 2; ++k) {
-            EIKX_CUDA(spad[k].ensure(spElems * sizeof(T)));
-            const int shift = k == 0 ? static_cast<int>(16 / sizeof(T)) - 1 : 0;
-            if (DIM == 3)
-                EIKX_CUDA((eikx::launchPadSlowness3<T, double>(spad[k].as<T>(), spPitch, shift, c->slow3.as<double>(),
-                                                               nx, ny, nz, c->stream)));
-            else
-                EIKX_CUDA((eikx::launchPadSlowness2<T, double>(spad[k].as<T>(), spPitch, shift, c->slow2.as<double>(),
-                                                               nx, nz, c->stream)));
-        }
-        spadValid = true;
-    }
-
-    // the factor tables are filled from the unshifted padded copy (FP32 sweeps)
-    for (auto &f : srcT64) {
-        if (f.bnx == 0)
-            return fail(EIKX_ERR_UNSUPPORTED, "near_fp64: the factored region of radius " +
-                                                  std::to_string(o.factored_radius) + " needs more than " +
-                                                  std::to_string(eikx::kMaxFactorTable) + " table entries");
-        f.sp = static_cast<const float *>(spad[1].p);
-    }
-
     // geometry in the sweep type (include/private/solver3d.hpp:31-44, solver2d.hpp:29-46)
     const double eps = std::numeric_limits<T>::epsilon() * 100;
     const bool uniform = DIM == 3 ? (std::abs(dx - dy) < eps && std::abs(dx - dz) < eps) : (std::abs(dx - dz) < eps);
-    // 2D, FP64, uniform: the padded copies multiplied by h, which the wave-step kernel reads
-    if (DIM == 2 && sizeof(T) == 8 && uniform && (!c->shadValid2 || c->shad2[0].bytes < spElems * sizeof(T))) {
-        if (c->shad2[0].bytes < spElems * sizeof(T)) dropGraph(c);
-        for (int k = 0; k < 2; ++k) {
-            EIKX_CUDA(c->shad2[k].ensure(spElems * sizeof(T)));
-            const int shift = k == 0 ? static_cast<int>(16 / sizeof(T)) - 1 : 0;
-            EIKX_CUDA((eikx::launchPadSlowness2<T, double>(c->shad2[k].as<T>(), spPitch, shift, c->slow2.as<double>(), nx, nz,
-                                                           c->stream, static_cast<T>(dx))));
-        }
-        c->shadValid2 = true;
-    }
     // options left at "auto" take the tuned configuration of this grid class
     if (DIM == 3 && o.sweep_kernel == 0 && o.block_shape == 0 && o.blocks_per_sm == 0 && !o.pair_fields) {
         // a stream launches its slots' fields, not all of its sources
@@ -833,6 +809,8 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
             o.blocks_per_sm = it->second.blocks_per_sm;
         }
     }
+    if (DIM == 3 && lean && (o.sweep_kernel == eikx::kWaveStep || (o.sweep_kernel == 0 && o.block_shape == 0)))
+        o.sweep_kernel = eikx::kChunkStep;
     // the FP64 factored branch runs in the wave-step and chunk-step kernels (their own instances)
     if (DIM == 3 && P == EIKX_F32 && o.near_fp64) {
         if (o.sweep_kernel == eikx::kNodeStep) o.sweep_kernel = eikx::kChunkStep;
@@ -855,20 +833,53 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                         (o.sweep_kernel == eikx::kWaveStep || (o.sweep_kernel == 0 && o.block_shape == 0));
     const int variant = wave ? eikx::kWaveStep : o.sweep_kernel == eikx::kNodeStep ? eikx::kNodeStep : eikx::kChunkStep;
     const bool chunkStep = DIM == 3 && !paired && variant == eikx::kChunkStep;
-    // uniform 3D grids: the padded copies multiplied by h, which the wave-step kernel and the
-    // FP64 chunk-step kernel read
-    DevBuf *shad = c->shad3[P];
-    if (DIM == 3 && uniform && (wave || (sizeof(T) == 8 && chunkStep)) &&
-        (!c->shadValid3[P] || shad[0].bytes < spElems * sizeof(T))) {
-        if (shad[0].bytes < spElems * sizeof(T)) dropGraph(c);
-        for (int k = 0; k < 2; ++k) {
-            EIKX_CUDA(shad[k].ensure(spElems * sizeof(T)));
-            const int shift = k == 0 ? static_cast<int>(16 / sizeof(T)) - 1 : 0;
-            EIKX_CUDA((eikx::launchPadSlowness3<T, double>(shad[k].as<T>(), spPitch, shift, c->slow3.as<double>(),
-                                                           nx, ny, nz, c->stream, static_cast<T>(dx))));
-        }
-        c->shadValid3[P] = true;
+    // 2D grids of up to 512 rows can run one CTA per field (sweep_kernel = 2); the warp-block
+    // kernel is the default: measured faster on GB300 for 1 to 512 fields of 501 x 251 nodes
+    const bool block2 = DIM == 2 && nz <= eikx::kMaxBlockRows2 && o.sweep_kernel == eikx::kChunkStep;
+
+    // Edge-replicated slowness in the sweep precision: one copy shifted by V-1 columns (16-byte
+    // chunks of V elements) for +x sweeps, one unshifted for -x sweeps, and the two multiplied by h.
+    // A solve makes those that its kernel reads: on uniform grids the wave-step kernel the scaled
+    // ones and, for its factored branch, the plain unshifted one (2D in double: the cells); the FP64
+    // chunk-step kernel the scaled ones too; all else the plain ones.
+    const bool scaled2 = DIM == 2 && sizeof(T) == 8 && uniform && !block2;
+    const bool scaled = DIM == 3 ? uniform && (wave || (sizeof(T) == 8 && chunkStep)) : scaled2;
+    DevBuf *spad = DIM == 3 ? c->spad3[P] : c->spad2[P];
+    bool *spadValid = DIM == 3 ? c->spadValid3[P] : c->spadValid2[P];
+    DevBuf *shad = DIM == 3 ? c->shad3[P] : c->shad2;
+    bool *shadValid = DIM == 3 ? c->shadValid3[P] : c->shadValid2;
+    const size_t spElems = static_cast<size_t>(spPitch) * (DIM == 3 ? ny + 1 : 1) * (nz + 1);
+    auto pad = [&](DevBuf &buf, bool &valid, int shift, T times) -> eikx_status {
+        if (valid && buf.bytes >= spElems * sizeof(T)) return EIKX_OK;
+        if (buf.bytes < spElems * sizeof(T)) dropGraph(c);
+        EIKX_CUDA(buf.ensure(spElems * sizeof(T)));
+        if (DIM == 3)
+            EIKX_CUDA((eikx::launchPadSlowness3<T, double>(buf.as<T>(), spPitch, shift, c->slow3.as<double>(), nx, ny, nz,
+                                                           c->stream, times)));
+        else
+            EIKX_CUDA((eikx::launchPadSlowness2<T, double>(buf.as<T>(), spPitch, shift, c->slow2.as<double>(), nx, nz,
+                                                           c->stream, times)));
+        valid = true;
+        return EIKX_OK;
+    };
+    const bool needPad[2] = {!(scaled2 || (DIM == 3 && uniform && wave)), !scaled2};
+    for (int k = 0; k < 2; ++k) {
+        const int shift = k == 0 ? static_cast<int>(16 / sizeof(T)) - 1 : 0;
+        if (needPad[k])
+            if (eikx_status r = pad(spad[k], spadValid[k], shift, T(0)); r != EIKX_OK) return r;
+        if (scaled)
+            if (eikx_status r = pad(shad[k], shadValid[k], shift, static_cast<T>(dx)); r != EIKX_OK) return r;
     }
+
+    // the factor tables are filled from the unshifted padded copy (FP32 sweeps)
+    for (auto &f : srcT64) {
+        if (f.bnx == 0)
+            return fail(EIKX_ERR_UNSUPPORTED, "near_fp64: the factored region of radius " +
+                                                  std::to_string(o.factored_radius) + " needs more than " +
+                                                  std::to_string(eikx::kMaxFactorTable) + " table entries");
+        f.sp = static_cast<const float *>(spad[1].p);
+    }
+
     // a stream of the sources through max_in_flight slots
     if constexpr (DIM == 3) {
         if (stream)
@@ -878,9 +889,6 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     const int nUnits = paired ? (nSrc + 1) / 2 : nSrc;   // work units: fields or field pairs
 
     // warp-block shape
-    // 2D grids of up to 512 rows can run one CTA per field (sweep_kernel = 2); the warp-block
-    // kernel is the default: measured faster on GB300 for 1 to 512 fields of 501 x 251 nodes
-    const bool block2 = DIM == 2 && nz <= eikx::kMaxBlockRows2 && o.sweep_kernel == eikx::kChunkStep;
     const int shape = chunkStep && o.block_shape > 0 ? o.block_shape - 1 : eikx::kShape8x4;
 
     // workspace
@@ -902,12 +910,13 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
     int blocks = std::min(c->numSMs * perSM, (nProgress + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock);
     blocks = std::max(blocks, 1);
-    const bool both = bothSweeps(DIM == 2 ? !block2 : wave, nProgress, static_cast<size_t>(c->numSMs) * perSM * eikx::kWarpsPerBlock);
+    const bool both = !lean && bothSweeps(DIM == 2 ? !block2 : wave, nProgress, static_cast<size_t>(c->numSMs) * perSM * eikx::kWarpsPerBlock);
     const size_t ttBytes = static_cast<size_t>(fieldStride) * nSrc * sizeof(T);
     const size_t mboxBytes = static_cast<size_t>(nProgress) * tl.faceWords * 8 * (both ? 2 : 1);
     const void *before[] = {w.tt.p, w.mbox.p, w.epoch.p, w.residual.p, w.converged.p,
                             w.iterations.p, w.order.p, w.srcs.p, w.corners.p, w.srcs64.p, w.factor.p};
     EIKX_CUDA(w.tt.ensure(ttBytes));
+    if (o.test_alloc_fail == 1 && !lean && (wave || DIM == 2)) return fail(EIKX_ERR_ALLOC, "test hook: the buffers do not fit");
     if (w.mbox.bytes < mboxBytes || !w.mbox.p) {
         // fresh words carry tag 0, which no sweep uses
         EIKX_CUDA(w.mbox.ensure(mboxBytes));
@@ -1037,7 +1046,11 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     sk.warmGate = warm ? o.warm_gate : 0;
     sk.variant = DIM == 3 ? variant : block2 ? 1 : 0;
     sk.shape = shape;
-    sk.tt = w.tt.p; sk.sp = spad[0].p; sk.hs = DIM == 3 ? shad[0].p : c->shad2[0].p; sk.srcs = w.srcs.p; sk.corners = w.corners.p;
+    sk.tt = w.tt.p; sk.srcs = w.srcs.p; sk.corners = w.corners.p;
+    for (int k = 0; k < 2; ++k) {
+        sk.sp[k] = needPad[k] ? spad[k].p : nullptr;
+        sk.hs[k] = scaled ? shad[k].p : nullptr;
+    }
     sk.early = early ? 1 : 0;
     sk.flags = iterFlags;
 
@@ -1137,8 +1150,9 @@ eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
                 a.sp2 = g;
                 if (block2) EIKX_CUDA(eikx::launchSweep2Block<T>(a, uniform, nSrc, c->stream));
                 else {
-                    if (sizeof(T) == 8 && uniform) {
-                        a.hsPos = c->shad2[0].as<T>(); a.hsNeg = c->shad2[1].as<T>();
+                    if (scaled2) {
+                        a.hsPos = shad[0].as<T>(); a.hsNeg = shad[1].as<T>();
+                        a.cells = c->slow2.as<double>();
                     }
                     EIKX_CUDA(eikx::launchSweep2Wave<T>(a, uniform, blocks, c->stream));
                 }
@@ -1365,6 +1379,37 @@ std::string checkModel(const eikx_model3d &m, int i) {
 
 // One schedule over the selected models of a batch (all with uniform or all with
 // non-uniform spacing).  Statistics are accumulated into `agg`.
+// Gives back what the wave-step kernels keep beside what the others do: the copies of the
+// slowness multiplied by h, and the mailboxes.
+void releaseWave(eikx_ctx *c) {
+    cudaGetLastError();   // the failed allocation's
+    cudaStreamSynchronize(c->stream);
+    dropGraph(c);
+    c->bw.dropGraph();
+    for (int p = 0; p < 2; ++p)
+        for (int k = 0; k < 2; ++k) {
+            c->shad3[p][k].release();
+            c->shadValid3[p][k] = false;
+        }
+    c->ws.mbox.release();
+    c->sw.mbox.release();
+    c->bw.mbox.release();
+    c->bw.sp.release();
+}
+
+// A solve.  The wave-step kernel needs more memory than the chunk-step kernel (in FP32 on a uniform grid
+// a third copy of the slowness; a mailbox of Px + 32 columns per warp block, twice where both
+// orderings share a launch): a call that asks for no kernel and whose buffers do not fit runs once
+// more with the chunk-step kernel, in 2D with one ordering per launch, so that what fits there runs.
+template <class T, int DIM>
+eikx_status solveImpl(eikx_ctx *c, const double *srcXYZ, int nSrc, const eikx_options &o, void *tOut, int where,
+                      const void *tInit = nullptr, int initWhere = EIKX_HOST, double gateTol = 0) {
+    const eikx_status r = solveOnce<T, DIM>(c, srcXYZ, nSrc, o, tOut, where, tInit, initWhere, gateTol, false);
+    if (r != EIKX_ERR_ALLOC || (DIM == 3 && (o.sweep_kernel != 0 || o.block_shape != 0))) return r;
+    releaseWave(c);
+    return solveOnce<T, DIM>(c, srcXYZ, nSrc, o, tOut, where, tInit, initWhere, gateTol, true);
+}
+
 template <class T>
 eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vector<int> &sel, bool uniform,
                         const eikx_options &o, eikx_stats &agg) {
@@ -1372,7 +1417,10 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     constexpr int V = 16 / sizeof(T);
     const int shape = o.block_shape > 0 ? o.block_shape - 1 : eikx::kShape8x4;
     const bool wave = o.sweep_kernel == 0 && o.block_shape == 0;   // as solveImpl
-    const int nCopies = wave && uniform ? 4 : 2;   // padded slowness copies: shifted, unshifted, then both times h
+    // padded slowness copies: the wave-step kernel on uniform grids reads shifted and unshifted ones times
+    // h and the plain unshifted one, the others the plain ones (as solveImpl)
+    const bool scaled = wave && uniform;
+    const int nCopies = scaled ? 3 : 2;
     const int nM = static_cast<int>(sel.size());
     struct Layout {
         int nx, ny, nz, Px, spPitch, tilesY, tilesZ, firstUnit, nSrc;
@@ -1428,6 +1476,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     const void *before[] = {w.tt.p, w.sp.p, w.mbox.p, w.epoch.p, w.residual.p, w.converged.p, w.iterations.p,
                             w.order.p, w.srcs.p, w.corners.p, w.units.p, w.srcs64.p, w.factor.p};
     EIKX_CUDA(w.tt.ensure(ttElems * sizeof(T)));
+    if (o.test_alloc_fail == 1 && wave) return fail(EIKX_ERR_ALLOC, "test hook: the buffers do not fit");
     EIKX_CUDA(w.sp.ensure(spElems * sizeof(T)));
     if (w.mbox.bytes < mboxWords * 8 || !w.mbox.p) {
         // fresh words carry tag 0, which no sweep uses
@@ -1458,7 +1507,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
                            w.order.p, w.srcs.p, w.corners.p, w.units.p, w.srcs64.p, w.factor.p};
     if (std::memcmp(before, after, sizeof(before)) != 0) w.dropGraph();
 
-    // models -> cell slowness (FP64, natural) -> two padded copies in the sweep precision;
+    // models -> cell slowness (FP64, natural) -> padded copies in the sweep precision;
     // sources located on each model as eikx_solve3d does.  The whole batch is one stream
     // of work with a single synchronisation: positivity is checked on the device into one
     // flag and only the source cells' slowness comes back to the host.
@@ -1510,13 +1559,13 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
             else EIKX_CUDA(eikx::launchCellsToNatural3<double>(slow, f, m.nx, m.ny, m.nz, m.ordering, c->stream));
         }
         EIKX_CUDA(eikx::launchCheckPositive(slow, static_cast<long long>(nCell), w.badFlag.as<int>(), c->stream));
-        EIKX_CUDA((eikx::launchPadSlowness3<T, double>(spBase + l.spOff, l.spPitch, V - 1, slow, m.nx, m.ny, m.nz,
-                                                       c->stream)));
-        EIKX_CUDA((eikx::launchPadSlowness3<T, double>(spBase + l.spOff + l.spElems, l.spPitch, 0, slow, m.nx, m.ny,
-                                                       m.nz, c->stream)));
-        for (int k = 2; k < nCopies; ++k)
-            EIKX_CUDA((eikx::launchPadSlowness3<T, double>(spBase + l.spOff + k * l.spElems, l.spPitch, k == 2 ? V - 1 : 0,
-                                                           slow, m.nx, m.ny, m.nz, c->stream, static_cast<T>(m.dx))));
+        T *shifted = spBase + l.spOff, *plain = shifted + l.spElems, *plainH = scaled ? plain + l.spElems : nullptr;
+        EIKX_CUDA((eikx::launchPadSlowness3<T, double>(shifted, l.spPitch, V - 1, slow, m.nx, m.ny, m.nz, c->stream,
+                                                       scaled ? static_cast<T>(m.dx) : T(0))));
+        EIKX_CUDA((eikx::launchPadSlowness3<T, double>(plain, l.spPitch, 0, slow, m.nx, m.ny, m.nz, c->stream)));
+        if (scaled)
+            EIKX_CUDA((eikx::launchPadSlowness3<T, double>(plainH, l.spPitch, 0, slow, m.nx, m.ny, m.nz, c->stream,
+                                                           static_cast<T>(m.dx))));
         for (int j = 0; j < m.n_src; ++j) {
             const int u = l.firstUnit + j;
             const size_t cell = (static_cast<size_t>(srcT[u].isz) * (m.ny - 1) + srcT[u].isy) * (m.nx - 1) + srcT[u].isx;
@@ -1526,10 +1575,10 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
         for (int j = 0; j < m.n_src; ++j) {
             eikx::Grid3Unit<T> &gu = units[l.firstUnit + j];
             gu.tt = ttBase + l.ttOff + static_cast<size_t>(j) * l.fieldStride;
-            gu.spPos = spBase + l.spOff;
-            gu.spNeg = spBase + l.spOff + l.spElems;
-            gu.hsPos = nCopies == 4 ? spBase + l.spOff + 2 * l.spElems : nullptr;
-            gu.hsNeg = nCopies == 4 ? spBase + l.spOff + 3 * l.spElems : nullptr;
+            gu.spPos = scaled ? nullptr : shifted;
+            gu.spNeg = plain;
+            gu.hsPos = scaled ? shifted : nullptr;
+            gu.hsNeg = plainH;
             gu.mbox = mbBase + (l.mboxOff + static_cast<size_t>(j) * l.tilesY * l.tilesZ * l.faceWords) * (both ? 2 : 1);
             gu.spPlane = l.spPlane;
             gu.spPitch = l.spPitch;
@@ -1871,12 +1920,17 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
     eikx_tuning pick{};
     for (size_t i = 0; i < cands.size(); ++i) {
         double ms = 0;
-        for (int rep = 0; rep < 2; ++rep) {
-            if (eikx_status r = solveImpl<T, 3>(c, xyz.data(), nSrc, cands[i], c->tuneOut.p, EIKX_DEVICE); r)
-                return r;
+        eikx_status r = EIKX_OK;
+        for (int rep = 0; rep < 2 && r == EIKX_OK; ++rep) {
+            r = solveImpl<T, 3>(c, xyz.data(), nSrc, cands[i], c->tuneOut.p, EIKX_DEVICE);
             ms = c->stats.sweep_ms / std::max(1, c->stats.sweeps_launched);
         }
-        if (i == 0) dflt = ms;
+        if (r == EIKX_ERR_ALLOC && cands[i].sweep_kernel == eikx::kWaveStep) {
+            releaseWave(c);   // it does not fit: the default is the next one here (solveImpl)
+            continue;
+        }
+        if (r != EIKX_OK) return r;
+        if (dflt < 0) dflt = ms;
         if (ms < best) {
             best = ms;
             pick.wave_step = cands[i].sweep_kernel == eikx::kWaveStep;
@@ -1993,8 +2047,7 @@ eikx_status eikx_set_grid3d(eikx_ctx *c, int nx, int ny, int nz, double dx, doub
     c->x0 = x0; c->y0 = y0; c->z0 = z0;
     c->haveGrid3 = true;
     c->haveSlow3 = false;
-    c->spadValid3[0] = c->spadValid3[1] = false;
-    c->shadValid3[0] = c->shadValid3[1] = false;
+    dropPads(c, 3);
     dropGraph(c);
     return EIKX_OK;
 }
@@ -2009,7 +2062,7 @@ eikx_status eikx_set_grid2d(eikx_ctx *c, int nx, int nz, double dx, double dz, d
     c->nx2 = nx; c->nz2 = nz; c->dx2 = dx; c->dz2 = dz; c->x02 = x0; c->z02 = z0;
     c->haveGrid2 = true;
     c->haveSlow2 = false;
-    c->spadValid2[0] = c->spadValid2[1] = c->shadValid2 = false;
+    dropPads(c, 2);
     dropGraph(c);
     return EIKX_OK;
 }
@@ -2149,8 +2202,16 @@ eikx_status eikx_solve3d_batch(eikx_ctx *c, const eikx_model3d *models, int nMod
     for (int pass = 0; pass < 2; ++pass) {
         const std::vector<int> &sel = pass == 0 ? uni : non;
         if (sel.empty()) continue;
-        eikx_status r = precision == EIKX_F32 ? solveBatch3<float>(c, models, sel, pass == 0, o, agg)
-                                              : solveBatch3<double>(c, models, sel, pass == 0, o, agg);
+        auto solve = [&] {
+            return precision == EIKX_F32 ? solveBatch3<float>(c, models, sel, pass == 0, o, agg)
+                                         : solveBatch3<double>(c, models, sel, pass == 0, o, agg);
+        };
+        eikx_status r = solve();
+        if (r == EIKX_ERR_ALLOC && o.sweep_kernel == 0 && o.block_shape == 0) {   // as solveImpl
+            releaseWave(c);
+            o.sweep_kernel = eikx::kChunkStep;
+            r = solve();
+        }
         if (r != EIKX_OK) return r;
     }
     c->stats = agg;

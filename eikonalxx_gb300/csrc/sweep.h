@@ -119,7 +119,10 @@ template <class T> struct Sweep2Args {
     int radius;
     T h;
     Spacing2<T> sp2;
-    const T *hsPos, *hsNeg;   // FP64 wave-step kernel on a uniform grid: the copies multiplied by h
+    // FP64 wave-step kernel on a uniform grid: the copies multiplied by h, and the model's cells for the
+    // operators that take the slowness as it is (spPos and spNeg are not read)
+    const T *hsPos, *hsNeg;
+    const double *cells;
 };
 
 // Launchers (sweep.cu).  blocks = persistent grid size.

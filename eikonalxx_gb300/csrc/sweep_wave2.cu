@@ -41,14 +41,21 @@ template <class T> struct Smem2 {
     static constexpr unsigned kHalo = 48 * kChunkB;
 };
 
-// Out of line: the factored branch, and all Cartesian operators, from the unscaled slowness (cell
-// (cx, cz) of spNeg at (cz + 1) pitch + cx + 1, edges replicated).
+// Out of line: the factored branch, and all Cartesian operators, from the unscaled slowness: cell
+// (cx, cz) of spNeg at (cz + 1) pitch + cx + 1, edges replicated, or (FP64 on a uniform grid) the
+// model's own cells with pitch nx - 1, so that a solve keeps two copies of the slowness and not four.
 template <class T, bool UNIFORM, bool NEAR>
 __device__ __noinline__ T node2(T h, const Spacing2<T> &g, const SourceT<T> &src, const SweepSigns sg, int ix, int iz, T t1,
-                                T t2, T t3, const T *sp, int pitch) {
+                                T t2, T t3, const T *sp, int pitch, int nz) {
     const bool fx = sg.ixShift > 0, fz = sg.izShift > 0;
     const int xu = fx ? ix + 1 : ix, xo = fx ? ix : ix + 1, zu = fz ? iz + 1 : iz, zo = fz ? iz : iz + 1;
-    auto S = [&](int x, int z) { return sp[static_cast<long long>(z) * pitch + x]; };
+    auto S = [&](int x, int z) -> T {
+        if constexpr (UNIFORM && sizeof(T) == 8) {
+            x = min(max(x - 1, 0), pitch - 1);
+            z = min(max(z - 1, 0), nz - 2);
+        }
+        return sp[static_cast<long long>(z) * pitch + x];
+    };
     const T s0 = S(xu, zu), s1 = S(xo, zu), s3 = S(xu, zo);
     if constexpr (UNIFORM)
         return NEAR ? fd2UniformNear<T>(h, src, sg, ix, iz, s0, s1, s3, t1, t2, t3) : fd2UniformFar<T>(h, s0, s1, s3, t1, t2, t3);
@@ -82,6 +89,9 @@ __global__ void __launch_bounds__(kThreads2) sweep2WaveKernel(const Sweep2Args<T
     }
     const T huge = static_cast<T>(1.e10);
     const int Px = a.pitch, nx = a.nx, nz = a.nz, nChunks = Px / kG;
+    const T *raw = a.spNeg;               // the unscaled slowness (node2)
+    if constexpr (SCALED) raw = a.cells;
+    const int rawPitch = SCALED ? nx - 1 : a.spPitch;
     const long long fieldWords = static_cast<long long>(a.tilesZ) * waveStepCap2(Px) * W;
     const float hF = view(a.h), dxF = view(a.sp2.dx), dzF = view(a.sp2.dz), dMinF = fminf(dxF, dzF);
     bool ok = true;
@@ -250,7 +260,7 @@ __global__ void __launch_bounds__(kThreads2) sweep2WaveKernel(const Sweep2Args<T
                     if (tileNear) {
                         if (rowNear && upd && static_cast<unsigned>(p - nearFrom) <= 2u * rx) {
                             need = false;
-                            const T tu = node2<T, UNIFORM, true>(a.h, a.sp2, src, sg, xa, za, o1, nP, N, a.spNeg, a.spPitch);
+                            const T tu = node2<T, UNIFORM, true>(a.h, a.sp2, src, sg, xa, za, o1, nP, N, raw, rawPitch, nz);
                             if (tu < v) v = tu;
                         }
                     }
@@ -297,7 +307,7 @@ __global__ void __launch_bounds__(kThreads2) sweep2WaveKernel(const Sweep2Args<T
                             };
                             const bool again = need & (edge(vo, !above(nP, o1)) | edge(vN, !above(nP, N)));
                             if (__any_sync(kFull, again)) {
-                                if (again) best = dmin(best, node2<T, UNIFORM, false>(a.h, a.sp2, src, sg, xa, za, o1, nP, N, a.spNeg, a.spPitch));
+                                if (again) best = dmin(best, node2<T, UNIFORM, false>(a.h, a.sp2, src, sg, xa, za, o1, nP, N, raw, rawPitch, nz));
                             }
                             if (need) v = best;
                         } else if constexpr (!UNIFORM && sizeof(T) == 8) {
@@ -416,7 +426,7 @@ template <class T> int sweep2WaveBlocksPerSM(bool uniform) {
 // The caller asks sweep2WaveBlocksPerSM for the grid size first, which sets the kernel's
 // shared-memory limit.
 template <class T> cudaError_t launchSweep2Wave(const Sweep2Args<T> &a, bool uniform, int blocks, cudaStream_t s) {
-    if (uniform && sizeof(T) == 8 && (!a.hsPos || !a.hsNeg)) return cudaErrorInvalidValue;
+    if (uniform && sizeof(T) == 8 && (!a.hsPos || !a.hsNeg || !a.cells)) return cudaErrorInvalidValue;
     return withWaveKernel2<T>(uniform, a.passMode != kOneSweep, [&](auto k) {
         k<<<blocks, wave::kThreads2, wave::smemBytes2<T>(), s>>>(a);
         return cudaGetLastError();

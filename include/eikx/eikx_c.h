@@ -114,7 +114,10 @@ typedef struct {
                               or chunk-step kernel (node-step and pair_fields give way); no CUDA graph
                               (the schedule follows convergence); the fields do not stay on
                               the device for eikx_gradient3d / eikx_station_times3d. */
-    int reserved;
+    int test_alloc_fail;   /* test hook, 0 in production: 1 = the buffers of a solve that asks for no
+                              kernel are taken not to fit at first, so that it runs in the form
+                              that needs less memory (3D: the chunk-step kernel; 2D: one ordering
+                              per launch; identical travel times) */
 } eikx_options;
 
 /* Fills *opt with the defaults above. */
