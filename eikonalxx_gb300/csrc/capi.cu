@@ -536,7 +536,7 @@ eikx_status solveStream3(eikx_ctx *c, const eikx_options &o, int nSrc, const std
     st.totalItems = nProgress - drop;
     const int spinLog2 = o.spin_limit_log2 > 0 ? std::min(o.spin_limit_log2, 40) : 22;
     st.spinLimit = 1ull << spinLog2;
-    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, false, near64)
+    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, false, false, near64)
                        : eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
     const int blocks = std::max(1, std::min(c->numSMs * perSM, (nProgress + eikx::kWarpsPerBlock - 1) / eikx::kWarpsPerBlock));
@@ -904,7 +904,7 @@ eikx_status solveOnce(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     Workspace &w = c->ws;
     int perSM = paired ? eikx::sweep3PairBlocksPerSM()
                 : DIM == 2 ? eikx::sweep2WaveBlocksPerSM<T>(uniform)
-                : wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, false, !srcT64.empty())
+                : wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, false, warm, !srcT64.empty())
                 : chunkStep ? eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape)
                             : eikx::sweep3BlocksPerSM<T>(uniform);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
@@ -1465,7 +1465,7 @@ eikx_status solveBatch3(eikx_ctx *c, const eikx_model3d *models, const std::vect
     const int resStride = nSweepKinds * (1 + nSweeps);
 
     const bool near64 = sizeof(T) == 4 && o.near_fp64;
-    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, true, near64)
+    int perSM = wave ? eikx::sweep3WaveBlocksPerSM<T>(uniform, true, false, near64)
                        : eikx::sweep3ChunkBlocksPerSM<T>(uniform, true, shape);
     if (o.blocks_per_sm > 0) perSM = std::min(perSM, o.blocks_per_sm);
     const int blocks = std::max(1, static_cast<int>(std::min<size_t>(
@@ -1908,7 +1908,7 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
         cands.push_back(o);
     };
     // the untuned default first: wave-step
-    add(eikx::kWaveStep, 0, 0, eikx::sweep3WaveBlocksPerSM<T>(uniform, false, false));
+    add(eikx::kWaveStep, 0, 0, eikx::sweep3WaveBlocksPerSM<T>(uniform, false, false, false));
     for (int shape = 0; shape < eikx::kNumShapes; ++shape) {
         const int mx = eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape);
         add(eikx::kChunkStep, 0, shape + 1, mx);

@@ -175,7 +175,7 @@ enum Sweep3Variant { kNodeStep = 1, kChunkStep = 2, kWaveStep = 3 };
 constexpr int kWaveLY = 8, kWaveLZ = 4;
 __host__ __device__ constexpr int waveStepCap(int Px) { return Px + 32; }
 template <class T> cudaError_t launchSweep3Wave(const Sweep3Args<T> &a, bool uniform, int blocks, cudaStream_t s);
-template <class T> int sweep3WaveBlocksPerSM(bool uniform, bool batch, bool near64);
+template <class T> int sweep3WaveBlocksPerSM(bool uniform, bool batch, bool warm, bool near64);
 // After a kBothSweeps launch whose first sweep was refinement sweep r (r even; `kinds` orderings, 8 or
 // 4 in 2D), and after the kSecondSweep launch behind it: the convergence test, and which fields hold the next odd sweep.
 cudaError_t launchCheckPair(const SolveState &st, int nFields, int kinds, int r, bool second, double tol, cudaStream_t s);
