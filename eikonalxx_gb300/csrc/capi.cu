@@ -829,8 +829,15 @@ eikx_status solveOnce(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     // Measured, us a refinement sweep, chunk-step and wave-step: 256 x 256 x 128 FP32, 1 field 915,
     // 257; 16 fields 1383, 866; 64 fields 3301, 2892; 64 x 64 x 32, 1 field 264, 76; 200 x 200 x 100 in
     // double, 4 fields 4691, 1519; flat cells (non-uniform), 151 x 131 x 87, 8 fields 811, 288.
+    // Except one field on a long thin non-uniform grid: there a step is the whole operator, one after the
+    // other along x', and chunk-step keeps four of them in registers between hand-overs.  Measured, us a
+    // solve of 4 x 8 sweeps, chunk-step and wave-step, FP32 (in double): 600 x 3 x 3 8936, 10387 (89.7, 103.6
+    // ms); 1000 x 10 x 6 17316, 17584; 3000 x 20 x 20 50978, 51423; beyond the line 300 x 6 x 6 6118, 5911;
+    // 600 x 9 x 9 11585, 11061; 300 x 3 x 3 with 2 fields 5688, 5500.
+    const long long across = static_cast<long long>(ny) + nz;
+    const bool thin = DIM == 3 && !uniform && nSrc == 1 && nx >= std::min(3 * across * across, 60 * across);
     const bool wave = DIM == 3 && !paired &&
-                        (o.sweep_kernel == eikx::kWaveStep || (o.sweep_kernel == 0 && o.block_shape == 0));
+                        (o.sweep_kernel == eikx::kWaveStep || (o.sweep_kernel == 0 && o.block_shape == 0 && !thin));
     const int variant = wave ? eikx::kWaveStep : o.sweep_kernel == eikx::kNodeStep ? eikx::kNodeStep : eikx::kChunkStep;
     const bool chunkStep = DIM == 3 && !paired && variant == eikx::kChunkStep;
     // 2D grids of up to 512 rows can run one CTA per field (sweep_kernel = 2); the warp-block

@@ -73,7 +73,8 @@ typedef struct {
     int sweep_kernel;      /* 3D sweep kernel: 0 (default) = the tuned kernel of this grid class
                               if eikx_autotune3d ran, else wave-step (a lane updates one node
                               per wavefront step, rows through a shared-memory ring) unless
-                              block_shape asks for chunk-step; 1 = node-step (the earlier kernel of
+                              block_shape asks for chunk-step or one source is solved on a long
+                              thin non-uniform grid (chunk-step, faster there); 1 = node-step (the earlier kernel of
                               one node per lane and step), 2 = chunk-step (a lane updates one
                               16-byte chunk, 4 FP32 / 2 FP64 nodes, per step).  2D: 0 and 1 =
                               wave-step warp blocks of 32 rows; 2 = one CTA per field, one

@@ -1,5 +1,5 @@
-"""Instances of the wave-step kernels that only large calls take: many models whose warp blocks
-are too many to run both orderings of a pair in one launch."""
+"""Routes of a 3D solve that few calls take: many models whose warp blocks are too many to run both
+orderings of a pair in one launch, and one source on a long thin non-uniform grid."""
 import numpy as np
 import pytest
 
@@ -45,3 +45,27 @@ def test_many_models_one_ordering_per_launch(ctx, oracle, spacing, precision, ne
         cell = [min(n - 2, int(q / h)) for q, n, h in zip(p, grid, spacing)]
         ref = oracle.solve3d(m["model"], (nx, ny, nz, *spacing), cell, p, n_sweeps=4, radius=3, tol=1e-5, near_fp64=near)
         assert np.array_equal(_bits(out[-1]), _bits(ref))
+
+
+# at the line nx = 3 (ny + nz)^2, and past 60 (ny + nz) below it; one source, non-uniform: chunk-step
+@pytest.mark.parametrize("precision,near", [(ex.F32, False), (ex.F32, True), (ex.F64, False)])
+@pytest.mark.parametrize("grid,spacing,sources,chunk", [((108, 3, 3), (50.0, 65.0, 40.0), 1, True), ((107, 3, 3), (50.0, 65.0, 40.0), 1, False),
+                                                        ((1321, 15, 7), (50.0, 65.0, 40.0), 1, True), ((108, 3, 3), (50.0, 65.0, 40.0), 2, False),
+                                                        ((108, 3, 3), (50.0, 50.0, 50.0), 1, False)])
+def test_one_source_on_a_long_thin_grid(ctx, oracle, grid, spacing, sources, chunk, precision, near):
+    nx, ny, nz = grid
+    rng = np.random.default_rng(19)
+    dt = np.float32 if precision == ex.F32 else np.float64
+    s = random_slowness(rng, (nz - 1) * (ny - 1) * (nx - 1), dtype=dt)
+    ctx.set_grid3d(*grid, *spacing)
+    ctx.set_slowness3d(s)
+    pos = rng.uniform(0, 1, (sources, 3)) * (np.array(grid) - 1) * spacing
+    opt = dict(n_sweeps=2, tolerance=-1, near_fp64=near)
+    ctx.solve3d(pos, ex.Options(**opt, sweep_kernel=2), precision)
+    launches = ctx.stats()["kernel_launches"]
+    t = ctx.solve3d(pos, ex.Options(**opt), precision)
+    assert (ctx.stats()["kernel_launches"] == launches) == chunk
+    for p, a in zip(pos, t):
+        cell = [min(n - 2, int(q / h)) for q, n, h in zip(p, grid, spacing)]
+        ref = oracle.solve3d(s, (nx, ny, nz, *spacing), cell, p, n_sweeps=2, radius=3, near_fp64=near)
+        assert np.array_equal(_bits(a), _bits(ref))
