@@ -9,6 +9,7 @@
 //     bilinear (2D) or trilinear (3D; x, then y, then z) interpolation elsewhere, in FP64.
 // The gradient is one HBM-bound pass (read the field, write 2 or 3 values per node).
 #include "sweep.h"
+#include "wave.cuh"
 
 namespace eikx {
 
@@ -18,7 +19,7 @@ namespace eikx {
 // built to sit at the edges of the shortcuts -- node times within a few units in the last
 // place of the operator's own value, neighbour differences at the 2D windows' limits
 // |t_a - t_b| = hs, homogeneous slowness, unreached (huge) neighbours -- min(t0, bounded)
-// must equal min(t0, fd3UniformFar) bit for bit.
+// must equal min(t0, fd3UniformFar) bit for bit.  In FP32 also the wave-step kernel's square root.
 __device__ __forceinline__ unsigned long long splitmix(unsigned long long &x) {
     unsigned long long z = (x += 0x9E3779B97F4A7C15ull);
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -79,8 +80,17 @@ __global__ void operatorSelftestKernel(long long n, unsigned long long seed, uns
         if (!(t0 >= 0)) t0 = 0;
         const T b = fd3UniformFarBounded<T>(h, st, t0);
         const T m1 = b < t0 ? b : t0, m2 = r < t0 ? r : t0;
+        bool exact = sameBits(m1, m2);
+        if constexpr (sizeof(T) == 4) {
+            // the wave-step kernel's square root: every mantissa with both parities of the exponent (2^24
+            // values from 0.5 on), and seeded values of all exponents that it is used for
+            const unsigned lo = __float_as_uint(wave::kRootMin), range = 0x7f800000u - lo;
+            const float even = __uint_as_float(0x3f000000u + static_cast<unsigned>(i & 0xffffff));
+            const float any = __uint_as_float(lo + static_cast<unsigned>(splitmix(x) % range));
+            exact = exact && sameBits(wave::rootFast(even), dsqrt(even)) && sameBits(wave::rootFast(any), dsqrt(any));
+        }
         local[0] += 1;
-        local[1] += sameBits(m1, m2) ? 0 : 1;
+        local[1] += exact ? 0 : 1;
         local[2] += sameBits(b, t0) ? 1 : 0;
         local[3] += sameBits(r, t0) ? 1 : 0;
     }
