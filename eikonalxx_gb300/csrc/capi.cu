@@ -132,6 +132,16 @@ eikx_status sweepPairs(int kinds, int pass, bool init, Sweep sweep, Check check)
     return EIKX_OK;
 }
 
+// One field on a long thin non-uniform grid, where the chunk-step kernel is the faster one: a wave-step
+// there is the whole operator, one after the other along x', and chunk-step keeps four of them in
+// registers between hand-overs.  Measured, us a solve of 4 x 8 sweeps, chunk-step and wave-step, FP32 (in
+// double): 600 x 3 x 3 8936, 10387 (89.7, 103.6 ms); 1000 x 10 x 6 17316, 17584; 3000 x 20 x 20 50978, 51423;
+// beyond the line 300 x 6 x 6 6118, 5911; 600 x 9 x 9 11585, 11061; 300 x 3 x 3 with 2 fields 5688, 5500.
+bool thinGrid(bool uniform, int nSrc, int nx, int ny, int nz) {
+    const long long across = static_cast<long long>(ny) + nz;
+    return !uniform && nSrc == 1 && nx >= std::min(3 * across * across, 60 * across);
+}
+
 // The host's copy of a workspace's sweep-tag base.  The device's reset kernel advances the
 // base by the previous solve's tag count at the start of every solve; the host repeats that
 // step and, before a solve whose 32-bit tags would wrap (and so could meet words an early
@@ -829,13 +839,8 @@ eikx_status solveOnce(eikx_ctx *c, const double *srcXYZ, int nSrc, eikx_options 
     // Measured, us a refinement sweep, chunk-step and wave-step: 256 x 256 x 128 FP32, 1 field 915,
     // 257; 16 fields 1383, 866; 64 fields 3301, 2892; 64 x 64 x 32, 1 field 264, 76; 200 x 200 x 100 in
     // double, 4 fields 4691, 1519; flat cells (non-uniform), 151 x 131 x 87, 8 fields 811, 288.
-    // Except one field on a long thin non-uniform grid: there a step is the whole operator, one after the
-    // other along x', and chunk-step keeps four of them in registers between hand-overs.  Measured, us a
-    // solve of 4 x 8 sweeps, chunk-step and wave-step, FP32 (in double): 600 x 3 x 3 8936, 10387 (89.7, 103.6
-    // ms); 1000 x 10 x 6 17316, 17584; 3000 x 20 x 20 50978, 51423; beyond the line 300 x 6 x 6 6118, 5911;
-    // 600 x 9 x 9 11585, 11061; 300 x 3 x 3 with 2 fields 5688, 5500.
-    const long long across = static_cast<long long>(ny) + nz;
-    const bool thin = DIM == 3 && !uniform && nSrc == 1 && nx >= std::min(3 * across * across, 60 * across);
+    // Except one field on a long thin non-uniform grid (thinGrid).
+    const bool thin = DIM == 3 && thinGrid(uniform, nSrc, nx, ny, nz);
     const bool wave = DIM == 3 && !paired &&
                         (o.sweep_kernel == eikx::kWaveStep || (o.sweep_kernel == 0 && o.block_shape == 0 && !thin));
     const int variant = wave ? eikx::kWaveStep : o.sweep_kernel == eikx::kNodeStep ? eikx::kNodeStep : eikx::kChunkStep;
@@ -1914,13 +1919,16 @@ eikx_status autotune3(eikx_ctx *c, const std::vector<double> &xyz, int nSrc, eik
         o.blocks_per_sm = perSM;
         cands.push_back(o);
     };
-    // the untuned default first: wave-step
-    add(eikx::kWaveStep, 0, 0, eikx::sweep3WaveBlocksPerSM<T>(uniform, false, false, false));
+    // the untuned default first: wave-step, or the first of chunk-step
+    const bool thin = thinGrid(uniform, nSrc, c->nx, c->ny, c->nz);
+    const int wavePerSM = eikx::sweep3WaveBlocksPerSM<T>(uniform, false, false, false);
+    if (!thin) add(eikx::kWaveStep, 0, 0, wavePerSM);
     for (int shape = 0; shape < eikx::kNumShapes; ++shape) {
         const int mx = eikx::sweep3ChunkBlocksPerSM<T>(uniform, false, shape);
         add(eikx::kChunkStep, 0, shape + 1, mx);
         if (mx / 2 >= 1 && mx / 2 < mx) add(eikx::kChunkStep, 0, shape + 1, mx / 2);
     }
+    if (thin) add(eikx::kWaveStep, 0, 0, wavePerSM);
     add(eikx::kNodeStep, 0, 1, eikx::sweep3BlocksPerSM<T>(uniform));
     if (std::is_same<T, float>::value && uniform && nSrc >= 2) add(eikx::kChunkStep, 1, 1, eikx::sweep3PairBlocksPerSM());
     double best = 1e300, dflt = -1;
