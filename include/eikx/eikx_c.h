@@ -383,8 +383,8 @@ eikx_status eikx_analytic2d(eikx_ctx *ctx, const eikx_source2d *src, double v_to
  * not allocate GPU memory while they run -- hosts whose framework owns every device
  * allocation through its own pool, real-time pipelines that forbid allocation after
  * start-up, code running where cudaMalloc would synchronise or is not allowed.
- * One FP32 3D field (FP64 corner initialisation) is solved with the sweep schedule of
- * eikx_solve3d; every intermediate buffer lives in a fixed 64 MiB array compiled into
+ * One FP32 3D field (FP64 corner initialisation) is solved with the sweeps of eikx_solve3d on
+ * its chunk-step kernel (or node-step); every intermediate buffer lives in a fixed 64 MiB array compiled into
  * the library, so once the array is resident the call makes no cudaMalloc, cudaFree or
  * other allocating call.
  *   slowness: device pointer, (nx-1)(ny-1)(nz-1) cell slownesses (s/m), natural order;
@@ -392,9 +392,8 @@ eikx_status eikx_analytic2d(eikx_ctx *ctx, const eikx_source2d *src, double v_to
  *             non-finite value returns EIKX_ERR_INVALID before any sweep runs).
  *   src, opt: host pointers (opt may be NULL for the defaults).  The options are checked
  *             as eikx_solve3d checks them; sweep_kernel, block_shape and blocks_per_sm
- *             are honoured, and the value 0 means the untuned default (chunk-step
- *             kernel, 8x4 warp blocks, full occupancy): there is no context, so no
- *             autotuned choice applies.
+ *             are honoured, and the value 0 means chunk-step, 8x4 warp blocks and full
+ *             occupancy: there is no context, so no autotuned choice applies.
  *   t_out:    device pointer, nx*ny*nz travel times, natural order.
  *   stream:   a cudaStream_t (NULL = the legacy default stream); the call returns when
  *             the field is written.
@@ -504,7 +503,9 @@ eikx_status eikx_warmnet_set_test_hooks(eikx_warmnet *net, int spin_limit_log2, 
  * slowness, unreached neighbours), are evaluated by the uniform-grid Cartesian operator with
  * and without its lower-bound exits and gated operators, in precision EIKX_F32 or EIKX_F64.
  * counts[0] = stencils evaluated, counts[1] = stencils where min(t0, result) differs in any
- * bit (0 when the shortcuts are exact), counts[2] = results equal to t0, counts[3] = stencils
+ * bit (0 when the shortcuts are exact) or, in FP32, where the wave-step kernel's square root is not
+ * sqrtf's (all mantissas of both exponent parities from n = 2^24 on, and a seeded value of any
+ * exponent per stencil), counts[2] = results equal to t0, counts[3] = stencils
  * whose t0 is the operator's own value.  A test of the sweep kernels' arithmetic; it
  * allocates 32 bytes of device memory for the call. */
 eikx_status eikx_selftest_operator3d(int device, int precision, long long n, unsigned long long seed,
